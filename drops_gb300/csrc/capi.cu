@@ -200,6 +200,7 @@ int tf_destroy(tf_context* t) {
         tf::release(c->sell_iperm[i]);
         tf::release(c->sell_halo[i]);
         tf::release(c->sell_coltr[i]);
+        tf::release(c->sell_cols[i]);
     }
     tf::release(c->dof_order);
     tf::release(c->order_keys);

@@ -1,21 +1,17 @@
 // Restarted GMRES with classical Gram-Schmidt and one reorthogonalisation
-// (CGS2), right preconditioning, as one persistent cooperative kernel; the
-// Arnoldi cycles run in V = float (mixed precision: every restart is one step
-// of FP64 iterative refinement, the true residual b - A x and the update of x
-// being FP64) or in V = double.
+// (CGS2), right preconditioning, as one persistent cooperative kernel in FP64
+// (tf_gmres_options(TF_ORTH_CGS2)), and the operator B = A P^{-1} (or P^{-1} A)
+// that it shares with the modified Gram-Schmidt solver of gmres.cu.
 //
-// Compared with the modified Gram-Schmidt solver of num/krylovsolver.h:320-463
-// (k_gmres, one grid barrier per projection, about restart/2 barriers per
-// Arnoldi step), CGS2 projects against all basis vectors at once: an Arnoldi
-// step costs three grid barriers, (1) w = B v_i fused with the first
-// projection dots, (2) first update fused with the second dots and |w1|^2
-// (|w2|^2 = |w1|^2 - |h'|^2 on the orthonormal basis), (3) second update and a
-// plain grid barrier.  The preconditioned operator B = A P^{-1} (P point
-// or nodal 2x2 block Jacobi) is formed once per matrix in SELL order, so the
-// Arnoldi loop is a plain SpMV; x += P^{-1} V y at the end of a cycle.  The
+// CGS2 projects against all basis vectors at once, twice: an Arnoldi step costs
+// three grid barriers, (1) w = B v_i fused with the first projection dots, (2)
+// first update fused with the second dots and |w1|^2 (|w2|^2 = |w1|^2 - |h'|^2
+// on the orthonormal basis), (3) second update and a plain grid barrier.  B (P
+// point or nodal 2x2 block Jacobi) is formed once per matrix in SELL order, so
+// the Arnoldi loop is a plain SpMV; x += P^{-1} V y at the end of a cycle.  The
 // Hessenberg matrix, Givens rotations and the small triangular solve are
-// computed by thread 0 of the block that completes a grid step, in V, and
-// published through global memory.
+// computed by thread 0 of the block that completes a grid step, and published
+// through global memory.
 #include <cmath>
 
 #include "krylov_dev.cuh"
@@ -65,9 +61,7 @@ struct Gm2Args {
 // block 0's shared-memory copy of the state (the Hessenberg matrix and the
 // Givens rotations live in block 0's shared memory too, so the serial scalar
 // work never waits on global-memory latency), publishes the state, and
-// releases the others, which copy it.  The Arnoldi dots of the FP32 cycles
-// reduce in FP32 all the way (S = float): FP64 instructions tie up the FP64
-// pipe whatever the number of active lanes, and the basis itself is FP32.
+// releases the others, which copy it.
 // Grid-step synchronisation words: arrivals of the non-master blocks on a
 // monotone counter (one release reduction each), the master's release of the
 // step on the generation word (also bumped by grid_barrier, so monotone too).
@@ -442,7 +436,7 @@ template <class V>
 __global__ void k_gm2_bvals(int64_t nslices, int64_t half, const int32_t* __restrict__ perm,
                             const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
                             const int32_t* __restrict__ src, const int32_t* __restrict__ rowptr,
-                            const double* __restrict__ aval, const double* __restrict__ diag,
+                            const double* __restrict__ aval, int left, const double* __restrict__ diag,
                             const double* __restrict__ binv, V* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     TF_SLICE_LOOP(nslices, sl) {
@@ -455,7 +449,7 @@ __global__ void k_gm2_bvals(int64_t nslices, int64_t half, const int32_t* __rest
             if (c >= 0 && row >= 0) {
                 const int32_t j = col[q];
                 if (!binv) {
-                    v = aval[c] / diag[j];
+                    v = aval[c] / diag[left ? row : j];
                 } else {
                     const int32_t r0 = rowptr[row], nr = rowptr[row + 1] - r0;
                     const int32_t pc = (c - r0 < nr / 2) ? c + nr / 2 : c - nr / 2;
@@ -492,34 +486,51 @@ __global__ void k_gm2_block_inv(int64_t half, const int32_t* __restrict__ rowptr
     }
 }
 
+// B = A P^{-1} (right) or P^{-1} A (left, point Jacobi) in SELL order, formed
+// again when the matrix or the side changes; the nodal inverses of a block
+// matrix are left in gm2_binv.
 template <class V>
-static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int* max_iter, double* tol, int rel) {
+int gmres_operator(Context* c, CSR& A, int left, const V** out) {
     const int64_t m = A.m;
     const bool block = &A == &c->mats[TF_MAT_BLOCK];
-    DBuf<V>& bv = *reinterpret_cast<DBuf<V>*>(sizeof(V) == 4 ? (void*)&c->gm2_b32 : (void*)&c->gm2_b64);
-    // preconditioner and B = A P^{-1}, once per matrix version
+    constexpr int f32 = sizeof(V) == 4;
+    DBuf<V>& bv = *reinterpret_cast<DBuf<V>*>(f32 ? (void*)&c->gm2_b32 : (void*)&c->gm2_b64);
     if (block) TF_TRY(ensure(c, c->gm2_binv, (size_t)(2 * m)));
-    if (c->gm2_src_version[sizeof(V) == 4] != A.version || c->gm2_src_gen[sizeof(V) == 4] != A.pattern_gen) {
+    const int kind = 2 * (int)(&A - c->mats) + (left ? 1 : 0);
+    if (c->gm2_src_version[f32] != A.version || c->gm2_src_gen[f32] != A.pattern_gen || c->gm2_src_kind[f32] != kind) {
         if (block) {
             k_gm2_block_inv<<<grid_for(c, m / 2), kBlock, 0, c->stream>>>(m / 2, A.rowptr, A.colind, A.vals, c->gm2_binv.p);
             ++c->launches;
         }
         TF_TRY(ensure(c, bv, (size_t)A.sell.npad));
         k_gm2_bvals<V><<<grid_for(c, A.sell.nslices * 32), kBlock, 0, c->stream>>>(
-            A.sell.nslices, m / 2, A.sell.perm, A.sell.ptr, A.sell.col, A.sell.src, A.rowptr, A.vals,
+            A.sell.nslices, m / 2, A.sell.perm, A.sell.ptr, A.sell.col, A.sell.src, A.rowptr, A.vals, left,
             block ? nullptr : A.diag, block ? c->gm2_binv.p : nullptr, bv.p);
         ++c->launches;
         TF_CUDA(c, cudaGetLastError());
-        c->gm2_src_version[sizeof(V) == 4] = A.version;
-        c->gm2_src_gen[sizeof(V) == 4] = A.pattern_gen;
+        c->gm2_src_version[f32] = A.version;
+        c->gm2_src_gen[f32] = A.pattern_gen;
+        c->gm2_src_kind[f32] = kind;
     }
+    *out = bv.p;
+    return TF_OK;
+}
+template int gmres_operator<double>(Context*, CSR&, int, const double**);
+template int gmres_operator<float>(Context*, CSR&, int, const float**);
+
+template <class V>
+static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int* max_iter, double* tol, int rel) {
+    const int64_t m = A.m;
+    const bool block = &A == &c->mats[TF_MAT_BLOCK];
+    const V* bval = nullptr;
+    TF_TRY(gmres_operator<V>(c, A, 0, &bval));
     const void* fn = (const void*)k_gmres2<V>;
     int blocks = 0;
     TF_TRY(coop_blocks(c, fn, A.sell.nslices, &blocks, kKryThreads));
     blocks = std::min(blocks, kGm2MaxBlocks);  // the master's partial reads cover kGm2MaxBlocks blocks
     // H (R+1) x R, cs R, sn R, s R+1, y R, scl R+1, coef R+1
     const size_t small = (size_t)(R + 1) * R + 6 * (size_t)R + 3;
-    DBuf<V>& basis = *reinterpret_cast<DBuf<V>*>(sizeof(V) == 4 ? (void*)&c->gm2_v32 : (void*)&c->gm2_v64);
+    DBuf<double>& basis = c->gm2_v64;
     TF_TRY(ensure(c, basis, (size_t)(R + 1) * m + small));
     TF_TRY(ensure(c, c->kry_part, (size_t)blocks * kGm2Stride + 16 + sizeof(Gm2Scal) / 8));
     TF_TRY(ensure(c, c->kry_bar, 4));
@@ -533,7 +544,7 @@ static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int
     g.perm = A.sell.perm;
     g.ptr = A.sell.ptr;
     g.col = A.sell.col;
-    g.bval = bv.p;
+    g.bval = bval;
     g.aval = A.sell.v64;
     g.b = b;
     g.x = x;
@@ -549,7 +560,7 @@ static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int
     g.max_iter = *max_iter;
     g.rel = rel;
     g.tol = *tol;
-    g.inner_floor = sizeof(V) == 4 ? 1e-5 : 0.0;
+    g.inner_floor = 0.0;
     g.out_iter = c->kry_iters.p;
     g.out_resid = c->kry_resid.p;
     g.out_cycles = c->kry_iters.p + 1;
@@ -569,14 +580,13 @@ static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int
     return it[0] >= 0 ? TF_OK : set_err(c, TF_ERR_NOT_CONVERGED, "gmres (CGS2): no convergence within max_iter");
 }
 
-int gmres2(Context* c, CSR& A, const double* b, double* x, int restart, bool mixed, int* max_iter, double* tol, int rel) {
+int gmres2(Context* c, CSR& A, const double* b, double* x, int restart, int* max_iter, double* tol, int rel) {
     if (!A.vals || A.m <= 0) return set_err(c, TF_ERR_BAD_INPUT, "gmres: empty matrix");
     if (restart < 2 || restart > kGm2MaxR) return set_err(c, TF_ERR_CAPACITY, "gmres (CGS2): restart in [2, 64]");
     TF_TRY(ensure_diag(c, A));
     TF_TRY(ensure_sell(c, A, false));
     TimedLaunch tl(c, TF_K_GMRES);
-    return mixed ? run_gmres2<float>(c, A, b, x, restart, max_iter, tol, rel)
-                 : run_gmres2<double>(c, A, b, x, restart, max_iter, tol, rel);
+    return run_gmres2<double>(c, A, b, x, restart, max_iter, tol, rel);
 }
 
 }  // namespace tf

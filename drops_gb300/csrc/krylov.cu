@@ -1483,282 +1483,9 @@ int pcg_jacobi(Context* c, CSR& A, const double* b, double* x, int precision, in
 }
 
 // ---------------------------------------------------------------------------
-// persistent restarted GMRES (num/krylovsolver.h:320-463)
-//
-// One cooperative kernel runs the whole solve.  Basis vectors are stored
-// unnormalised with a scale factor (v_k = sc_k * V_k), so v_{i+1} = w / h_{i+1,i}
-// needs no extra pass.  Modified Gram-Schmidt keeps the reference's order:
-// one grid barrier per projection.  The Hessenberg matrix, the Givens
-// rotations and the right-hand side s live in shared memory of every block and
-// are updated redundantly (bit-identical in all blocks).
+// GMRES entry (num/krylovsolver.h:320-463)
 // ---------------------------------------------------------------------------
 constexpr int kMaxRestart = 64;
-
-struct GmresArgs {
-    double* result;
-    int64_t m, nslices;
-    const int32_t* perm;
-    const int32_t* ptr;
-    const int32_t* col;
-    const double* val;
-    const double* diag;
-    const double* b;
-    double* x;
-    double* V;     // [R][m] unnormalised basis
-    double* part;  // [2][nblocks][2]
-    GridSync gs;
-    int R;         // restart
-    int left;      // 1: left preconditioning, 0: right
-    const double* binv;  // nodal 2x2 block-Jacobi inverses [m/2][4] (NULL: point Jacobi)
-    double* Z;           // work vector for the block preconditioner
-    int max_iter;
-    double tol;
-    int rel;
-    int* out_iter;
-    double* out_resid;
-};
-
-__global__ void __launch_bounds__(kKryThreads, 2) k_gmres(GmresArgs a) {
-    const int lane = threadIdx.x & 31;
-    __shared__ double H[kMaxRestart][kMaxRestart];
-    __shared__ double cs[kMaxRestart], sn[kMaxRestart], s[kMaxRestart + 1], y[kMaxRestart], sc[kMaxRestart];
-    const int64_t m = a.m;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
-    double* partA = a.part;
-    double* partB = a.part + (size_t)gridDim.x * 2;
-    int flip = 0;
-    auto P = [&]() { flip ^= 1; return flip ? partB : partA; };
-
-    // r0 = b - A x (right) or M^{-1}(b - A x) (left) into V_0; <r,r>, |b| or |M^{-1} b|
-    {
-        double* pp = P();
-        double v[2] = {0., 0.};
-        const double* x0 = a.x;
-        TF_SLICE_LOOP_BAL(a.nslices, sl) {
-            const double ax = sell_row<double>(a.ptr, a.col, a.val, sl, lane, [&](int32_t j) { return kld(x0 + j); });
-            const int32_t row = __ldg(a.perm + sl * 32 + lane);
-            if (row >= 0) {
-                double r = a.b[row] - ax, bb = a.b[row];
-                if (a.left) {
-                    r = r / a.diag[row];
-                    bb = bb / a.diag[row];
-                }
-                a.V[row] = r;
-                v[0] += r * r;
-                v[1] += bb * bb;
-            }
-        }
-        block_partials<2>(v, pp);
-        double t[2];
-        if (!grid_sync_reduce<2>(a.gs, pp, a.result, t)) return;
-        double beta = sqrt(t[0]);
-        double normb = sqrt(t[1]);
-        if (normb == 0.0 || !a.rel) normb = 1.0;
-        double resid = beta / normb;
-        if (resid <= a.tol) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                *a.out_iter = 0;
-                *a.out_resid = resid;
-            }
-            return;
-        }
-        int j = 1;
-        while (j <= a.max_iter) {
-            if (threadIdx.x == 0) {
-                sc[0] = 1.0 / beta;
-                s[0] = beta;
-                for (int k = 1; k <= a.R; ++k) s[k] = 0.;
-            }
-            __syncthreads();
-            int i;
-            bool done = false;
-            for (i = 0; i < a.R - 1 && j <= a.max_iter; ++i, ++j) {
-                const double* Vi = a.V + (size_t)i * m;
-                double* W = a.V + (size_t)(i + 1) * m;
-                const double sci = sc[i], sc0 = sc[0];
-                // block Jacobi (right): Z = P^{-1} v_i node by node, then w = A Z
-                if (a.binv) {
-                    const int64_t half = m / 2;
-                    for (int64_t e = tid; e < half; e += nth) {
-                        const double va = sci * kld(Vi + e), vb = sci * kld(Vi + e + half);
-                        const double* q4 = a.binv + 4 * e;
-                        a.Z[e] = q4[0] * va + q4[1] * vb;
-                        a.Z[e + half] = q4[2] * va + q4[3] * vb;
-                    }
-                    if (!grid_barrier(a.gs)) return;
-                }
-                // w = A M^{-1} v_i (right) or M^{-1} A v_i (left); <w, v_0>
-                {
-                    double* pq = P();
-                    double v1[1] = {0.};
-                    const bool left = a.left;
-                    const double* dg = a.diag;
-                    const double* Zp = a.binv ? a.Z : nullptr;
-                    TF_SLICE_LOOP_BAL(a.nslices, s2) {
-                        double acc = sell_row<double>(a.ptr, a.col, a.val, s2, lane, [&](int32_t j) {
-                            if (Zp) return kld(Zp + j);
-                            const double vj = sci * kld(Vi + j);
-                            return left ? vj : vj / __ldg(dg + j);
-                        });
-                        const int32_t row = __ldg(a.perm + s2 * 32 + lane);
-                        if (row >= 0) {
-                            if (a.left) acc = acc / a.diag[row];
-                            W[row] = acc;
-                            v1[0] += acc * (sc0 * kld(a.V + row));
-                        }
-                    }
-                    block_partials<1>(v1, pq);
-                    double h[1];
-                    if (!grid_sync_reduce<1>(a.gs, pq, a.result + 2 + flip, h)) return;
-                    if (threadIdx.x == 0) H[0][i] = h[0];
-                    __syncthreads();
-                }
-                // modified Gram-Schmidt: w -= h_k v_k, then <w, v_{k+1}> (or <w,w>)
-                for (int k = 0; k <= i; ++k) {
-                    double* pq = P();
-                    const double hk = H[k][i] * sc[k];
-                    const double* Vk = a.V + (size_t)k * m;
-                    const double* Vn = k < i ? a.V + (size_t)(k + 1) * m : nullptr;
-                    const double scn = k < i ? sc[k + 1] : 0.;
-                    double v1[1] = {0.};
-                    for (int64_t e = tid; e < m; e += nth) {
-                        const double w = kld(W + e) - hk * kld(Vk + e);
-                        W[e] = w;
-                        v1[0] += k < i ? w * (scn * kld(Vn + e)) : w * w;
-                    }
-                    block_partials<1>(v1, pq);
-                    double h[1];
-                    if (!grid_sync_reduce<1>(a.gs, pq, a.result + 2 + flip, h)) return;
-                    if (threadIdx.x == 0) {
-                        if (k < i) H[k + 1][i] = h[0];
-                        else H[i + 1][i] = sqrt(h[0]);
-                    }
-                    __syncthreads();
-                }
-                if (threadIdx.x == 0) {
-                    sc[i + 1] = 1.0 / H[i + 1][i];
-                    for (int k = 0; k < i; ++k) {
-                        const double t0 = cs[k] * H[k][i] + sn[k] * H[k + 1][i];
-                        H[k + 1][i] = -sn[k] * H[k][i] + cs[k] * H[k + 1][i];
-                        H[k][i] = t0;
-                    }
-                    const double dx = H[i][i], dy = H[i + 1][i];
-                    if (dy == 0.0) {
-                        cs[i] = 1.0;
-                        sn[i] = 0.0;
-                    } else {
-                        const double r = sqrt(dx * dx + dy * dy);
-                        cs[i] = dx / r;
-                        sn[i] = dy / r;
-                    }
-                    double t0 = cs[i] * H[i][i] + sn[i] * H[i + 1][i];
-                    H[i + 1][i] = -sn[i] * H[i][i] + cs[i] * H[i + 1][i];
-                    H[i][i] = t0;
-                    t0 = cs[i] * s[i] + sn[i] * s[i + 1];
-                    s[i + 1] = -sn[i] * s[i] + cs[i] * s[i + 1];
-                    s[i] = t0;
-                }
-                __syncthreads();
-                resid = fabs(s[i + 1]) / normb;
-                if (resid <= a.tol) {
-                    done = true;
-                    break;
-                }
-            }
-            // x += V y (left) or x += M^{-1} V y (right) with k = i (converged) or i - 1
-            const int kk = done ? i : i - 1;
-            if (threadIdx.x == 0) {
-                for (int q = 0; q <= kk; ++q) y[q] = s[q];
-                for (int q = kk; q >= 0; --q) {
-                    y[q] /= H[q][q];
-                    for (int p = q - 1; p >= 0; --p) y[p] -= H[p][q] * y[q];
-                }
-            }
-            __syncthreads();
-            if (a.binv) {
-                const int64_t half = m / 2;
-                for (int64_t e = tid; e < half; e += nth) {
-                    double za = 0., zb = 0.;
-                    for (int q = 0; q <= kk; ++q) {
-                        za += y[q] * (sc[q] * kld(a.V + (size_t)q * m + e));
-                        zb += y[q] * (sc[q] * kld(a.V + (size_t)q * m + e + half));
-                    }
-                    const double* q4 = a.binv + 4 * e;
-                    a.x[e] = a.x[e] + (q4[0] * za + q4[1] * zb);
-                    a.x[e + half] = a.x[e + half] + (q4[2] * za + q4[3] * zb);
-                }
-            } else {
-                for (int64_t e = tid; e < m; e += nth) {
-                    double z = 0.;
-                    for (int q = 0; q <= kk; ++q) z += y[q] * (sc[q] * kld(a.V + (size_t)q * m + e));
-                    if (!a.left) z = z / a.diag[e];
-                    a.x[e] = a.x[e] + z;
-                }
-            }
-            if (done) {
-                if (blockIdx.x == 0 && threadIdx.x == 0) {
-                    *a.out_iter = j;
-                    *a.out_resid = resid;
-                }
-                return;
-            }
-            if (!grid_barrier(a.gs)) return;
-            // new residual into V_0
-            {
-                double* pq = P();
-                double v1[1] = {0.};
-                const double* x1 = a.x;
-                TF_SLICE_LOOP_BAL(a.nslices, s3) {
-                    const double ax = sell_row<double>(a.ptr, a.col, a.val, s3, lane, [&](int32_t j) { return kld(x1 + j); });
-                    const int32_t row = __ldg(a.perm + s3 * 32 + lane);
-                    if (row >= 0) {
-                        double r = a.b[row] - ax;
-                        if (a.left) r = r / a.diag[row];
-                        a.V[row] = r;
-                        v1[0] += r * r;
-                    }
-                }
-                block_partials<1>(v1, pq);
-                double t1[1];
-                if (!grid_sync_reduce<1>(a.gs, pq, a.result + 2 + flip, t1)) return;
-                beta = sqrt(t1[0]);
-                resid = beta / normb;
-                if (resid <= a.tol) {
-                    if (blockIdx.x == 0 && threadIdx.x == 0) {
-                        *a.out_iter = j;
-                        *a.out_resid = resid;
-                    }
-                    return;
-                }
-            }
-        }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            *a.out_iter = -(j - 1);
-            *a.out_resid = resid;
-        }
-    }
-}
-
-// nodal 2x2 block-Jacobi inverses of a 2x2 block system (rows i and i + m/2)
-__global__ void k_block_inv(int64_t half, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
-                            const double* __restrict__ vals, double* __restrict__ inv) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < half; i += (int64_t)gridDim.x * blockDim.x) {
-        double a11 = 0, a12 = 0, a21 = 0, a22 = 0;
-        for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-            if (colind[k] == i) a11 = vals[k];
-            if (colind[k] == i + half) a12 = vals[k];
-        }
-        for (int32_t k = rowptr[i + half]; k < rowptr[i + half + 1]; ++k) {
-            if (colind[k] == i) a21 = vals[k];
-            if (colind[k] == i + half) a22 = vals[k];
-        }
-        const double det = a11 * a22 - a12 * a21;
-        inv[4 * i] = a22 / det;
-        inv[4 * i + 1] = -a12 / det;
-        inv[4 * i + 2] = -a21 / det;
-        inv[4 * i + 3] = a11 / det;
-    }
-}
 
 int gmres_jacobi(Context* c, CSR& A, const double* b, double* x, int restart, int method, int precision, int* max_iter,
                  double* tol, int rel) {
@@ -1766,70 +1493,17 @@ int gmres_jacobi(Context* c, CSR& A, const double* b, double* x, int restart, in
     const bool block = &A == &c->mats[TF_MAT_BLOCK];
     if (block && method == 1)
         return set_err(c, TF_ERR_BAD_INPUT, "gmres: the block-Jacobi preconditioner is applied from the right (method 0)");
-    if (precision == TF_PREC_MIXED || (precision == TF_PREC_FP64 && c->gmres_orth == TF_ORTH_CGS2)) {
+    if (precision != TF_PREC_MIXED && precision != TF_PREC_FP64) return set_err(c, TF_ERR_BAD_INPUT, "gmres: precision");
+    if (precision == TF_PREC_MIXED || c->gmres_orth == TF_ORTH_CGS2) {
         if (method != 0) return set_err(c, TF_ERR_BAD_INPUT, "gmres (CGS2 / mixed): right preconditioning only");
-        return gmres2(c, A, b, x, restart, precision == TF_PREC_MIXED, max_iter, tol, rel);
+        if (precision == TF_PREC_FP64) return gmres2(c, A, b, x, restart, max_iter, tol, rel);
+        if (restart < 2 || restart > kMaxRestart)
+            return set_err(c, TF_ERR_CAPACITY, "gmres (mixed): restart in [2, 64]");
+        return gmres_ls<float>(c, A, b, x, restart, 0, max_iter, tol, rel);
     }
     if (restart > kMaxRestart) return set_err(c, TF_ERR_CAPACITY, "gmres: restart > 64");
-    if (precision != TF_PREC_FP64) return set_err(c, TF_ERR_BAD_INPUT, "gmres: precision");
-    TF_TRY(ensure_diag(c, A));
-    TF_TRY(ensure_sell(c, A, false));
-    const int64_t m = A.m;
     const int R = restart <= *max_iter ? restart : (*max_iter > 1 ? *max_iter : 2);
-    TimedLaunch tl(c, TF_K_GMRES);
-    TF_TRY(ensure(c, c->kry64, (size_t)(R + 1) * m + (block ? 2 * m : 0)));
-    double* binv = nullptr;
-    if (block) {
-        binv = c->kry64.p + (size_t)(R + 1) * m;
-        k_block_inv<<<grid_for(c, m / 2), kBlock, 0, c->stream>>>(m / 2, A.rowptr, A.colind, A.vals, binv);
-        ++c->launches;
-        TF_CUDA(c, cudaGetLastError());
-    }
-    const void* fn = (const void*)k_gmres;
-    int blocks = 0;
-    TF_TRY(coop_blocks(c, fn, A.sell.nslices, &blocks, kKryThreads));
-    TF_TRY(ensure(c, c->kry_part, (size_t)blocks * 2 * 2 + 8));
-    TF_TRY(ensure(c, c->kry_bar, 2));
-    TF_TRY(ensure(c, c->kry_iters, 1));
-    TF_TRY(ensure(c, c->kry_resid, 1));
-    TF_CUDA(c, cudaMemsetAsync(c->kry_bar.p, 0, 2 * sizeof(unsigned), c->stream));
-    TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
-    GmresArgs g;
-    g.m = m;
-    g.nslices = A.sell.nslices;
-    g.perm = A.sell.perm;
-    g.ptr = A.sell.ptr;
-    g.col = A.sell.col;
-    g.val = A.sell.v64;
-    g.diag = A.diag;
-    g.b = b;
-    g.x = x;
-    g.V = c->kry64.p;
-    g.part = c->kry_part.p;
-    g.result = c->kry_part.p + (size_t)blocks * 2 * 2;
-    g.gs = GridSync{c->kry_bar.p, c->kry_bar.p + 1, c->status.p};
-    g.R = R;
-    g.left = method == 1;
-    g.binv = binv;
-    g.Z = c->kry64.p + (size_t)R * m;
-    g.max_iter = *max_iter;
-    g.tol = *tol;
-    g.rel = rel;
-    g.out_iter = c->kry_iters.p;
-    g.out_resid = c->kry_resid.p;
-    void* args[] = {&g};
-    TF_CUDA(c, cudaLaunchCooperativeKernel(fn, blocks, kKryThreads, args, 0, c->stream));
-    ++c->launches;
-    int it = 0;
-    double res = 0;
-    TF_CUDA(c, cudaMemcpyAsync(&it, c->kry_iters.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    TF_CUDA(c, cudaMemcpyAsync(&res, c->kry_resid.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    int st = 0;
-    TF_TRY(sync_status(c, &st));
-    if (st) return set_err(c, st, "gmres: grid barrier watchdog fired");
-    *max_iter = it >= 0 ? it : -it;
-    *tol = res;
-    return it >= 0 ? TF_OK : set_err(c, TF_ERR_NOT_CONVERGED, "gmres: no convergence within max_iter");
+    return gmres_ls<double>(c, A, b, x, R, method == 1, max_iter, tol, rel);
 }
 
 }  // namespace tf

@@ -67,6 +67,97 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// Sums of doubles in fixed point.  An FP64 add holds a quarter of the SM's
+// FP64 pipe for 64 cycles on GB300 whatever the number of active lanes (a
+// chain of adds costs 66 cycles each, measured), so a butterfly or a serial sum
+// of partials is a chain of hundreds of cycles.  Here every mantissa is aligned
+// to the largest exponent of the sum (rounded to nearest, at 2^-2 to 2^-9 ulp of
+// the largest value) and the integers are added: a sum in any order gives the
+// same bits, about 15 integer instructions per value and one FP64-pipe
+// instruction per result (the conversion back, the only rounding to 53 bits).
+struct FxTerm {
+    unsigned e;            // biased exponent, 1 for subnormals and zero
+    unsigned long long m;  // mantissa with the hidden bit
+    bool neg;
+};
+__device__ __forceinline__ FxTerm fx_term(double v) {
+    const long long b = __double_as_longlong(v);
+    const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+    FxTerm t;
+    t.e = max(e, 1u);
+    t.m = ((unsigned long long)b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+    t.neg = b < 0;
+    return t;
+}
+// the term in units of 2^(emax - 1075 - left)
+__device__ __forceinline__ long long fx_align(const FxTerm& t, unsigned emax, int left) {
+    const unsigned sh = emax - t.e;
+    const unsigned long long m = sh < 62u ? ((t.m << left) + ((1ull << sh) >> 1)) >> sh : 0ull;
+    return t.neg ? -(long long)m : (long long)m;
+}
+__device__ __forceinline__ double fx_value(long long t, unsigned emax, int left) {
+    if (t == 0) return 0.0;
+    const int k = (int)emax - 1075 - left;
+    const long long d = __double_as_longlong(__ll2double_rn(t));
+    const int ed = (int)(d >> 52 & 0x7ff) + k;
+    if (ed <= 0 || ed >= 0x7ff) return ldexp(__longlong_as_double(d), k);
+    return __longlong_as_double(d + ((long long)k << 52));
+}
+constexpr int fx_log2(int n) { return n <= 1 ? 0 : 1 + fx_log2((n + 1) / 2); }
+
+// sum of N values of this lane
+template <int N>
+__device__ __forceinline__ double fx_sum(const double (&v)[N]) {
+    constexpr int kLeft = 10 - fx_log2(N);
+    FxTerm t[N];
+    unsigned emax = 1;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        t[k] = fx_term(v[k]);
+        emax = max(emax, t[k].e);
+    }
+    if (emax >= 0x7ffu) {  // infinities and NaN
+        double s = v[0];
+#pragma unroll
+        for (int k = 1; k < N; ++k) s += v[k];
+        return s;
+    }
+    long long s = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) s += fx_align(t[k], emax, kLeft);
+    return fx_value(s, emax, kLeft);
+}
+
+// sum over all lanes and N values per lane, in every lane
+template <int N>
+__device__ __forceinline__ double warp_fx_sum(const double (&v)[N]) {
+    constexpr int kLeft = 5 - fx_log2(N);
+    FxTerm t[N];
+    unsigned emax = 1;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        t[k] = fx_term(v[k]);
+        emax = max(emax, t[k].e);
+    }
+    emax = __reduce_max_sync(0xffffffffu, emax);
+    if (emax >= 0x7ffu) {
+        double s = v[0];
+#pragma unroll
+        for (int k = 1; k < N; ++k) s += v[k];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    }
+    long long s = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) s += fx_align(t[k], emax, kLeft);
+    // three limbs of 24, 24 and 16 bits, each summed over the warp
+    const int l0 = (int)(s & 0xffffff), l1 = (int)(s >> 24 & 0xffffff), l2 = (int)(s >> 48);
+    const long long tot = (long long)__reduce_add_sync(0xffffffffu, l0) +
+                          ((long long)__reduce_add_sync(0xffffffffu, l1) << 24) +
+                          ((long long)__reduce_add_sync(0xffffffffu, l2) << 48);
+    return fx_value(tot, emax, kLeft);
+}
+
 // Eight sums over the warp at once (a transposing butterfly): round 16 swaps
 // half of the values between the half-warps, round 8 and 4 likewise, then two
 // plain xor rounds; 9 shuffles instead of 40, in independent chains.  Lane l
@@ -91,6 +182,29 @@ __device__ __forceinline__ T warp_sum8(const T (&v)[8], int lane) {
     return a1;
 }
 
+// the same for doubles in fixed point
+__device__ __forceinline__ double warp_fx_sum8(const double (&v)[8], int lane) {
+    constexpr int kLeft = 5;
+    FxTerm t[8];
+    unsigned em[8], all = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        t[k] = fx_term(v[k]);
+        em[k] = __reduce_max_sync(0xffffffffu, t[k].e);
+        all = max(all, em[k]);
+    }
+    if (all >= 0x7ffu) return warp_sum8(v, lane);
+    long long s[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s[k] = fx_align(t[k], em[k], kLeft);
+    const long long tot = warp_sum8(s, lane);
+    const int idx = warp_sum8_index(lane);
+    unsigned e = em[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) e = idx == k ? em[k] : e;
+    return fx_value(tot, e, kLeft);
+}
+
 template <int NV, class T>
 __device__ void block_partials(T (&v)[NV], double* part /* [nblocks][NV] */) {
     __shared__ double red[NV][32];
@@ -107,89 +221,6 @@ __device__ void block_partials(T (&v)[NV], double* part /* [nblocks][NV] */) {
             if (lane == 0) part[(size_t)blockIdx.x * NV + k] = x;
         }
     __syncthreads();
-}
-
-template <int NV>
-__device__ void grid_reduce(const double* part, double (&out)[NV]) {
-    __shared__ double red[NV][32];
-    __shared__ double res[NV];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = 0; k < NV; ++k) {
-        double x = 0.;
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) x += __ldcg(part + (size_t)b * NV + k);
-        x = warp_sum(x);
-        if (lane == 0) red[k][w] = x;
-    }
-    __syncthreads();
-    if (w == 0)
-        for (int k = 0; k < NV; ++k) {
-            double x = lane < nw ? red[k][lane] : 0.;
-            x = warp_sum(x);
-            if (lane == 0) res[k] = x;
-        }
-    __syncthreads();
-    for (int k = 0; k < NV; ++k) out[k] = res[k];
-    __syncthreads();
-}
-
-// Barrier and reduction in one: every block has written its NV partials; the
-// last block to arrive sums all of them in a fixed order (so the result does
-// not depend on which block is last), publishes the NV sums, and releases the
-// others.  Cost: one reduction of nblocks values instead of one per block.
-template <int NV>
-__device__ bool grid_sync_reduce(const GridSync& g, const double* part, double* result, double (&out)[NV]) {
-    __shared__ int last;
-    __shared__ double red[NV][32];
-    __shared__ int st;
-    __syncthreads();
-    unsigned my = 0;
-    if (threadIdx.x == 0) {
-        volatile unsigned* vgen = g.gen;
-        my = *vgen;
-        __threadfence();
-        last = atomicAdd(g.count, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last) {
-        __threadfence();
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        for (int k = 0; k < NV; ++k) {
-            double x = 0.;
-            for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) x += __ldcg(part + (size_t)b * NV + k);
-            x = warp_sum(x);
-            if (lane == 0) red[k][w] = x;
-        }
-        __syncthreads();
-        if (w == 0)
-            for (int k = 0; k < NV; ++k) {
-                double x = lane < nw ? red[k][lane] : 0.;
-                x = warp_sum(x);
-                if (lane == 0) result[k] = x;
-            }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            *g.count = 0;
-            __threadfence();
-            atomicAdd(g.gen, 1u);
-        }
-    } else if (threadIdx.x == 0) {
-        volatile unsigned* vgen = g.gen;
-        long long spins = 0;
-        while (*vgen == my) {
-            if (++spins > kSpinLimit) {
-                atomicCAS(g.status, 0, TF_ERR_WATCHDOG);
-                break;
-            }
-            if (spins > 256) __nanosleep(32);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) st = *((volatile int*)g.status);
-    __syncthreads();
-    if (st != 0) return false;
-    for (int k = 0; k < NV; ++k) out[k] = __ldcg(result + k);
-    return true;
 }
 
 // Scalar state of a persistent Krylov solve in global memory.  Only thread 0
@@ -358,72 +389,118 @@ static_assert(kArMax == 8, "records of eight values");
 
 // Sums v[k] over every thread of the grid into out[k] (identical in all
 // threads).  Call from all threads of every block, in uniform control flow.
-template <class T, int NV>
-__device__ bool grid_allreduce(const GridAR& g, unsigned long long& epoch, const T (&v)[NV], T (&out)[NV]) {
+// FP64 values: fixed-point warp sums, value k in warp k, so no chain of FP64
+// adds is left on the way.
+template <int NV>
+__device__ bool grid_allreduce_f64(const GridAR& g, unsigned long long& epoch, const double (&v)[NV],
+                                   double (&out)[NV]) {
     static_assert(NV >= 1 && NV <= kArMax, "all-reduce width");
-    constexpr int kReadWarps = 8;  // warps that load block records
-    __shared__ T red[kArMax][32];
-    __shared__ T tot_w[kArMax][kReadWarps];
-    __shared__ T res[kArMax];
+    __shared__ double red[NV][32];
+    __shared__ double res[NV];
     __shared__ int st;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    T* part = ar_part<T>(g) + (size_t)(epoch & 1) * gridDim.x * kArMax;
-    // all NV sums of a warp at once (transposing butterfly, 9 shuffles)
-    const int idx = warp_sum8_index(lane);
-    {
-        T v8[8];
+    double* part = g.partd + (size_t)(epoch & 1) * gridDim.x * kArMax;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v8[k] = k < NV ? v[k] : T(0);
-        const T tot = warp_sum8(v8, lane);
-        if ((lane & 3) == 0 && idx < NV) red[idx][w] = tot;
+    for (int k = 0; k < NV; ++k) {
+        const double one[1] = {v[k]};
+        const double tot = warp_fx_sum(one);
+        if (lane == 0) red[k][w] = tot;
     }
     __syncthreads();
-    if (threadIdx.x < NV) {
-        T x = T(0);
-        for (int ww = 0; ww < nw; ++ww) x += red[threadIdx.x][ww];
-        part[(size_t)blockIdx.x * kArMax + threadIdx.x] = x;
+    for (int k = w; k < NV; k += nw) {
+        const double one[1] = {lane < nw ? red[k][lane] : 0.};
+        const double x = warp_fx_sum(one);
+        if (lane == 0) part[(size_t)blockIdx.x * kArMax + k] = x;
     }
     if (!ar_arrive_wait(g, epoch, &st)) return false;
     ++epoch;
-    // the block records (kArMax values: 32 or 64 bytes, 16-byte loads, one
-    // L2 sector request per record) are spread over up to kReadWarps warps,
-    // one record per lane, so that they are in flight at once; each warp sums
-    // its records (in the order of the chunks it took, then the fixed shuffle
-    // tree), and NV lanes of warp 0 add the warp totals in warp order, so
-    // every block derives the same bits.  Only the NV used values are added:
-    // FP64 adds issue at a small fraction of the FP32 rate.
-    // FP64 records (the FP64 solvers, up to 3 blocks per SM) stay on one warp:
-    // the warp-sum trees of eight warps cost more FP64 issue than the
-    // sequential loads save
-    const int nchunks = (int)((gridDim.x + 31) / 32);
-    const int nread = sizeof(T) == 8 ? 1 : nw < kReadWarps ? nw : kReadWarps;
-    if (w < nread) {
-        T acc[8];
+    for (int k = w; k < NV; k += nw) {
+        double x = 0.;
+        for (unsigned c0 = 0; c0 < gridDim.x; c0 += 256) {
+            double p[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = T(0);
-        for (int ch = w; ch < nchunks; ch += nread) {
-            const unsigned b = (unsigned)ch * 32u + (unsigned)lane;
-            if (b < gridDim.x) {
-                T rec[8];
-                ar_load_record(part + (size_t)b * kArMax, rec);
-#pragma unroll
-                for (int k = 0; k < NV; ++k) acc[k] += rec[k];
+            for (int u = 0; u < 8; ++u) {
+                const unsigned b = c0 + 32 * u + lane;
+                p[u] = b < gridDim.x ? __ldcg(part + (size_t)b * kArMax + k) : 0.;
             }
+            const double s = warp_fx_sum(p);
+            x = c0 ? x + s : s;
         }
-        const T tot = warp_sum8(acc, lane);
-        if ((lane & 3) == 0 && idx < NV) tot_w[idx][w] = tot;
-    }
-    __syncthreads();
-    if (threadIdx.x < NV) {
-        const int nused = nchunks < nread ? nchunks : nread;
-        T x = tot_w[threadIdx.x][0];
-        for (int ww = 1; ww < nused; ++ww) x += tot_w[threadIdx.x][ww];
-        res[threadIdx.x] = x;
+        if (lane == 0) res[k] = x;
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NV; ++k) out[k] = res[k];
     return true;
+}
+
+// the same sums in T = float (or double, above)
+template <class T, int NV>
+__device__ bool grid_allreduce(const GridAR& g, unsigned long long& epoch, const T (&v)[NV], T (&out)[NV]) {
+    static_assert(NV >= 1 && NV <= kArMax, "all-reduce width");
+    if constexpr (sizeof(T) == 8) {
+        return grid_allreduce_f64<NV>(g, epoch, v, out);
+    } else {
+        constexpr int kReadWarps = 8;  // warps that load block records
+        __shared__ T red[kArMax][32];
+        __shared__ T tot_w[kArMax][kReadWarps];
+        __shared__ T res[kArMax];
+        __shared__ int st;
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        T* part = ar_part<T>(g) + (size_t)(epoch & 1) * gridDim.x * kArMax;
+        // all NV sums of a warp at once (transposing butterfly, 9 shuffles)
+        const int idx = warp_sum8_index(lane);
+        {
+            T v8[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v8[k] = k < NV ? v[k] : T(0);
+            const T tot = warp_sum8(v8, lane);
+            if ((lane & 3) == 0 && idx < NV) red[idx][w] = tot;
+        }
+        __syncthreads();
+        if (threadIdx.x < NV) {
+            T x = T(0);
+            for (int ww = 0; ww < nw; ++ww) x += red[threadIdx.x][ww];
+            part[(size_t)blockIdx.x * kArMax + threadIdx.x] = x;
+        }
+        if (!ar_arrive_wait(g, epoch, &st)) return false;
+        ++epoch;
+        // the block records (kArMax values: 32 or 64 bytes, 16-byte loads, one
+        // L2 sector request per record) are spread over up to kReadWarps warps,
+        // one record per lane, so that they are in flight at once; each warp sums
+        // its records (in the order of the chunks it took, then the fixed shuffle
+        // tree), and NV lanes of warp 0 add the warp totals in warp order, so
+        // every block derives the same bits.
+        const int nchunks = (int)((gridDim.x + 31) / 32);
+        const int nread = nw < kReadWarps ? nw : kReadWarps;
+        if (w < nread) {
+            T acc[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k] = T(0);
+            for (int ch = w; ch < nchunks; ch += nread) {
+                const unsigned b = (unsigned)ch * 32u + (unsigned)lane;
+                if (b < gridDim.x) {
+                    T rec[8];
+                    ar_load_record(part + (size_t)b * kArMax, rec);
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) acc[k] += rec[k];
+                }
+            }
+            const T tot = warp_sum8(acc, lane);
+            if ((lane & 3) == 0 && idx < NV) tot_w[idx][w] = tot;
+        }
+        __syncthreads();
+        if (threadIdx.x < NV) {
+            const int nused = nchunks < nread ? nchunks : nread;
+            T x = tot_w[threadIdx.x][0];
+            for (int ww = 1; ww < nused; ++ww) x += tot_w[threadIdx.x][ww];
+            res[threadIdx.x] = x;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NV; ++k) out[k] = res[k];
+        return true;
+    }
 }
 
 // plain barrier on the same counter

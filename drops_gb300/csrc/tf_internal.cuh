@@ -341,6 +341,8 @@ struct Context {
     DBuf<float2> sell_v2f[TF_NUM_MATS];
     DBuf<int32_t> sell_rexp[TF_NUM_MATS];
     DBuf<int32_t> sell_iperm[TF_NUM_MATS], sell_halo[TF_NUM_MATS];
+    DBuf<int32_t> sell_cols[TF_NUM_MATS];  // GMRES: SELL columns as slots
+    int64_t sell_cols_gen[TF_NUM_MATS] = {-1, -1, -1, -1, -1, -1, -1, -1};
     DBuf<uint16_t> sell_coltr[TF_NUM_MATS];
     bool pcg_resident = true;   // PCG: block share of the system resident in shared memory where it fits
     bool autotune = true;       // measured launch shapes per matrix structure (tune.cu)
@@ -411,6 +413,7 @@ struct Context {
     DBuf<float> gm2_b32, gm2_v32;
     DBuf<double> gm2_b64, gm2_v64, gm2_binv;
     int64_t gm2_src_version[2] = {-1, -1}, gm2_src_gen[2] = {-1, -1};
+    int gm2_src_kind[2] = {-1, -1};  // matrix handle and side of the preconditioner
     int gmres_orth = TF_ORTH_MGS;
 };
 
@@ -535,7 +538,11 @@ int gmres_jacobi(Context* c, CSR& A, const double* b, double* x, int restart, in
                  int* max_iter, double* tol, int rel);
 int ensure_diag(Context* c, CSR& A);
 int coop_blocks(Context* c, const void* fn, int64_t nslices, int* out, int threads, size_t dyn_smem = 0);
-int gmres2(Context* c, CSR& A, const double* b, double* x, int restart, bool mixed, int* max_iter, double* tol, int rel);
+int gmres2(Context* c, CSR& A, const double* b, double* x, int restart, int* max_iter, double* tol, int rel);
+template <class V>
+int gmres_operator(Context* c, CSR& A, int left, const V** out);
+template <class V>
+int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, int* max_iter, double* tol, int rel);
 int ch_steps(Context* c, int nsteps, double dt, double mob, double eps, double beta_s, double xi, double rho_vol,
              int restart, double tol, int max_iter, int warm, int* iters, double* resids);
 void release_solver_workspace(Context* c);

@@ -329,11 +329,13 @@ int tf_autotune_info(tf_context* ctx, int mat, int* spmv_threads, int* spmv_bloc
 int tf_gmres_jacobi(tf_context* ctx, int mat, int vec_b, int vec_x, int restart, int method, int precision,
                     int* max_iter, double* tol, int rel);
 /* Orthogonalisation of tf_gmres_jacobi in FP64: TF_ORTH_MGS (default) is the
- * reference's modified Gram-Schmidt, one grid barrier per projection;
+ * reference's modified Gram-Schmidt, its coefficients from one grid reduction
+ * per Arnoldi step (forward substitution with the basis' inner products);
  * TF_ORTH_CGS2 is classical Gram-Schmidt with one reorthogonalisation, three
  * grid barriers per Arnoldi step, right preconditioning only.  TF_PREC_MIXED
- * always uses CGS2 with FP32 Arnoldi cycles, each restart being one step of
- * FP64 iterative refinement (true residual and update of x in FP64).          */
+ * always uses modified Gram-Schmidt with FP32 Arnoldi cycles, each restart
+ * being one step of FP64 iterative refinement (true residual and update of x
+ * in FP64).                                                                    */
 #define TF_ORTH_MGS 0
 #define TF_ORTH_CGS2 1
 int tf_gmres_options(tf_context* ctx, int orth);

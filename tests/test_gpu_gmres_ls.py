@@ -1,0 +1,78 @@
+"""Two-grid-step MGS GMRES on general matrices: sizes around the slices and runs of its blocks, every side and restart."""
+import numpy as np
+import pytest
+
+import drops_gb300 as tf
+from oracle import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-11
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from drops_gb300 import build
+
+    build.build()
+    c = tf.TraceFEM()
+    yield c
+    c.close()
+
+
+def banded(m, seed):
+    """Nonsymmetric CSR matrix with diagonal 2 and off-diagonal row sums of absolute values at most 1, so
+    |A^-1|_inf <= 1: entries at distance 1, 7 and m // 3."""
+    rng = np.random.default_rng(seed)
+    rows, cols, vals = [np.arange(m)], [np.arange(m)], [np.full(m, 2.0)]
+    for d in {1, 7, max(m // 3, 1)}:
+        for s in (d, -d):
+            i = np.arange(max(0, -s), m - max(0, s))
+            if i.size:
+                rows.append(i)
+                cols.append(i + s)
+                vals.append(rng.uniform(-1.0, 1.0, i.size) / 6.0)
+    rows, cols, vals = (np.concatenate(x) for x in (rows, cols, vals))
+    o = np.lexsort((cols, rows))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=m))]).astype(np.int64)
+    return rp, cols[o].astype(np.int64), vals[o], rng.standard_normal(m)
+
+
+def solve(ctx, A, b, restart, method, prec):
+    ctx.matrix_upload(*A)
+    ctx.vec_upload(tf.VEC_B, b)
+    ctx.vec_upload(tf.VEC_X, np.zeros(b.size))
+    st, it, res = ctx.gmres_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, restart=restart, tol=TOL, method=method, precision=prec)
+    assert st == tf.OK and res <= TOL
+    return it, ctx.vec_download(tf.VEC_X)
+
+
+@pytest.mark.parametrize("m", [1, 31, 33, 512, 513, 20011])
+@pytest.mark.parametrize("restart,method,prec", [(2, 0, 0), (3, 1, 0), (50, 0, 0), (64, 1, 0), (64, 0, 0), (2, 0, 1),
+                                                 (64, 0, 1)])
+def test_gmres_sizes(ctx, m, restart, method, prec):
+    """Both solvers stop at |r| <= TOL |b| (left: |D^-1 r| <= TOL |D^-1 b|, D = 2), and |A^-1|_inf <= 1, so the
+    solutions differ by at most 2 TOL |b| in the maximum norm (10% more for the rounding of the residuals)."""
+    rp, ci, v, b = banded(m, m + restart)
+    it, x = solve(ctx, (rp, ci, v), b, restart, method, prec)
+    _, ox, oit, _ = O.gmres_jacobi(rp, ci, v, b, restart=restart, tol=TOL, method=method)
+    assert np.abs(x - ox).max() <= 2.2 * TOL * np.linalg.norm(b)
+    if prec == tf.PREC_FP64:
+        assert abs(it - oit) <= 2, (it, oit)
+
+
+def test_gmres_run_beyond_shared_memory(ctx):
+    """More rows per block than its shared memory holds (FP64, 1.7 million rows): w and v_i from global memory."""
+    rp, ci, v, b = banded(1700000, 3)
+    _, x = solve(ctx, (rp, ci, v), b, 10, 0, tf.PREC_FP64)
+    r = b - O.spmv(rp, ci, v, x)
+    assert np.linalg.norm(r) <= 1.01 * TOL * np.linalg.norm(b)
+
+
+def test_gmres_uneven_magnitudes(ctx):
+    """Right-hand side over 200 decades: the fixed-point sums align every term to the largest of its sum, so the
+    residual reached is the one a 64-bit sum reports."""
+    rp, ci, v, b = banded(3000, 9)
+    b = b * 10.0 ** np.random.default_rng(1).uniform(-200, 0, b.size)
+    _, x = solve(ctx, (rp, ci, v), b, 50, 0, tf.PREC_FP64)
+    r = b - O.spmv(rp, ci, v, x)
+    assert np.linalg.norm(r) <= 1.01 * TOL * np.linalg.norm(b)
