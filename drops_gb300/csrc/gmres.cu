@@ -73,6 +73,7 @@ struct GmLsArgs {
     V* zrow;               // m values (block Jacobi: the update before P^{-1})
     V* part;               // [2][blocks][kLsVals]
     GridAR g;
+    PackedAR pkd, pkn;     // dots, norm
     int R, max_iter, rel, left, nloc;  // nloc: slots of the largest run held in shared memory (0: none)
     double tol, inner_floor;
     int* out_iter;
@@ -96,6 +97,7 @@ struct LsSmall {  // least-squares state, identical in every block
     double resid, normb, beta;
     int flag;
     int lmax;                // largest |L_kj| of the cycle (bits of a float)
+    int amax, Ew;            // largest |<w, v_k>| of the step (bits), exponent of the last |w|
 };
 
 __device__ __forceinline__ float ls_add(const float (&p)[16]) {
@@ -184,6 +186,13 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
         return true;
     };
 
+    PkState pkn;
+    unsigned pepoch = 0;
+    unsigned long long plast[4] = {0ull, 0ull, 0ull, 0ull};
+    if (threadIdx.x == 0) {
+        q.Ew = kPkUnknown;
+        q.amax = 0;
+    }
     bool first = true;
     for (;;) {
         // ---- residual r = b - A x (FP64) into basis_0, its norm ----
@@ -288,22 +297,67 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                     if ((lane & 3) == 0) q.pd[warp * 8 + warp_sum8_index(lane)] = tot;
                 }
                 __syncthreads();
-                if ((int)threadIdx.x < 2 * i + 1) {
-                    const int u = (int)threadIdx.x <= i ? 0 : 4, k = (int)threadIdx.x <= i ? threadIdx.x : threadIdx.x - i - 1;
+                // thread j < 2 i + 1: <w, v_j> (j <= i), then <v_i, v_k>, over the block; one word of a packed
+                // reduction per value (two in FP64), its unit from |w| of the step before (1 for <v_i, v_k>)
+                const int n = 2 * i + 1, j = threadIdx.x;
+                V sum = V(0);
+                if (j < n) {
+                    const int u = j <= i ? 0 : 4, k = j <= i ? j : j - i - 1;
                     const V* p = q.pd + (k >> 2) * 8 + u + (k & 3);
-                    V sum = p[0];
+                    sum = p[0];
                     for (int t = 1; t < parts; ++t) sum += p[t * groups * 8];
-                    a.part[((size_t)(epoch & 1) * gridDim.x + blockIdx.x) * kLsVals + threadIdx.x] = sum;
+                    sum *= q.scl[k];
+                    if (j > i) sum *= sci;
+                }
+                int st = 1;
+                const int Ew = q.Ew;
+                if (Ew != kPkUnknown) {
+                    st = 0;
+                    if (j < n) {
+                        const int E = j <= i ? Ew : 0;
+                        const int odd = pepoch & 1;
+                        if constexpr (kMixed) {
+                            unsigned long long* w = a.pkd.w + odd * kPkWords + j;
+                            bool bad;
+                            const long long t = pk_fix(sum, E, &bad);
+                            red_relaxed_add_u64(w, pk_word(t, bad));
+                            unsigned long long diff = 0;
+                            if (!pk_wait(w, odd ? plast[1] : plast[0], a.pkd.status, &diff)) st = 2;
+                            else if (pk_misfit(diff)) st = 1;
+                            q.tot[j] = pk_value(pk_sum(diff), E);
+                        } else {
+                            unsigned long long* w = a.pkd.w + odd * kPkWords + 2 * j;
+                            bool bad;
+                            long long hi, lo;
+                            pk_fix(sum, E, &hi, &lo, &bad);
+                            if (!pk_carry(&hi, &lo)) bad = true;
+                            red_relaxed_add_u64(w, pk_word(hi, bad));
+                            red_relaxed_add_u64(w + 1, pk_word(lo, bad));
+                            unsigned long long dh = 0, dl = 0;
+                            if (!pk_wait(w, odd ? plast[1] : plast[0], a.pkd.status, &dh) ||
+                                !pk_wait(w + 1, odd ? plast[3] : plast[2], a.pkd.status, &dl))
+                                st = 2;
+                            else if (pk_misfit(dh)) st = 1;
+                            q.tot[j] = pk_value(pk_sum(dh), (long long)(dl >> 16), E);
+                        }
+                    }
+                    ++pepoch;
+                    if (__syncthreads_or(st == 2)) return;
+                    st = __syncthreads_or(st);
+                }
+                if (st) {  // no |w| yet, or a value beyond the range of its unit
+                    if (j < n) a.part[((size_t)(epoch & 1) * gridDim.x + blockIdx.x) * kLsVals + j] = sum;
+                    if (!reduce(n)) return;
                 }
             }
-            if (!reduce(2 * i + 1)) return;
             // h = (I + L)^{-1} a.  While max |L|^2 is below the rounding of a, h = a - L a to that rounding: a
             // product over four warps; else forward substitution, two entries per lane of warp 0.
             if ((int)threadIdx.x <= i) {
                 const int k = threadIdx.x;
-                q.aw[k] = q.scl[k] * q.tot[k];
+                q.aw[k] = q.tot[k];
+                atomicMax(&q.amax, __float_as_int(fabsf((float)q.tot[k])));
                 if (k < i) {
-                    const V l = q.scl[k] * (sci * q.tot[i + 1 + k]);
+                    const V l = q.tot[i + 1 + k];
                     q.L[k][i] = l;
                     atomicMax(&q.lmax, __float_as_int(fabsf((float)l)));
                 }
@@ -382,7 +436,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                 nrm[0] += w * w;
             }
             V o[1];
-            if (!grid_allreduce<V, 1>(a.g, epoch, nrm, o)) return;
+            if (!packed_allreduce<1>(a.pkn, pkn, a.g, epoch, nrm, o, true)) return;
             ++it;
             if (warp == 0) {
                 // lane 0: 1 / |w|; lane 1: 1 / r, r = |(hlast, |w|)|
@@ -395,6 +449,8 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                     const bool zero = n2 == V(0);
                     const V c = zero ? V(1) : t * ir, s = zero ? V(0) : hn * ir;
                     q.scl[i + 1] = ih;
+                    q.Ew = pk_exp(fmaxf(__int_as_float(q.amax), fabsf((float)hn)));
+                    q.amax = 0;
                     q.cs[i] = c;
                     q.sn[i] = s;
                     q.H[i][i] = c * t + s * hn;
@@ -521,7 +577,7 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     const int64_t ns = A.sell.nslices, ld = ns * 32;
     // at least two slices per block: a block's share of the reductions (its
     // partials are read by every other block) outweighs less work per block
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(c->num_sms, ns / 2));
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(c->num_sms, kPkMaxBlocks), ns / 2));
     DBuf<V>& basis = *reinterpret_cast<DBuf<V>*>(sizeof(V) == 4 ? (void*)&c->gm2_v32 : (void*)&c->gm2_v64);
     TF_TRY(ensure(c, basis, (size_t)(R + 1) * ld + (block ? (size_t)m : 0)));
     const size_t part_v = (size_t)2 * blocks * kLsVals, part_r = (size_t)2 * blocks * kArMax;
@@ -531,6 +587,8 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     TF_TRY(ensure(c, c->kry_resid, 1));
     TF_CUDA(c, cudaMemsetAsync(c->kry_bar.p, 0, 4 * sizeof(unsigned), c->stream));
     TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
+    unsigned long long* pw = nullptr;
+    TF_TRY(packed_words(c, 2, &pw));
     const void* fn = (const void*)k_gmres_ls<V>;
     cudaFuncAttributes fa{};
     int optin = 0;
@@ -567,6 +625,8 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     g.g.partd = c->kry_part.p + part_v;
     g.g.partf = reinterpret_cast<float*>(c->kry_part.p + part_v + part_r);
     g.g.status = c->status.p;
+    g.pkd = PackedAR{pw, c->status.p};
+    g.pkn = PackedAR{pw + 2 * kPkWords, c->status.p};
     g.R = R;
     g.max_iter = *max_iter;
     g.rel = rel;

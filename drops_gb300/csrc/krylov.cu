@@ -1239,6 +1239,7 @@ void release_solver_workspace(Context* c) {
     release(c->kry_part);
     release(c->kry_resid);
     release(c->kry_bar);
+    release(c->kry_packed);
     release(c->kry_iters);
 }
 
@@ -1408,6 +1409,11 @@ int pcg_jacobi(Context* c, CSR& A, const double* b, double* x, int precision, in
         if (c->pcg_fp64_kernel == TF_PCG_FP64_CG1) {
             bool applied = false;
             const int st = pcg_resident<double>(c, A, b, x, max_iter, tol, rel, &applied);
+            if (applied || st != TF_OK) return st;
+        }
+        if (c->pcg_resident) {
+            bool applied = false;
+            const int st = pcg64_resident(c, A, b, x, max_iter, tol, rel, &applied);
             if (applied || st != TF_OK) return st;
         }
         TF_TRY(ensure(c, c->kry64, (size_t)(5 * m)));

@@ -133,6 +133,7 @@ struct PcgResArgs {
     V* V1;
     T* P;
     GridAR g;
+    PackedAR pk;
     int max_iter;
     double tol;
     int rel;
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
     __shared__ double sh[4];
 
     unsigned long long epoch = 0;
+    PkState pk;
     V* Vc = a.V0;
     V* Vn = a.V1;
     const int64_t sb0 = balanced_part_start(a.ptr, a.nslices, blockIdx.x, gridDim.x);
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
                 v[5] += rn * rn;
             }
         }
-        if (!grid_allreduce<T, 6>(a.g, epoch, v, o)) return false;
+        if (!packed_allreduce<6>(a.pk, pk, a.g, epoch, v, o, true)) return false;
         V* t = Vc;
         Vc = Vn;
         Vn = t;
@@ -391,6 +393,195 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *a.out_iter = converged ? it : -1 - it;
         *a.out_updates = updates;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 PCG with the reference's recurrences on the resident structure
+// (PCGSolverCL<JACPcCL>::Solve, num/krylovsolver.h:107-189): two reductions per
+// iteration, <p, A p> and then <r, r>, <z, r>.  A block keeps its rows' p, r, x
+// and 1/d, its translated columns and its values in shared memory, and its own
+// copy of the halo rows' p, which it advances itself (p = z + beta p) from the
+// owners' published z: one 8-byte load per halo row and iteration, one FP64
+// multiply-add per stored entry, no division in the row updates.
+//
+// Bound: latency of the two reductions and the FP64 pipe (64 cycles per warp
+// instruction and quarter of an SM).  Against the kernel that walks the SELL
+// matrix in global memory and forms z + beta p per entry (k_pcg, which remains
+// for systems whose block share does not fit), per iteration on GB300:
+// RESFILL
+// ---------------------------------------------------------------------------
+struct Pcg64Args {
+    int64_t m, nslices;
+    const int32_t* perm;
+    const int32_t* ptr;
+    const uint16_t* col_tr;
+    const int32_t* halo_rows;
+    const int32_t* halo_n;
+    const double* val;
+    const double* diag;
+    const double* b;
+    double* x;
+    double* Z;
+    GridAR g;
+    PackedAR pk1, pk2;
+    int max_iter;
+    double tol;
+    int rel;
+    int* out_iter;
+    double* out_resid;
+    int smax, hmax;
+    int32_t ccap, vcap;
+};
+
+// dynamic shared memory: Ps[slots + hmax] p, rs, xs, ds, qs[slots] each, sperm[slots], hrow[hmax],
+// ccol[ccap] (16-bit), cval[vcap]
+inline size_t pcg64_fixed_bytes(int smax, int hmax, int32_t ccap) {
+    const size_t slots = (size_t)smax * 32;
+    return slots * (5 * sizeof(double) + sizeof(int32_t)) + (size_t)hmax * (sizeof(double) + sizeof(int32_t)) +
+           (((size_t)ccap * 2 + 31) & ~(size_t)31);
+}
+
+__global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
+    constexpr int NW = kResThreads / 32;
+    const int lane = threadIdx.x & 31;
+    extern __shared__ __align__(32) unsigned char res_dyn[];
+    const size_t slots = (size_t)a.smax * 32;
+    double* Ps = reinterpret_cast<double*>(res_dyn);
+    double* rs = Ps + slots + a.hmax;
+    double* xs = rs + slots;
+    double* ds = xs + slots;  // 1 / diagonal
+    double* qs = ds + slots;
+    int32_t* sperm = reinterpret_cast<int32_t*>(qs + slots);
+    int32_t* hrow = sperm + slots;
+    uint16_t* ccol = reinterpret_cast<uint16_t*>(hrow + a.hmax);
+    double* cval = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ccol) + (((size_t)a.ccap * 2 + 31) & ~(size_t)31));
+    __shared__ BalShared<NW, double> bsh;
+    __shared__ double sh[4];
+    __shared__ int flag;
+
+    unsigned long long epoch = 0;
+    PkState pk1, pk2;
+    const int64_t sb0 = balanced_part_start(a.ptr, a.nslices, blockIdx.x, gridDim.x);
+    const int64_t sb1 = balanced_part_start(a.ptr, a.nslices, blockIdx.x + 1, gridDim.x);
+    const int S = (int)(sb1 - sb0), NS = S * 32;
+    const int32_t pb = __ldg(a.ptr + sb0), nslot = __ldg(a.ptr + sb1) - pb;
+    const int nh = __ldg(a.halo_n + blockIdx.x);
+    for (int k = threadIdx.x; k < NS; k += kResThreads) {
+        const int32_t row = __ldg(a.perm + sb0 * 32 + k);
+        sperm[k] = row;
+        const double x = row >= 0 ? a.x[row] : 0.;
+        xs[k] = x;
+        Ps[k] = x;  // operand of the first product
+        ds[k] = row >= 0 ? 1.0 / a.diag[row] : 0.;
+    }
+    for (int h = threadIdx.x; h < nh; h += kResThreads) {
+        const int32_t row = __ldg(a.halo_rows + (size_t)blockIdx.x * kHaloMax + h);
+        hrow[h] = row;
+        Ps[NS + h] = a.x[row];
+    }
+    for (int32_t k = threadIdx.x; k < nslot; k += kResThreads) {
+        ccol[k] = __ldg(a.col_tr + pb + k);
+        if (k < a.vcap) cval[k] = __ldg(a.val + pb + k);
+    }
+    sell_block_plan<NW, double>(bsh, a.ptr, sb0, S);  // ends with a block barrier
+    // q = A Ps over the run; returns this thread's part of <q, Ps>
+    auto walk = [&]() -> double {
+        double pq = 0.;
+        sell_block_walk_fn<NW, double>(
+            bsh, sb0, S,
+            [&](int64_t s, int32_t c0, int32_t n) {
+                const int i = (int)(s - sb0);
+                const int32_t p0 = 32 * (bsh.P[i] + c0) + lane;
+                const bool vsh = 32 * bsh.P[i + 1] <= a.vcap;
+                return res_row<double>(ccol + p0, vsh ? cval + p0 : a.val + pb + p0, vsh, n, Ps);
+            },
+            [&](int64_t s, double val) {
+                const int ls = (int)(s - sb0) * 32 + lane;
+                qs[ls] = val;
+                pq += val * Ps[ls];
+            });
+        return pq;
+    };
+    double thr2, rr;
+    int it = 0;
+    {
+        walk();
+        double v[3] = {0., 0., 0.};
+        for (int t = threadIdx.x; t < NS; t += kResThreads) {
+            const int32_t row = sperm[t];
+            double r = 0., z = 0.;
+            if (row >= 0) {
+                const double bi = a.b[row];
+                r = bi - qs[t];
+                z = r * ds[t];
+                a.Z[row] = z;
+                v[1] += bi * bi;
+            }
+            rs[t] = r;
+            Ps[t] = 0.;
+            v[0] += r * r;
+            v[2] += z * r;
+        }
+        for (int h = threadIdx.x; h < nh; h += kResThreads) Ps[NS + h] = 0.;
+        double o[3];
+        if (!grid_allreduce<double, 3>(a.g, epoch, v, o)) return;
+        double nb = 1.0;
+        if (threadIdx.x == 0) {
+            nb = sqrt(o[1]);
+            if (nb == 0.0 || !a.rel) nb = 1.0;
+            sh[0] = nb;
+            sh[1] = 0.;                // beta
+            sh[2] = 1.0 / o[2];        // 1 / rho
+            sh[3] = (a.tol * nb) * (a.tol * nb);
+            flag = o[0] <= sh[3] || a.max_iter <= 0;
+        }
+        rr = o[0];
+        __syncthreads();
+        thr2 = sh[3];
+    }
+    const double normb = sh[0];
+    bool done = flag != 0;
+    while (!done) {
+        const double beta = sh[1];
+        // p = z + beta p on the halo and the block's rows
+        for (int h = threadIdx.x; h < nh; h += kResThreads) Ps[NS + h] = __ldcg(a.Z + hrow[h]) + beta * Ps[NS + h];
+        for (int t = threadIdx.x; t < NS; t += kResThreads) Ps[t] = rs[t] * ds[t] + beta * Ps[t];
+        __syncthreads();
+        double v1[1], o1[1];
+        v1[0] = walk();
+        if (!packed_allreduce<1>(a.pk1, pk1, a.g, epoch, v1, o1, false)) return;
+        if (threadIdx.x == 0) sh[0] = 1.0 / (o1[0] * sh[2]);  // alpha = rho / <p, A p>
+        __syncthreads();
+        const double alpha = sh[0];
+        double v[2] = {0., 0.}, o[2];
+        for (int t = threadIdx.x; t < NS; t += kResThreads) {
+            const int32_t row = sperm[t];
+            xs[t] += alpha * Ps[t];
+            const double r = rs[t] - alpha * qs[t];
+            const double z = r * ds[t];
+            rs[t] = r;
+            if (row >= 0) a.Z[row] = z;
+            v[0] += r * r;
+            v[1] += z * r;
+        }
+        if (!packed_allreduce<2>(a.pk2, pk2, a.g, epoch, v, o, true)) return;
+        ++it;
+        rr = o[0];
+        if (threadIdx.x == 0) {
+            sh[1] = o[1] * sh[2];
+            flag = rr <= thr2 || it >= a.max_iter;
+        }
+        __syncthreads();
+        // 1 / rho of the next iteration, off the path of the others (read after two barriers)
+        if (threadIdx.x == kResThreads - 32) sh[2] = 1.0 / o[1];
+        done = flag != 0;
+    }
+    for (int t = threadIdx.x; t < NS; t += kResThreads)
+        if (sperm[t] >= 0) a.x[sperm[t]] = xs[t];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.out_iter = rr <= thr2 ? it : -1 - it;
+        *a.out_resid = sqrt(rr) / normb;
     }
 }
 
@@ -545,7 +736,32 @@ int ensure_res_plan(Context* c, CSR& A, int blocks) {
     return TF_OK;
 }
 
+// Blocks of a resident solve: one per SM, and at least two slices each (a
+// smaller share saves less than another block adds to the reductions).
+int res_blocks(const Context* c, const CSR& A) {
+    return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(c->num_sms, kPkMaxBlocks), A.sell.nslices / 2));
+}
+
+// shared memory a block of fn can use besides its static part
+int res_room(Context* c, const void* fn, int64_t* room) {
+    cudaFuncAttributes fa{};
+    int optin = 0;
+    TF_CUDA(c, cudaFuncGetAttributes(&fa, fn));
+    TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    *room = (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024;
+    return TF_OK;
+}
+
 }  // namespace
+
+// zeroed words for n packed reductions
+int packed_words(Context* c, int n, unsigned long long** w) {
+    const size_t words = (size_t)n * 2 * kPkWords;
+    TF_TRY(ensure(c, c->kry_packed, words));
+    TF_CUDA(c, cudaMemsetAsync(c->kry_packed.p, 0, sizeof(unsigned long long) * words, c->stream));
+    *w = c->kry_packed.p;
+    return TF_OK;
+}
 
 // Resident single-barrier PCG; *applied = false (nothing launched) when a
 // block's run does not fit the shared memory.
@@ -555,15 +771,12 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     *applied = false;
     const int64_t m = A.m;
     const void* fn = (const void*)k_pcg_res<T>;
-    const int blocks = c->num_sms;  // one 512-thread block per SM
+    const int blocks = res_blocks(c, A);
     TF_TRY(ensure_res_plan(c, A, blocks));
     const Sell& S = A.sell;
     if (!S.res_ok || S.res_smax <= 0 || S.res_smax > kBalMaxSlices) return TF_OK;
-    cudaFuncAttributes fa{};
-    int optin = 0;
-    TF_CUDA(c, cudaFuncGetAttributes(&fa, fn));
-    TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    const int64_t room = (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024;
+    int64_t room = 0;
+    TF_TRY(res_room(c, fn, &room));
     const int32_t ccap = (S.res_maxslots + 15) & ~15;
     const int64_t fixed = (int64_t)res_fixed_bytes<T>(S.res_smax, S.res_hmax, ccap);
     if (fixed > room) return TF_OK;
@@ -602,7 +815,10 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     TF_TRY(ensure(c, c->kry_resid, 1));
     TF_CUDA(c, cudaMemsetAsync(c->kry_bar.p, 0, 2 * sizeof(unsigned), c->stream));
     TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
+    unsigned long long* pw = nullptr;
+    TF_TRY(packed_words(c, 1, &pw));
     PcgResArgs<T> g;
+    g.pk = PackedAR{pw, c->status.p};
     g.m = m;
     g.nslices = S.nslices;
     g.perm = S.perm;
@@ -654,5 +870,79 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
 
 template int pcg_resident<float>(Context*, CSR&, const double*, double*, int*, double*, int, bool*);
 template int pcg_resident<double>(Context*, CSR&, const double*, double*, int*, double*, int, bool*);
+
+// FP64 PCG (reference recurrences) on the resident structure; *applied = false
+// (nothing launched) when a block's run does not fit the shared memory.
+int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied) {
+    *applied = false;
+    const int64_t m = A.m;
+    const void* fn = (const void*)k_pcg64_res;
+    const int blocks = res_blocks(c, A);
+    TF_TRY(ensure_res_plan(c, A, blocks));
+    const Sell& S = A.sell;
+    if (!S.res_ok || S.res_smax <= 0 || S.res_smax > kBalMaxSlices) return TF_OK;
+    const int32_t ccap = (S.res_maxslots + 15) & ~15;
+    int64_t room = 0;
+    TF_TRY(res_room(c, fn, &room));
+    const int64_t fixed = (int64_t)pcg64_fixed_bytes(S.res_smax, S.res_hmax, ccap);
+    if (fixed > room) return TF_OK;
+    const int32_t vcap = (int32_t)std::min<int64_t>((room - fixed) / (int64_t)sizeof(double), (int64_t)ccap) & ~7;
+    const size_t dyn = (size_t)fixed + (size_t)vcap * sizeof(double);
+    TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    int per_sm = 0;
+    TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kResThreads, dyn));
+    if (per_sm < 1) return TF_OK;
+    TF_TRY(ensure(c, c->kry64, (size_t)m));
+    const size_t part_d = (size_t)2 * blocks * kArMax;
+    TF_TRY(ensure(c, c->kry_part, part_d + 16));
+    TF_TRY(ensure(c, c->kry_bar, 2));
+    TF_TRY(ensure(c, c->kry_iters, 4));
+    TF_TRY(ensure(c, c->kry_resid, 1));
+    TF_CUDA(c, cudaMemsetAsync(c->kry_bar.p, 0, 2 * sizeof(unsigned), c->stream));
+    TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
+    unsigned long long* pw = nullptr;
+    TF_TRY(packed_words(c, 2, &pw));
+    Pcg64Args g{};
+    g.pk1 = PackedAR{pw, c->status.p};
+    g.pk2 = PackedAR{pw + 2 * kPkWords, c->status.p};
+    g.m = m;
+    g.nslices = S.nslices;
+    g.perm = S.perm;
+    g.ptr = S.ptr;
+    g.col_tr = S.col_tr;
+    g.halo_rows = S.halo_rows;
+    g.halo_n = S.halo_n;
+    g.val = S.v64;
+    g.diag = A.diag;
+    g.b = b;
+    g.x = x;
+    g.Z = c->kry64.p;
+    g.g.count = reinterpret_cast<unsigned long long*>(c->kry_bar.p);
+    g.g.partd = c->kry_part.p;
+    g.g.status = c->status.p;
+    g.max_iter = *max_iter;
+    g.tol = *tol;
+    g.rel = rel;
+    g.out_iter = c->kry_iters.p;
+    g.out_resid = c->kry_resid.p;
+    g.smax = S.res_smax;
+    g.hmax = S.res_hmax;
+    g.ccap = ccap;
+    g.vcap = vcap;
+    void* args[] = {&g};
+    TF_CUDA(c, cudaLaunchCooperativeKernel(fn, blocks, kResThreads, args, dyn, c->stream));
+    ++c->launches;
+    *applied = true;
+    int it = 0;
+    double res = 0;
+    TF_CUDA(c, cudaMemcpyAsync(&it, c->kry_iters.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    TF_CUDA(c, cudaMemcpyAsync(&res, c->kry_resid.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    int st = 0;
+    TF_TRY(sync_status(c, &st));
+    if (st) return set_err(c, st, "pcg: grid barrier watchdog fired");
+    *max_iter = it >= 0 ? it : -1 - it;
+    *tol = res;
+    return it >= 0 ? TF_OK : set_err(c, TF_ERR_NOT_CONVERGED, "pcg: no convergence within max_iter");
+}
 
 }  // namespace tf

@@ -311,6 +311,7 @@ struct Context {
     DBuf<double> kry64, kry_part, kry_resid;
     DBuf<float> kry32;
     DBuf<unsigned> kry_bar;
+    DBuf<unsigned long long> kry_packed;  // words of the packed reductions
     DBuf<int> kry_iters;
     // scratch
     DBuf<unsigned char> scratch;
@@ -528,6 +529,8 @@ int spmv(Context* c, const CSR& A, const double* x, double* y);
 int pcg_jacobi(Context* c, CSR& A, const double* b, double* x, int precision, int* max_iter, double* tol, int rel);
 template <class T>
 int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);
+int packed_words(Context* c, int n, unsigned long long** w);
+int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);
 // kinds of the single-barrier mixed PCG (autotuned per matrix structure, tune.cu)
 constexpr int kPcgResident = 0, kPcgCg1_512 = 1, kPcgCg1_256 = 2;
 int pcg_mixed_kind(Context* c, CSR& A, const double* b, double* x, int kind, int* max_iter, double* tol, int rel);
