@@ -15,7 +15,8 @@
 // block's rows.  Every pass then
 //   1. forms u = (r - alpha (w + beta s)) / d for the block's rows and, from
 //      the state gathered once from global memory, for its halo rows, into one
-//      array (the halo loads are issued first, in one round);
+//      array (the halo loads are issued first, in one round; states lie in slot
+//      order and a halo list ascends, so neighbouring threads share sectors);
 //   2. walks its SELL run entirely in shared memory (column, value, u);
 //   3. updates its rows, publishes their new state to the global double
 //      buffer for the other blocks' halos, and joins the grid all-reduce.
@@ -32,6 +33,13 @@
 // max_iter, and then confirms convergence on the true residual b - A x.  The
 // precomputed u keeps it at one FP64 multiply-add per stored entry (the
 // on-the-fly u of k_pcg_cg1 would cost three more on GB300's narrow FP64 pipe).
+//
+// Mixed, per iteration on GB300 (P2 sphere on 96^3 cubes, 146,042 rows): 12.4 us
+// with the counter all-reduce, states in row order and p of the halo kept in
+// shared memory; 11.3 us with the packed reduction and the room given to matrix
+// values (a block whose last slices' values came from L2 walked 6.2 us instead of
+// 4.4); 9.3 us with the states in slot order and ascending halo lists (the block
+// with the largest halo loaded it in 2.6 us against 1.2 in the mean).
 //
 // Applicability is decided on the host: every block's run (slot rows, halo,
 // translated columns) must fit the shared memory and its vector 16-bit
@@ -89,7 +97,8 @@ __device__ __forceinline__ T res_u(const V& v, T al, T be) {
 
 // n columns of one slot row: translated columns cp[32 k] (shared memory),
 // values vp[32 k] (shared memory when vsh, else global), vector xs (shared
-// memory).  Terms are summed in column order.
+// memory).  The columns and values of the next eight are loaded while the
+// gathers of the current eight are in flight.  Terms are summed in column order.
 template <class T>
 __device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* __restrict__ vp, bool vsh, int32_t n,
                                      const T* __restrict__ xs) {
@@ -122,7 +131,7 @@ struct PcgResArgs {
     const int32_t* ptr;
     const int32_t* col;
     const uint16_t* col_tr;    // SELL columns translated to the owning block's vector
-    const int32_t* halo_rows;  // [block][kHaloMax]
+    const int32_t* halo_slots;  // [block][kHaloMax]
     const int32_t* halo_n;     // [block]
     const T* val;              // SELL values in T
     const double* val64;       // SELL values in FP64 (true residual)
@@ -148,13 +157,13 @@ struct PcgResArgs {
 };
 
 // dynamic shared memory of one block, in this order (every part a multiple of 32 bytes):
-// Vs[slots] state, Us[slots + hmax] u, Ps[slots + hmax] p, sdx[slots], wsm[slots], ssm[slots],
+// Vs[slots] state, Us[slots + hmax] u, Ps[slots] p, sdx[slots], wsm[slots], ssm[slots],
 // sperm[slots], hrow[hmax], ccol[ccap] (16-bit), cval[vcap]
 template <class T>
 inline size_t res_fixed_bytes(int smax, int hmax, int32_t ccap) {
     using V = typename ResState<T>::V;
     const size_t slots = (size_t)smax * 32;
-    return slots * (sizeof(V) + 5 * sizeof(T) + sizeof(int32_t)) + (size_t)hmax * (2 * sizeof(T) + sizeof(int32_t)) +
+    return slots * (sizeof(V) + 5 * sizeof(T) + sizeof(int32_t)) + (size_t)hmax * (sizeof(T) + sizeof(int32_t)) +
            (((size_t)ccap * 2 + 31) & ~(size_t)31);
 }
 
@@ -167,8 +176,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
     const size_t slots = (size_t)a.smax * 32;
     V* Vs = reinterpret_cast<V*>(res_dyn);
     T* Us = reinterpret_cast<T*>(Vs + slots);
-    T* Ps = Us + slots + a.hmax;  // own slots: p; halo part: p of the halo rows (refresh)
-    T* sdx = Ps + slots + a.hmax;
+    T* Ps = Us + slots + a.hmax;
+    T* sdx = Ps + slots;
     T* wsm = sdx + slots;  // products A u; with ssm also the FP64 residual products
     T* ssm = wsm + slots;  // products A p (refresh)
     double* rres = reinterpret_cast<double*>(wsm);
@@ -188,6 +197,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
     const int64_t sb1 = balanced_part_start(a.ptr, a.nslices, blockIdx.x + 1, gridDim.x);
     const int S = (int)(sb1 - sb0);
     const int NS = S * 32;  // own slots; halo entries follow at NS + h
+    const int64_t NS0 = sb0 * 32;  // first own slot: states and p are published in slot order
     const int32_t pb = __ldg(a.ptr + sb0), pe = __ldg(a.ptr + sb1);
     const int32_t nslot = pe - pb;
     const int nh = __ldg(a.halo_n + blockIdx.x);
@@ -197,7 +207,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
         Ps[k] = T(0);
         sdx[k] = T(0);
     }
-    for (int h = threadIdx.x; h < nh; h += kResThreads) hrow[h] = __ldg(a.halo_rows + (size_t)blockIdx.x * kHaloMax + h);
+    for (int h = threadIdx.x; h < nh; h += kResThreads) hrow[h] = __ldg(a.halo_slots + (size_t)blockIdx.x * kHaloMax + h);
     for (int32_t k = threadIdx.x; k < nslot; k += kResThreads) {
         ccol[k] = __ldg(a.col_tr + pb + k);
         if (k < a.vcap) cval[k] = __ldg(a.val + pb + k);
@@ -227,13 +237,13 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
                 V vc;
                 if (first) {
                     vc = mk_state((T)ri, T(0), T(0), T(1) / a.diag[row]);
-                    a.P[row] = T(0);
+                    a.P[NS0 + ls] = T(0);
                 } else {
                     vc = Vs[ls];
                     vc.x = (T)ri;
                 }
                 Vs[ls] = vc;
-                st_st(Vc + row, vc);
+                st_st(Vc + NS0 + ls, vc);
                 v[0] += ri * ri;
                 if (first) v[1] += bi * bi;
             }
@@ -269,80 +279,76 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
     auto pass = [&](bool refresh, T (&o)[6]) -> bool {
         T v[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
         const T al = refresh ? T(0) : alpha, be = refresh ? T(0) : beta;
-        // u of the block's rows and of its halo, p of the halo on a refresh: the
-        // halo states (global memory) are loaded first, kHaloRegs per thread at
-        // once, and the block's own rows (shared memory) are done while they
+        // u of the block's rows and of its halo: the halo states (global memory) are loaded first,
+        // kHaloRegs per thread at once, and the block's own rows (shared memory) are done while they
         // are in flight (fewer at once for the 32-byte FP64 state: registers)
         constexpr int kHaloRegs = sizeof(T) == 4 ? 4 : 2;
         V hv[kHaloRegs];
-        T hp[kHaloRegs];
 #pragma unroll
         for (int q = 0; q < kHaloRegs; ++q) {
             const int h = threadIdx.x + q * kResThreads;
-            if (h < nh) {
-                const int32_t r = hrow[h];
-                hv[q] = st_ld(Vc + r);
-                if (refresh) hp[q] = kld(a.P + r);
-            }
+            if (h < nh) hv[q] = st_ld(Vc + hrow[h]);
         }
         for (int t = threadIdx.x; t < NS; t += kResThreads) Us[t] = sperm[t] >= 0 ? res_u<T>(Vs[t], al, be) : T(0);
 #pragma unroll
         for (int q = 0; q < kHaloRegs; ++q) {
             const int h = threadIdx.x + q * kResThreads;
-            if (h < nh) {
-                Us[NS + h] = res_u<T>(hv[q], al, be);
-                if (refresh) Ps[NS + h] = hp[q];
-            }
+            if (h < nh) Us[NS + h] = res_u<T>(hv[q], al, be);
         }
-        for (int h = threadIdx.x + kHaloRegs * kResThreads; h < nh; h += kResThreads) {
-            const int32_t r = hrow[h];
-            Us[NS + h] = res_u<T>(st_ld(Vc + r), al, be);
-            if (refresh) Ps[NS + h] = kld(a.P + r);
-        }
+        for (int h = threadIdx.x + kHaloRegs * kResThreads; h < nh; h += kResThreads)
+            Us[NS + h] = res_u<T>(st_ld(Vc + hrow[h]), al, be);
         __syncthreads();
         // the slice offsets of the run come from the plan in shared memory:
         // ptr[sb0 + i] - pb = 32 * bsh.P[i]
-        auto walk = [&](const T* xs, T* out) {
+        auto walk = [&](auto emit) {
             sell_block_walk_fn<NW, T>(
                 bsh, sb0, S,
                 [&](int64_t s, int32_t c0, int32_t n) {
                     const int i = (int)(s - sb0);
                     const int32_t p0 = 32 * (bsh.P[i] + c0) + lane;
                     const bool vsh = 32 * bsh.P[i + 1] <= a.vcap;
-                    return res_row<T>(ccol + p0, vsh ? cval + p0 : a.val + pb + p0, vsh, n, xs);
+                    return res_row<T>(ccol + p0, vsh ? cval + p0 : a.val + pb + p0, vsh, n, Us);
                 },
-                [&](int64_t s, T val) { out[(s - sb0) * 32 + lane] = val; });
+                [&](int64_t s, T val) { emit((int)(s - sb0) * 32 + lane, val); });
         };
-        walk(Us, wsm);
-        if (refresh) walk(Ps, ssm);  // s = A p recomputed, ending the drift of its recurrence
-        for (int i = wid; i < S; i += NW) {
-            const int ls = i * 32 + lane;
-            const int32_t row = sperm[ls];
-            if (row >= 0) {
-                const V vc = Vs[ls];
-                T sn, rn, pn;
-                if (refresh) {
-                    sn = ssm[ls];
-                    rn = vc.x;
-                    pn = Ps[ls];
-                } else {
-                    sn = fma_rn(be, vc.z, vc.y);
-                    rn = fma_rn(-al, sn, vc.x);
-                    pn = fma_rn(be, Ps[ls], mul_rn(vc.x, vc.w));
-                    Ps[ls] = pn;
-                    sdx[ls] = fma_rn(al, pn, sdx[ls]);
-                }
-                const T un = mul_rn(rn, vc.w), wn = wsm[ls];
-                const V nv = mk_state(rn, wn, sn, vc.w);
-                Vs[ls] = nv;
-                st_st(Vn + row, nv);
-                v[0] += rn * un;
-                v[1] += un * wn;
-                v[2] += un * sn;
-                v[3] += pn * wn;
-                v[4] += pn * sn;
-                v[5] += rn * rn;
+        // row update of one slot from its product w = A u (refresh: and s = A p)
+        auto row_update = [&](int ls, T wn, T sx) {
+            if (sperm[ls] < 0) return;
+            const V vc = Vs[ls];
+            T sn, rn, pn;
+            if (refresh) {
+                sn = sx;
+                rn = vc.x;
+                pn = Ps[ls];
+            } else {
+                sn = fma_rn(be, vc.z, vc.y);
+                rn = fma_rn(-al, sn, vc.x);
+                pn = fma_rn(be, Ps[ls], mul_rn(vc.x, vc.w));
+                Ps[ls] = pn;
+                sdx[ls] = fma_rn(al, pn, sdx[ls]);
             }
+            const T un = mul_rn(rn, vc.w);
+            const V nv = mk_state(rn, wn, sn, vc.w);
+            Vs[ls] = nv;
+            st_st(Vn + NS0 + ls, nv);
+            v[0] += rn * un;
+            v[1] += un * wn;
+            v[2] += un * sn;
+            v[3] += pn * wn;
+            v[4] += pn * sn;
+            v[5] += rn * rn;
+        };
+        if (!refresh) {
+            walk([&](int ls, T val) { wsm[ls] = val; });
+            for (int i = wid; i < S; i += NW) row_update(i * 32 + lane, wsm[i * 32 + lane], T(0));
+        } else {
+            // w = A u, then s = A p recomputed, ending the drift of its recurrence
+            walk([&](int ls, T val) { wsm[ls] = val; });
+            for (int t = threadIdx.x; t < NS; t += kResThreads) Us[t] = Ps[t];
+            for (int h = threadIdx.x; h < nh; h += kResThreads) Us[NS + h] = kld(a.P + hrow[h]);
+            __syncthreads();
+            walk([&](int ls, T val) { ssm[ls] = val; });
+            for (int i = wid; i < S; i += NW) row_update(i * 32 + lane, wsm[i * 32 + lane], ssm[i * 32 + lane]);
         }
         if (!packed_allreduce<6>(a.pk, pk, a.g, epoch, v, o, true)) return false;
         V* t = Vc;
@@ -359,7 +365,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
             if (row >= 0) {
                 a.x[row] += (double)sdx[ls];
                 sdx[ls] = T(0);
-                a.P[row] = Ps[ls];
+                a.P[NS0 + ls] = Ps[ls];
             }
         }
         return grid_sync_ar(a.g, epoch);
@@ -409,14 +415,15 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
 // instruction and quarter of an SM).  Against the kernel that walks the SELL
 // matrix in global memory and forms z + beta p per entry (k_pcg, which remains
 // for systems whose block share does not fit), per iteration on GB300:
-// RESFILL
+// P2 torus on 41^3 cubes (35,592 rows, 152 blocks) 23.1 -> 11.7 us, P1 sphere on
+// 16^3 (664 rows, 16 blocks) 12.1 -> 8.4 us.
 // ---------------------------------------------------------------------------
 struct Pcg64Args {
     int64_t m, nslices;
     const int32_t* perm;
     const int32_t* ptr;
     const uint16_t* col_tr;
-    const int32_t* halo_rows;
+    const int32_t* halo_slots;
     const int32_t* halo_n;
     const double* val;
     const double* diag;
@@ -476,9 +483,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
         ds[k] = row >= 0 ? 1.0 / a.diag[row] : 0.;
     }
     for (int h = threadIdx.x; h < nh; h += kResThreads) {
-        const int32_t row = __ldg(a.halo_rows + (size_t)blockIdx.x * kHaloMax + h);
-        hrow[h] = row;
-        Ps[NS + h] = a.x[row];
+        const int32_t slot = __ldg(a.halo_slots + (size_t)blockIdx.x * kHaloMax + h);
+        hrow[h] = slot;
+        Ps[NS + h] = a.x[__ldg(a.perm + slot)];
     }
     for (int32_t k = threadIdx.x; k < nslot; k += kResThreads) {
         ccol[k] = __ldg(a.col_tr + pb + k);
@@ -515,9 +522,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
                 const double bi = a.b[row];
                 r = bi - qs[t];
                 z = r * ds[t];
-                a.Z[row] = z;
                 v[1] += bi * bi;
             }
+            a.Z[sb0 * 32 + t] = z;
             rs[t] = r;
             Ps[t] = 0.;
             v[0] += r * r;
@@ -556,12 +563,11 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
         const double alpha = sh[0];
         double v[2] = {0., 0.}, o[2];
         for (int t = threadIdx.x; t < NS; t += kResThreads) {
-            const int32_t row = sperm[t];
             xs[t] += alpha * Ps[t];
             const double r = rs[t] - alpha * qs[t];
             const double z = r * ds[t];
             rs[t] = r;
-            if (row >= 0) a.Z[row] = z;
+            a.Z[sb0 * 32 + t] = z;
             v[0] += r * r;
             v[1] += z * r;
         }
@@ -597,87 +603,84 @@ __global__ void k_sell_iperm(int64_t nslots, const int32_t* __restrict__ perm, i
     }
 }
 
-// Per part b of the balanced partition (one block each): the halo rows (the
-// distinct columns of the run whose slots lie outside it, numbered in the
-// order of an open-addressing table of kHashSlots entries -- deterministic:
-// the table's content does not depend on insertion order, and the numbering
-// is a scan over its slots) and the run's columns translated to the block's
-// vector (own slot, or NS + halo number).  info[0]: set when a table or a
-// halo overflows or an index needs more than 16 bits; info[1]: largest run
-// in slices, info[2]: largest run in slots, info[3]: largest halo.
+// Per part b of the balanced partition (one block each): the halo slots (the
+// distinct columns of the run, as slots, that lie outside it), ascending, so
+// that consecutive threads read neighbouring states, and the run's columns
+// translated to the block's vector (own slot, or NS + halo number).  An open-
+// addressing table finds the distinct ones, a bitonic sort orders them, a
+// binary search translates.  info[0]: set when a table or a halo overflows or an
+// index needs more than 16 bits; info[1]: largest run in slices, info[2]: largest
+// run in slots, info[3]: largest halo.
 __device__ __forceinline__ uint32_t halo_hash(int32_t c) { return ((uint32_t)c * 2654435761u) >> 19; }  // 13 bits
 static_assert(kHashSlots == 1 << 13, "hash width");
 
 __global__ void __launch_bounds__(512) k_res_halo(const int32_t* __restrict__ ptr, int64_t nslices,
                                                   const int32_t* __restrict__ col, const int32_t* __restrict__ iperm,
-                                                  uint16_t* __restrict__ col_tr, int32_t* __restrict__ halo_rows,
+                                                  uint16_t* __restrict__ col_tr, int32_t* __restrict__ halo_slots,
                                                   int32_t* __restrict__ halo_n, int* __restrict__ info) {
-    extern __shared__ int32_t hsh[];  // keys[kHashSlots], ids[kHashSlots]
+    extern __shared__ int32_t hsh[];  // keys[kHashSlots], list[kHaloMax]
     int32_t* keys = hsh;
-    int32_t* ids = hsh + kHashSlots;
-    __shared__ int32_t wsum[16];
-    __shared__ int bad;
+    int32_t* list = hsh + kHashSlots;
+    __shared__ int bad, cnt;
     const int64_t sb0 = balanced_part_start(ptr, nslices, blockIdx.x, gridDim.x);
     const int64_t sb1 = balanced_part_start(ptr, nslices, blockIdx.x + 1, gridDim.x);
     const int NS = (int)(sb1 - sb0) * 32;
     const int32_t lo = (int32_t)(sb0 * 32), hi = (int32_t)(sb1 * 32);
     const int32_t pb = ptr[sb0], pe = ptr[sb1];
     for (int i = threadIdx.x; i < kHashSlots; i += blockDim.x) keys[i] = -1;
-    if (threadIdx.x == 0) bad = 0;
+    if (threadIdx.x == 0) bad = cnt = 0;
     __syncthreads();
     for (int32_t k = pb + threadIdx.x; k < pe; k += blockDim.x) {
-        const int32_t c = col[k];
-        const int32_t sl = iperm[c];
+        const int32_t sl = iperm[col[k]];
         if (sl >= lo && sl < hi) continue;
-        uint32_t h = halo_hash(c);
+        uint32_t h = halo_hash(sl);
         int probe = 0;
         for (; probe < kHashSlots; ++probe) {
-            const int32_t old = atomicCAS(&keys[h], -1, c);
-            if (old == -1 || old == c) break;
+            const int32_t old = atomicCAS(&keys[h], -1, sl);
+            if (old == -1) {
+                const int id = atomicAdd(&cnt, 1);  // the order is lost in the sort
+                if (id < kHaloMax) list[id] = sl;
+            }
+            if (old == -1 || old == sl) break;
             h = (h + 1) & (kHashSlots - 1);
         }
         if (probe == kHashSlots) bad = 1;
     }
     __syncthreads();
-    // number the occupied table entries in slot order (block scan, 16 entries per thread)
-    constexpr int kPer = kHashSlots / 512;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    int cnt = 0;
-    for (int q = 0; q < kPer; ++q) cnt += keys[t * kPer + q] >= 0;
-    int inc = cnt;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) wsum[w] = inc;
-    __syncthreads();
-    int base = 0;
-    for (int q = 0; q < w; ++q) base += wsum[q];
-    int id = base + inc - cnt;
-    for (int q = 0; q < kPer; ++q) {
-        const int i = t * kPer + q;
-        if (keys[i] >= 0) {
-            ids[i] = id;
-            if (id < kHaloMax) halo_rows[(size_t)blockIdx.x * kHaloMax + id] = keys[i];
-            ++id;
-        }
-    }
-    __syncthreads();
-    int nh = 0;
-    for (int q = 0; q < 16; ++q) nh += wsum[q];
-    if (nh > kHaloMax || NS + nh > 65535) bad = 1;
+    const int nh = cnt;
+    if (threadIdx.x == 0 && (nh > kHaloMax || NS + nh > 65535)) bad = 1;
     __syncthreads();
     if (!bad) {
+        int np = 1;
+        while (np < nh) np <<= 1;  // at most kHaloMax
+        for (int i = nh + threadIdx.x; i < np; i += blockDim.x) list[i] = 0x7fffffff;
+        __syncthreads();
+        for (int size = 2; size <= np; size <<= 1)
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int i = threadIdx.x; i < np; i += blockDim.x) {
+                    const int p = i ^ stride;
+                    if (p > i) {
+                        const int32_t x = list[i], y = list[p];
+                        if ((x > y) == ((i & size) == 0)) {
+                            list[i] = y;
+                            list[p] = x;
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+        for (int i = threadIdx.x; i < nh; i += blockDim.x) halo_slots[(size_t)blockIdx.x * kHaloMax + i] = list[i];
         for (int32_t k = pb + threadIdx.x; k < pe; k += blockDim.x) {
-            const int32_t c = col[k];
-            const int32_t sl = iperm[c];
-            int32_t tr;
-            if (sl >= lo && sl < hi) {
-                tr = sl - lo;
-            } else {
-                uint32_t h = halo_hash(c);
-                while (keys[h] != c) h = (h + 1) & (kHashSlots - 1);  // present: inserted above
-                tr = NS + ids[h];
+            const int32_t sl = iperm[col[k]];
+            int32_t tr = sl - lo;
+            if (sl < lo || sl >= hi) {
+                int l = 0, r = nh - 1;  // list[l] == sl at the end: inserted above
+                while (l < r) {
+                    const int mid = (l + r) >> 1;
+                    if (list[mid] < sl) l = mid + 1;
+                    else r = mid;
+                }
+                tr = NS + l;
             }
             col_tr[k] = (uint16_t)tr;
         }
@@ -714,13 +717,13 @@ int ensure_res_plan(Context* c, CSR& A, int blocks) {
         TF_TRY(ensure(c, c->sell_coltr[id], (size_t)(S.npad > 0 ? S.npad : 1)));
         TF_TRY(ensure(c, c->sell_halo[id], (size_t)blocks * kHaloMax + blocks));
         S.col_tr = c->sell_coltr[id].p;
-        S.halo_rows = c->sell_halo[id].p;
+        S.halo_slots = c->sell_halo[id].p;
         S.halo_n = c->sell_halo[id].p + (size_t)blocks * kHaloMax;
         TF_TRY(ensure(c, c->kry_iters, 4));
         TF_CUDA(c, cudaMemsetAsync(c->kry_iters.p, 0, 4 * sizeof(int), c->stream));
-        const size_t hsm = 2 * sizeof(int32_t) * kHashSlots;
+        const size_t hsm = sizeof(int32_t) * (kHashSlots + kHaloMax);
         TF_CUDA(c, cudaFuncSetAttribute((const void*)k_res_halo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
-        k_res_halo<<<blocks, 512, hsm, c->stream>>>(S.ptr, S.nslices, S.col, S.iperm, S.col_tr, S.halo_rows, S.halo_n,
+        k_res_halo<<<blocks, 512, hsm, c->stream>>>(S.ptr, S.nslices, S.col, S.iperm, S.col_tr, S.halo_slots, S.halo_n,
                                                     c->kry_iters.p);
         ++c->launches;
         TF_CUDA(c, cudaGetLastError());
@@ -789,23 +792,24 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kResThreads, dyn));
     if (per_sm < 1) return TF_OK;
 
-    // workspace: V0, V1 (m states each), p (m), T diagonal (m)
+    // workspace: V0, V1 (a state per slot each), p (per slot), T diagonal (m)
+    const int64_t ns = S.nslices * 32;
     const T* diag = nullptr;
     V* V0 = nullptr;
     T* P = nullptr;
     if constexpr (sizeof(T) == 4) {
-        TF_TRY(ensure(c, c->kry32, (size_t)(10 * m)));
+        TF_TRY(ensure(c, c->kry32, (size_t)(9 * ns + m)));
         float* base = c->kry32.p;
-        k_res_diag32<<<grid_for(c, m), kBlock, 0, c->stream>>>(m, A.diag, base + 9 * m);
+        k_res_diag32<<<grid_for(c, m), kBlock, 0, c->stream>>>(m, A.diag, base + 9 * ns);
         ++c->launches;
         V0 = reinterpret_cast<V*>(base);
-        P = base + 8 * m;
-        diag = base + 9 * m;
+        P = base + 8 * ns;
+        diag = base + 9 * ns;
     } else {
-        TF_TRY(ensure(c, c->kry64, (size_t)(9 * m)));
+        TF_TRY(ensure(c, c->kry64, (size_t)(9 * ns)));
         double* base = c->kry64.p;
         V0 = reinterpret_cast<V*>(base);
-        P = base + 8 * m;
+        P = base + 8 * ns;
         diag = A.diag;
     }
     const size_t part_d = (size_t)2 * blocks * kArMax;
@@ -825,7 +829,7 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     g.ptr = S.ptr;
     g.col = S.col;
     g.col_tr = S.col_tr;
-    g.halo_rows = S.halo_rows;
+    g.halo_slots = S.halo_slots;
     g.halo_n = S.halo_n;
     if constexpr (sizeof(T) == 4) g.val = S.v32;
     else g.val = S.v64;
@@ -834,7 +838,7 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     g.b = b;
     g.x = x;
     g.V0 = V0;
-    g.V1 = V0 + m;
+    g.V1 = V0 + ns;
     g.P = P;
     g.g.count = reinterpret_cast<unsigned long long*>(c->kry_bar.p);
     g.g.partd = c->kry_part.p;
@@ -892,7 +896,7 @@ int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter
     int per_sm = 0;
     TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kResThreads, dyn));
     if (per_sm < 1) return TF_OK;
-    TF_TRY(ensure(c, c->kry64, (size_t)m));
+    TF_TRY(ensure(c, c->kry64, (size_t)(S.nslices * 32)));
     const size_t part_d = (size_t)2 * blocks * kArMax;
     TF_TRY(ensure(c, c->kry_part, part_d + 16));
     TF_TRY(ensure(c, c->kry_bar, 2));
@@ -910,7 +914,7 @@ int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter
     g.perm = S.perm;
     g.ptr = S.ptr;
     g.col_tr = S.col_tr;
-    g.halo_rows = S.halo_rows;
+    g.halo_slots = S.halo_slots;
     g.halo_n = S.halo_n;
     g.val = S.v64;
     g.diag = A.diag;

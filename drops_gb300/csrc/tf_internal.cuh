@@ -231,7 +231,7 @@ struct Sell {
     int32_t* iperm = nullptr;
     int64_t iperm_gen = -1;
     uint16_t* col_tr = nullptr;
-    int32_t* halo_rows = nullptr;  // [block][halo capacity]
+    int32_t* halo_slots = nullptr;  // [block][halo capacity]
     int32_t* halo_n = nullptr;     // [block]
     int res_blocks = 0, res_smax = 0, res_hmax = 0;
     int32_t res_maxslots = 0;
