@@ -20,6 +20,7 @@
 // segmented sum over contributions sorted by (row, column, tet), i.e. in the
 // reference's triangulation-order accumulation, without atomics.
 #include <climits>
+#include <cstring>
 
 #include <cub/device/device_radix_sort.cuh>
 
@@ -842,60 +843,138 @@ __global__ void k_row_counts(int64_t n_active, int nl, const int32_t* __restrict
     }
 }
 
-__global__ void k_bucket(int64_t n_active, int nl, const int32_t* __restrict__ l2g, const uint8_t* __restrict__ mask,
+// One thread per (tet, local row): it reserves the row's places for all its
+// columns with one atomic and writes them next to each other.
+template <int NL>
+__global__ void k_bucket(int64_t n_active, const int32_t* __restrict__ l2g, const uint8_t* __restrict__ mask,
                          const int32_t* __restrict__ start, int32_t* __restrict__ cursor, uint64_t* __restrict__ contrib) {
-    const int nl2 = nl * nl;
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n_active * nl2;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = c / nl2;
-        const int ij = (int)(c - r * nl2);
-        const int i = ij / nl, j = ij - (ij / nl) * nl;
-        const int32_t row = l2g[r * nl + i], col = l2g[r * nl + j];
-        if (row < 0 || col < 0 || (mask && !mask[r])) continue;
-        const int32_t pos = start[row] + atomicAdd(&cursor[row], 1);
-        contrib[pos] = ((uint64_t)(uint32_t)col << 32) | (uint64_t)(uint32_t)c;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n_active * NL;
+         q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = q / NL;
+        const int i = (int)(q - r * NL);
+        const int32_t row = l2g[q];
+        if (row < 0 || (mask && !mask[r])) continue;
+        int32_t col[NL];
+        int nc = 0;
+#pragma unroll
+        for (int j = 0; j < NL; ++j) {
+            col[j] = l2g[r * NL + j];
+            nc += col[j] >= 0;
+        }
+        int32_t pos = start[row] + atomicAdd(&cursor[row], nc);
+        const uint32_t c0 = (uint32_t)(r * (NL * NL) + i * NL);
+#pragma unroll
+        for (int j = 0; j < NL; ++j)
+            if (col[j] >= 0) contrib[pos++] = ((uint64_t)(uint32_t)col[j] << 32) | (uint64_t)(c0 + j);
     }
 }
 
-// warp per row: bitonic sort of the row's keys in shared memory, unique count
-__global__ void k_row_sort(int64_t m, const int32_t* __restrict__ start, uint64_t* __restrict__ contrib,
-                           int32_t* __restrict__ ucnt, int* __restrict__ status) {
+// Bitonic sort of 32 K keys in registers, key lane * K + k in a[k] of `lane`:
+// strides below K stay inside a lane, the other 15 stages are shuffles.
+template <int K>
+__device__ __forceinline__ void warp_sort(uint64_t (&a)[K], int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32 * K; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= K) {
+                const int x = stride / K;
+                const bool keep_min = ((lane & x) == 0) == (((lane * K) & size) == 0);
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const uint64_t o = __shfl_xor_sync(0xffffffffu, a[k], x);
+                    a[k] = keep_min == (a[k] < o) ? a[k] : o;
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    if ((k & stride) == 0) {
+                        const bool up = size < K ? (k & size) == 0 : ((lane * K) & size) == 0;
+                        const uint64_t u = a[k], v = a[k | stride];
+                        const bool sw = (u > v) == up;
+                        a[k] = sw ? v : u;
+                        a[k | stride] = sw ? u : v;
+                    }
+            }
+        }
+    }
+}
+// n <= 32 K keys at p sorted in place; returns the number of distinct columns (high words)
+template <int K>
+__device__ __forceinline__ int row_sort_regs(uint64_t* __restrict__ p, int n, int lane) {
+    uint64_t a[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) a[k] = lane * K + k < n ? p[lane * K + k] : ~0ull;
+    warp_sort<K>(a, lane);
+    uint32_t prev = __shfl_up_sync(0xffffffffu, (uint32_t)(a[K - 1] >> 32), 1);
+    int u = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const uint32_t col = (uint32_t)(a[k] >> 32);
+        if (lane * K + k < n) {
+            p[lane * K + k] = a[k];
+            u += (lane * K + k == 0) || col != prev;
+        }
+        prev = col;
+    }
+    return __reduce_add_sync(0xffffffffu, u);
+}
+
+// Warp per row: the row's keys sorted (up to 256 in registers, up to kRowCap in
+// shared memory), distinct columns counted.  Bound: instruction issue and the
+// latency of one row per warp.  One warp used to take 32 rows one after the
+// other, all in shared memory: at 96^3 P2 (146,042 rows, 49 keys in the mean)
+// 476 -> 100 us, at 16^3 P1 (664 rows) 160 -> 4.4 us.
+__global__ void __launch_bounds__(128) k_row_sort(int64_t m, const int32_t* __restrict__ start,
+                                                  uint64_t* __restrict__ contrib, int32_t* __restrict__ ucnt,
+                                                  int* __restrict__ status) {
     __shared__ uint64_t buf[4][kRowCap];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint64_t* b = buf[wib];
     for (int64_t row = (int64_t)blockIdx.x * 4 + wib; row < m; row += (int64_t)gridDim.x * 4) {
-        const int32_t s = start[row], n = start[row + 1] - start[row];
+        const int32_t s = start[row], n = start[row + 1] - s;
+        uint64_t* p = contrib + s;
+        int u = 0;
         if (n > kRowCap) {
             if (lane == 0) set_status(status, TF_ERR_CAPACITY, row);
             continue;
         }
-        int np = 1;
-        while (np < n) np <<= 1;
-        for (int k = lane; k < np; k += 32) b[k] = k < n ? contrib[s + k] : ~0ull;
-        __syncwarp();
-        for (int size = 2; size <= np; size <<= 1)
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int k = lane; k < np; k += 32) {
-                    const int partner = k ^ stride;
-                    if (partner > k) {
-                        const bool up = (k & size) == 0;
-                        const uint64_t a = b[k], c = b[partner];
-                        if ((a > c) == up) {
-                            b[k] = c;
-                            b[partner] = a;
+        if (n <= 32) {
+            u = row_sort_regs<1>(p, n, lane);
+        } else if (n <= 64) {
+            u = row_sort_regs<2>(p, n, lane);
+        } else if (n <= 128) {
+            u = row_sort_regs<4>(p, n, lane);
+        } else if (n <= 256) {
+            u = row_sort_regs<8>(p, n, lane);
+        } else {
+            uint64_t* b = buf[wib];
+            int np = 512;
+            while (np < n) np <<= 1;
+            for (int k = lane; k < np; k += 32) b[k] = k < n ? p[k] : ~0ull;
+            __syncwarp();
+            for (int size = 2; size <= np; size <<= 1)
+                for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                    for (int k = lane; k < np; k += 32) {
+                        const int partner = k ^ stride;
+                        if (partner > k) {
+                            const bool up = (k & size) == 0;
+                            const uint64_t x = b[k], y = b[partner];
+                            if ((x > y) == up) {
+                                b[k] = y;
+                                b[partner] = x;
+                            }
                         }
                     }
+                    __syncwarp();
                 }
-                __syncwarp();
+            for (int k = lane; k < n; k += 32) {
+                p[k] = b[k];
+                u += (k == 0) || ((b[k] >> 32) != (b[k - 1] >> 32));
             }
-        int u = 0;
-        for (int k = lane; k < n; k += 32) {
-            contrib[s + k] = b[k];
-            u += (k == 0) || ((b[k] >> 32) != (b[k - 1] >> 32));
+            u = __reduce_add_sync(0xffffffffu, u);
+            __syncwarp();
         }
-        for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
         if (lane == 0) ucnt[row] = u;
-        __syncwarp();
     }
 }
 
@@ -904,6 +983,7 @@ __global__ void k_row_emit(int64_t m, const int32_t* __restrict__ start, const u
                            const int32_t* __restrict__ rowptr, int32_t* __restrict__ colind,
                            int32_t* __restrict__ seg_start, int32_t* __restrict__ diag_slot) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && threadIdx.x == 0) seg_start[rowptr[m]] = start[m];
     for (int64_t row = (int64_t)blockIdx.x * 4 + wib; row < m; row += (int64_t)gridDim.x * 4) {
         const int32_t s = start[row], n = start[row + 1] - start[row];
         int32_t carry = rowptr[row];
@@ -981,46 +1061,40 @@ static int build_pattern(Context* c, const uint8_t* mask = nullptr) {
     const int64_t ncontrib = na * nl * nl;
     if (ncontrib >= INT32_MAX) return set_err(c, TF_ERR_CAPACITY, "pattern: too many contributions for 32-bit offsets");
     TimedLaunch tl(c, TF_K_PATTERN);
+    const size_t bytes = sizeof(int32_t) * (size_t)(m + 1);
     TF_TRY(ensure(c, c->row_cursor, (size_t)m + 1));
-    TF_CUDA(c, cudaMemsetAsync(c->row_cursor.p, 0, sizeof(int32_t) * (size_t)(m + 1), c->stream));
+    TF_TRY(ensure(c, c->row_start, (size_t)m + 1));
+    TF_TRY(ensure(c, c->rowptr, (size_t)m + 1));
+    TF_TRY(ensure(c, c->contrib, (size_t)ncontrib + 1));
+    TF_TRY(ensure(c, c->diag_slot, (size_t)(m > 0 ? m : 1)));
+    TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, kStatusWords * sizeof(int), c->stream));
+    TF_CUDA(c, cudaMemsetAsync(c->row_cursor.p, 0, bytes, c->stream));
     k_row_counts<<<grid_for(c, na * nl), kBlock, 0, c->stream>>>(na, nl, c->loc2glo.p, mask, c->row_cursor.p);
     ++c->launches;
-    TF_TRY(ensure(c, c->rowptr, (size_t)m + 1));
-    int64_t total = 0;
-    // bucket starts -> rowptr buffer (temporarily)
-    TF_TRY(exclusive_scan_i32_to_i32(c, c->row_cursor.p, c->rowptr.p, m, &total));
-    TF_CUDA(c, cudaMemsetAsync(c->row_cursor.p, 0, sizeof(int32_t) * (size_t)(m + 1), c->stream));
-    TF_TRY(ensure(c, c->contrib, (size_t)ncontrib + 1));
-    k_bucket<<<grid_for(c, ncontrib), kBlock, 0, c->stream>>>(na, nl, c->loc2glo.p, mask, c->rowptr.p, c->row_cursor.p,
-                                                              c->contrib.p);
-    ++c->launches;
-    TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
-    // unique counts into row_cursor
-    k_row_sort<<<grid_for(c, m, 128, 16), 128, 0, c->stream>>>(m, c->rowptr.p, c->contrib.p, c->row_cursor.p,
-                                                                 c->status.p);
-    ++c->launches;
-    TF_CUDA(c, cudaGetLastError());
+    TF_TRY(exclusive_scan_i32_status(c, c->row_cursor.p, c->row_start.p, m));  // starts of the rows' contributions
+    TF_CUDA(c, cudaMemsetAsync(c->row_cursor.p, 0, bytes, c->stream));
+    if (nl == 10)
+        k_bucket<10><<<grid_for(c, na * nl), kBlock, 0, c->stream>>>(na, c->loc2glo.p, mask, c->row_start.p,
+                                                                    c->row_cursor.p, c->contrib.p);
+    else
+        k_bucket<4><<<grid_for(c, na * nl), kBlock, 0, c->stream>>>(na, c->loc2glo.p, mask, c->row_start.p,
+                                                                   c->row_cursor.p, c->contrib.p);
+    // distinct columns per row into row_cursor, then the row pointers
+    k_row_sort<<<grid_for(c, m, 4, 28), 128, 0, c->stream>>>(m, c->row_start.p, c->contrib.p, c->row_cursor.p, c->status.p);
+    c->launches += 2;
+    TF_TRY(exclusive_scan_i32_status(c, c->row_cursor.p, c->rowptr.p, m));
     int st = 0;
     TF_TRY(sync_status(c, &st));
     if (st) return set_err(c, st, "pattern: a matrix row has more than 1024 element contributions");
-    // keep bucket starts in seg_start's tail? copy them to a separate array
-    DBuf<int32_t> bstart;
-    TF_TRY(ensure(c, bstart, (size_t)m + 1));
-    TF_CUDA(c, cudaMemcpyAsync(bstart.p, c->rowptr.p, sizeof(int32_t) * (size_t)(m + 1), cudaMemcpyDeviceToDevice,
-                               c->stream));
     int64_t nnz = 0;
-    TF_TRY(exclusive_scan_i32_to_i32(c, c->row_cursor.p, c->rowptr.p, m, &nnz));
+    std::memcpy(&nnz, c->h_status + 4, sizeof nnz);
+    if (nnz > INT32_MAX) return set_err(c, TF_ERR_CAPACITY, "scan total exceeds int32 range");
     TF_TRY(ensure(c, c->colind, (size_t)(nnz > 0 ? nnz : 1)));
     TF_TRY(ensure(c, c->seg_start, (size_t)nnz + 1));
-    TF_TRY(ensure(c, c->diag_slot, (size_t)(m > 0 ? m : 1)));
     TF_CUDA(c, cudaMemsetAsync(c->diag_slot.p, 0xff, sizeof(int32_t) * (size_t)(m > 0 ? m : 1), c->stream));
-    k_row_emit<<<grid_for(c, m, 128, 16), 128, 0, c->stream>>>(m, bstart.p, c->contrib.p, c->rowptr.p, c->colind.p,
-                                                                 c->seg_start.p, c->diag_slot.p);
+    k_row_emit<<<grid_for(c, m, 4, 64), 128, 0, c->stream>>>(m, c->row_start.p, c->contrib.p, c->rowptr.p, c->colind.p,
+                                                             c->seg_start.p, c->diag_slot.p);
     ++c->launches;
-    int32_t tot32 = (int32_t)total;  // contributions actually bucketed
-    TF_CUDA(c, cudaMemcpyAsync(c->seg_start.p + nnz, &tot32, sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
-    TF_CUDA(c, cudaStreamSynchronize(c->stream));
-    release(bstart);
     TF_CUDA(c, cudaGetLastError());
     const int64_t gen = ++c->pattern_counter;
     for (int f = 0; f < TF_NUM_MATS; ++f) {
@@ -1125,26 +1199,18 @@ int setup_fe_system(Context* c, unsigned forms, int rhs_kind, const double* rhs_
         ++c->launches;
         TF_CUDA(c, cudaGetLastError());
     }
-    int st = 0;
-    TF_TRY(sync_status(c, &st));
-    if (st == TF_ERR_ZERO_PATTERN)
-        return set_err(c, st, "RefPatchCL::instance: found a full body in the zero level set, grid is too coarse");
-    if (st) return set_err(c, st, "assembly failed");
     // values
     double* v[4] = {nullptr, nullptr, nullptr, nullptr};
     const int64_t nnz = c->mats[0].nnz;
     for (int f = 0; f < TF_NUM_FORMS; ++f) {
         if (!(forms & (1u << f))) continue;
         TF_TRY(ensure(c, c->mat_vals[f], (size_t)(nnz > 0 ? nnz : 1)));
-        c->mats[f].vals = c->mat_vals[f].p;
-        ++c->mats[f].version;
-        v[f] = c->mats[f].vals;
+        v[f] = c->mat_vals[f].p;
     }
     double* vN = nullptr;
     if (wantN) {
         TF_TRY(ensure(c, c->mat_vals[TF_FORM_N], (size_t)(nnz > 0 ? nnz : 1)));
-        c->mats[TF_FORM_N].vals = vN = c->mat_vals[TF_FORM_N].p;
-        ++c->mats[TF_FORM_N].version;
+        vN = c->mat_vals[TF_FORM_N].p;
     }
     if (nnz > 0) {
         TimedLaunch tl(c, TF_K_SCATTER);
@@ -1167,7 +1233,18 @@ int setup_fe_system(Context* c, unsigned forms, int rhs_kind, const double* rhs_
         }
         TF_CUDA(c, cudaGetLastError());
     }
-    TF_CUDA(c, cudaStreamSynchronize(c->stream));
+    // one wait for the patches' status and the values
+    int st = 0;
+    TF_TRY(sync_status(c, &st));
+    if (st == TF_ERR_ZERO_PATTERN)
+        return set_err(c, st, "RefPatchCL::instance: found a full body in the zero level set, grid is too coarse");
+    if (st) return set_err(c, st, "assembly failed");
+    for (int f = 0; f < TF_NUM_MATS; ++f) {
+        double* p = f < TF_NUM_FORMS ? v[f] : f == TF_FORM_N ? vN : nullptr;
+        if (!p) continue;
+        c->mats[f].vals = p;
+        ++c->mats[f].version;
+    }
     return TF_OK;
 }
 
@@ -1740,8 +1817,6 @@ __global__ void k_legacy_active(MeshView M, int64_t n_cand, const int32_t* __res
         act_flag[r] = a;
     }
 }
-
-int compact_active(Context* c, int64_t* n_active);
 
 // local-to-global map of the cut tets under the legacy numbering (-1: vertex not numbered)
 __global__ void k_legacy_l2g(MeshView M, int64_t n, const int32_t* __restrict__ tets,

@@ -140,12 +140,12 @@ int tf_create(tf_context** out, int device) {
     if (const char* e = std::getenv("TF_PREP_SORT")) c->prep_sort = std::atoi(e) != 0;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-        cudaMallocHost((void**)&c->h_status, 4 * sizeof(int)) != cudaSuccess ||
-        tf::ensure(c, c->status, 4) != TF_OK) {
+        cudaMallocHost((void**)&c->h_status, (tf::kStatusWords + 8) * sizeof(int)) != cudaSuccess ||
+        tf::ensure(c, c->status, tf::kStatusWords) != TF_OK) {
         delete t;
         return TF_ERR_CUDA;
     }
-    cudaMemset(c->status.p, 0, 4 * sizeof(int));
+    cudaMemset(c->status.p, 0, tf::kStatusWords * sizeof(int));
     // the module must hold code for this device: a first kernel launch tells
     if (tf::ensure_tables(c) != TF_OK || cudaDeviceSynchronize() != cudaSuccess) {
         delete t;
@@ -179,6 +179,7 @@ int tf_destroy(tf_context* t) {
     tf::release(c->colind);
     tf::release(c->seg_start);
     tf::release(c->row_cursor);
+    tf::release(c->row_start);
     tf::release(c->diag_slot);
     tf::release(c->contrib);
     tf::release(c->elem);

@@ -85,12 +85,16 @@ int dof_locality_order(Context* c, const int32_t** order) {
                                                                                    kin);
         c->launches += 2;
         TF_CUDA(c, cudaGetLastError());
+        // only the bits a position of this grid can have: 3 passes instead of 8 up to 127 cubes per side
+        int bits = 21;
+        if (!M.explicit_mesh)
+            for (bits = 1; (1 << bits) <= 2 * std::max({M.b.n1, M.b.n2, M.b.n3}); ++bits) {}
         size_t bytes = 0;
-        TF_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kin + m, rin, c->dof_order.p, (int)m, 0, 63,
+        TF_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kin + m, rin, c->dof_order.p, (int)m, 0, 3 * bits,
                                                   c->stream));
         TF_TRY(ensure(c, c->order_tmp, bytes > 0 ? bytes : 1));
         TF_CUDA(c, cub::DeviceRadixSort::SortPairs(c->order_tmp.p, bytes, kin, kin + m, rin, c->dof_order.p, (int)m, 0,
-                                                  63, c->stream));
+                                                  3 * bits, c->stream));
         c->launches += 4;  // the radix sort's passes
         c->dof_order_version = c->dof_version;
     }

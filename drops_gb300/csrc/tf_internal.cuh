@@ -260,6 +260,8 @@ struct CSR {
     int64_t vals32_version = -1, diag_version = -1;
 };
 
+constexpr int kStatusWords = 8;
+
 struct KernelTimer {
     double total_ms = 0;
     int64_t launches = 0;
@@ -292,11 +294,11 @@ struct Context {
     DBuf<unsigned long long> order_keys;
     DBuf<unsigned char> order_tmp;
     int64_t dof_order_version = -1;
-    DBuf<uint8_t> flags;
+    DBuf<uint8_t> flags;     // classification: activity bits of the tets of one cube (or one tet)
     DBuf<int32_t> keys_v, keys_e, owner;
     // pattern
     int64_t pattern_dof_version = -1;
-    DBuf<int32_t> rowptr, colind, seg_start, row_cursor, diag_slot;
+    DBuf<int32_t> rowptr, colind, seg_start, row_cursor, row_start, diag_slot;
     DBuf<uint64_t> contrib;  // sorted (col << 32 | contribution) per row
     DBuf<double> elem;       // packed element matrices [form][tet][nsym]
     DBuf<double> elem_rhs;   // [tet][nl]
@@ -316,8 +318,8 @@ struct Context {
     // scratch
     DBuf<unsigned char> scratch;
     DBuf<int64_t> scan_tmp;
-    DBuf<int> status;  // device status word(s)
-    int* h_status = nullptr;  // pinned
+    DBuf<int> status;  // device status words: code, where, two counters, a 64-bit total, spare
+    int* h_status = nullptr;  // pinned: the status words, then 8 words of staging
     // timing
     bool timing = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -483,9 +485,11 @@ struct TimedLaunch {
 // device-wide exclusive scan of int32 counts -> int64 offsets (out[n] = total)
 int exclusive_scan_i32(Context* c, const int32_t* in, int64_t* out, int64_t n);
 int exclusive_scan_i32_to_i32(Context* c, const int32_t* in, int32_t* out, int64_t n, int64_t* total);
+int exclusive_scan_i32_status(Context* c, const int32_t* in, int32_t* out, int64_t n);
 // *order: the rows of the current DistributeDOFs numbering in Morton order of
 // their nodes, or nullptr where there is none (explicit or batch meshes)
 int dof_locality_order(Context* c, const int32_t** order);
+// fetches the status words (kStatusWords) into h_status and waits
 int sync_status(Context* c, int* status_out);
 int fill_f64(Context* c, double* p, int64_t n, double v);
 
