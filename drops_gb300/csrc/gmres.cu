@@ -53,7 +53,7 @@ namespace {
 constexpr int kLsThreads = 512;
 constexpr int kLsWarps = kLsThreads / 32;
 constexpr int kLsMaxR = 64;                 // restart length
-constexpr int kLsVals = 2 * kLsMaxR + 8;    // values of one reduction, per block
+constexpr int kLsVals = 2 * kLsMaxR + 8;    // values of one reduction, per block (at most 2 R)
 
 template <class V>
 struct GmLsArgs {
@@ -92,12 +92,13 @@ struct LsSmall {  // least-squares state, identical in every block
     V hp[4][kLsMaxR];        // parts of L a
     V rc[kLsMaxR], rs[kLsMaxR], rt[kLsMaxR];
     V pd[kLsWarps * 8];      // dots of one warp each
+    V pw[kLsWarps];          // |w|^2 of one warp each
     V grp[kLsThreads];       // partial sums of the reduction
     V hlast;                 // last entry of the rotated column before the new rotation
     double resid, normb, beta;
     int flag;
     int lmax;                // largest |L_kj| of the cycle (bits of a float)
-    int amax, Ew;            // largest |<w, v_k>| of the step (bits), exponent of the last |w|
+    int Ew;                  // exponent of the last |w| before its projection
 };
 
 __device__ __forceinline__ float ls_add(const float (&p)[16]) {
@@ -109,6 +110,12 @@ __device__ __forceinline__ float ls_add(const float (&p)[16]) {
 __device__ __forceinline__ double ls_add(const double (&p)[16]) { return fx_sum(p); }
 __device__ __forceinline__ float ls_sum8(const float (&v)[8], int lane) { return warp_sum8(v, lane); }
 __device__ __forceinline__ double ls_sum8(const double (&v)[8], int lane) { return warp_fx_sum8(v, lane); }
+
+__device__ __forceinline__ float ls_sum1(float v) { return warp_sum(v); }
+__device__ __forceinline__ double ls_sum1(double v) {
+    const double one[1] = {v};
+    return warp_fx_sum(one);
+}
 
 // 1 / sqrt(x): FP64 from an FP32 seed and two Newton steps (relative error
 // about 2^-52; a square root and a division are 1,200 cycles of the FP64 pipe
@@ -188,10 +195,9 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
 
     PkState pkn;
     unsigned pepoch = 0;
-    unsigned long long plast[4] = {0ull, 0ull, 0ull, 0ull};
+    unsigned long long plast[2] = {0ull, 0ull}, plast2[2] = {0ull, 0ull};
     if (threadIdx.x == 0) {
         q.Ew = kPkUnknown;
-        q.amax = 0;
     }
     bool first = true;
     for (;;) {
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                 const int groups = (i + 4) >> 2, parts = kLsWarps / groups;
                 const int grp = warp % groups, pt = warp / groups;
                 if (pt < parts) {
-                    V d[8];
+                    V d[8], dw = V(0);
 #pragma unroll
                     for (int u = 0; u < 8; ++u) d[u] = V(0);
                     const V* vk[4];
@@ -285,6 +291,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
 #pragma unroll 2
                     for (int e = pt * 32 + lane; e < nl; e += 32 * parts) {
                         const V we = wl[e], ve = vl[e];
+                        if (grp == 0) dw += we * we;
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
                             if (u < nk) {
@@ -295,57 +302,61 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                     }
                     const V tot = ls_sum8(d, lane);
                     if ((lane & 3) == 0) q.pd[warp * 8 + warp_sum8_index(lane)] = tot;
+                    if (grp == 0) {
+                        const V t = ls_sum1(dw);
+                        if (lane == 0) q.pw[pt] = t;
+                    }
                 }
                 __syncthreads();
-                // thread j < 2 i + 1: <w, v_j> (j <= i), then <v_i, v_k>, over the block; one word of a packed
-                // reduction per value (two in FP64), its unit from |w| of the step before (1 for <v_i, v_k>)
-                const int n = 2 * i + 1, j = threadIdx.x;
+                // thread j: <w, v_j> (j <= i), <v_i, v_k> (i of them), then |w|^2, over the block; a packed
+                // reduction, the unit of each from |w| of the step before (1 for <v_i, v_k>)
+                const int n = 2 * i + 2, j = threadIdx.x;
                 V sum = V(0);
-                if (j < n) {
+                if (j < n - 1) {
                     const int u = j <= i ? 0 : 4, k = j <= i ? j : j - i - 1;
                     const V* p = q.pd + (k >> 2) * 8 + u + (k & 3);
                     sum = p[0];
                     for (int t = 1; t < parts; ++t) sum += p[t * groups * 8];
                     sum *= q.scl[k];
                     if (j > i) sum *= sci;
+                } else if (j == n - 1) {
+                    sum = q.pw[0];
+                    for (int t = 1; t < parts; ++t) sum += q.pw[t];
                 }
                 int st = 1;
                 const int Ew = q.Ew;
                 if (Ew != kPkUnknown) {
                     st = 0;
                     if (j < n) {
-                        const int E = j <= i ? Ew : 0;
-                        const int odd = pepoch & 1;
+                        const int E = j <= i ? Ew : j < n - 1 ? 0 : 2 * Ew + 1;
+                        V val;
                         if constexpr (kMixed) {
-                            unsigned long long* w = a.pkd.w + odd * kPkWords + j;
                             bool bad;
                             const long long t = pk_fix(sum, E, &bad);
-                            red_relaxed_add_u64(w, pk_word(t, bad));
                             unsigned long long diff = 0;
-                            if (!pk_wait(w, odd ? plast[1] : plast[0], a.pkd.status, &diff)) st = 2;
-                            else if (pk_misfit(diff)) st = 1;
-                            q.tot[j] = pk_value(pk_sum(diff), E);
+                            st = pk_exchange(a.pkd, pepoch, plast, j, t, !bad, &diff);
+                            val = pk_value(pk_sum(diff), E);
                         } else {
-                            unsigned long long* w = a.pkd.w + odd * kPkWords + 2 * j;
                             bool bad;
                             long long hi, lo;
                             pk_fix(sum, E, &hi, &lo, &bad);
-                            if (!pk_carry(&hi, &lo)) bad = true;
-                            red_relaxed_add_u64(w, pk_word(hi, bad));
-                            red_relaxed_add_u64(w + 1, pk_word(lo, bad));
+                            const bool fits = pk_carry(&hi, &lo) && !bad;
+                            unsigned long long* w = a.pkd.w + (pepoch & 1) * kPkWords + 2 * j;
+                            red_relaxed_add_u64(w + 1, pk_word(lo, !fits));  // both words on their way before the waits
                             unsigned long long dh = 0, dl = 0;
-                            if (!pk_wait(w, odd ? plast[1] : plast[0], a.pkd.status, &dh) ||
-                                !pk_wait(w + 1, odd ? plast[3] : plast[2], a.pkd.status, &dl))
-                                st = 2;
-                            else if (pk_misfit(dh)) st = 1;
-                            q.tot[j] = pk_value(pk_sum(dh), (long long)(dl >> 16), E);
+                            st = pk_exchange(a.pkd, pepoch, plast, 2 * j, hi, fits, &dh);
+                            if (!pk_wait(w + 1, pepoch & 1 ? plast2[1] : plast2[0], a.pkd.status, &dl)) st = 2;
+                            val = pk_value(pk_sum(dh), (long long)(dl >> 16), E);
                         }
+                        q.tot[j] = val;
+                        // |w| far below the unit's: the dots would lack bits
+                        if (j == n - 1 && pk_exp(val) < E - 2 * (kMixed ? kPkDrop32 : kPkDrop64)) st = max(st, 1);
                     }
                     ++pepoch;
                     if (__syncthreads_or(st == 2)) return;
                     st = __syncthreads_or(st);
                 }
-                if (st) {  // no |w| yet, or a value beyond the range of its unit
+                if (st) {  // no |w| yet, or a value outside the range of its unit
                     if (j < n) a.part[((size_t)(epoch & 1) * gridDim.x + blockIdx.x) * kLsVals + j] = sum;
                     if (!reduce(n)) return;
                 }
@@ -355,7 +366,6 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
             if ((int)threadIdx.x <= i) {
                 const int k = threadIdx.x;
                 q.aw[k] = q.tot[k];
-                atomicMax(&q.amax, __float_as_int(fabsf((float)q.tot[k])));
                 if (k < i) {
                     const V l = q.tot[i + 1 + k];
                     q.L[k][i] = l;
@@ -449,8 +459,8 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                     const bool zero = n2 == V(0);
                     const V c = zero ? V(1) : t * ir, s = zero ? V(0) : hn * ir;
                     q.scl[i + 1] = ih;
-                    q.Ew = pk_exp(fmaxf(__int_as_float(q.amax), fabsf((float)hn)));
-                    q.amax = 0;
+                    const int e2 = pk_exp(q.tot[2 * i + 1]);
+                    q.Ew = e2 == kPkUnknown ? kPkUnknown : e2 >> 1;
                     q.cs[i] = c;
                     q.sn[i] = s;
                     q.H[i][i] = c * t + s * hn;

@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
         } else {
             auto& sh = *reinterpret_cast<BalShared<NW, Pair2>*>(raw);
             sell_block_plan<NW, Pair2>(sh, ptr, c0, S);
-            sell_block_walk_fn<NW, Pair2>(
+            sell_block_walk_fn(
                 sh, c0, S,
                 [&](int64_t s, int32_t cc, int32_t n) {
                     const int32_t p0 = __ldg(ptr + s) + 32 * cc;

@@ -513,20 +513,22 @@ __device__ bool grid_allreduce(const GridAR& g, unsigned long long& epoch, const
 // arrivals whose partial did not fit, bits 16..63 hold the sum.  A block that
 // polls the word sees the finished sum with the last arrival: one atomic add
 // and one poll.  Integer sums do not depend on the order of arrival, so every
-// block gets the same bits.  The unit of a value follows from its previous sum
-// (2^30 units for FP32, 2^67 in two words for FP64: 48-bit high part, 40-bit
-// low part), which all blocks know; a partial beyond 2^9 (FP32) or 2^12 (FP64)
-// times that sum, or one that is not finite, is flagged, and all blocks repeat
-// the reduction with grid_allreduce.  FP32 sums keep 6 bits below FP32's own,
-// FP64 sums 14.
+// block gets the same bits.  The unit of a value follows from its previous sum,
+// which all blocks know: an FP32 value takes one word with 2^34 units to that
+// sum, an FP64 value two (a 48-bit high and a 40-bit low part) with 2^67.  The
+// blocks repeat the reduction with grid_allreduce when a partial exceeds the
+// previous sum 2^5 (2^12) times or is not finite, and when the sum is smaller
+// than 2^-10 (2^-14) of it, so that no sum has fewer bits than its type holds.
+// (Without the second condition a GMRES basis vector a thousand times shorter
+// than the one before lost its norm, and the solver stagnated.)
 //
 // Words are never reset: two buffers alternate, and a block remembers the value
 // each of its words had when it last read it (a block is at most one reduction
 // ahead of a reader).  Grids of up to 255 blocks.
 //
-// Measured on GB300, 152 blocks of 512 threads, per reduction: 6 FP32 values
-// 2.70 -> 0.93 us (1.26 with the fence that publishes other data), 2 FP64 values
-// 3.63 us with grid_allreduce.
+// Measured on GB300, 152 blocks of 512 threads, per reduction of 6 words: 2.70
+// (grid_allreduce of 6 FP32 values) -> 0.93 us, 1.26 us with the fence that
+// publishes other data; grid_allreduce of 2 FP64 values takes 3.63 us.
 // ---------------------------------------------------------------------------
 constexpr int kPkWords = 256;  // words of one buffer
 constexpr int kPkMaxBlocks = 255;
@@ -571,16 +573,6 @@ __device__ __forceinline__ int pk_exp(double x) {
     const int e = __double2hiint(x) >> 20 & 0x7ff;
     return e == 0 || e == 2047 ? kPkUnknown : e - 1023;
 }
-// x in units of 2^(E - 30), rounded to nearest; *bad when it exceeds 2^39 units
-__device__ __forceinline__ long long pk_fix(float x, int E, bool* bad) {
-    const int b = __float_as_int(x), e = b >> 23 & 0xff;
-    const long long m = (b & 0x7fffff) | (e ? 0x800000 : 0);
-    const int s = max(e, 1) - 150 - E + 30;  // m 2^(e - 150) in units of 2^(E - 30)
-    *bad = e == 255 || s > 15;
-    const long long t = s >= 0 ? m << min(s, 15) : (s > -40 ? (m + ((1ll << -s) >> 1)) >> -s : 0ll);
-    return b < 0 ? -t : t;
-}
-__device__ __forceinline__ float pk_value(long long t, int E) { return ldexpf(__ll2float_rn(t), E - 30); }
 // x in units of 2^(E - 67) as hi 2^40 + lo (both with the sign of x); *bad when it exceeds 2^87 units
 __device__ __forceinline__ void pk_fix(double x, int E, long long* hi, long long* lo, bool* bad) {
     const long long b = __double_as_longlong(x);
@@ -600,34 +592,61 @@ __device__ __forceinline__ bool pk_carry(long long* hi, long long* lo) {
     *lo &= 0xffffffffffll;
     return *hi < (1ll << 39) && *hi > -(1ll << 39);
 }
-__device__ __forceinline__ double pk_value(long long hi, long long lo, int E) {
-    __int128 t = ((__int128)hi << 40) + lo;
-    const bool neg = t < 0;
-    unsigned __int128 u = neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
-    int k = 0;
+// x in units of 2^(E - 34), rounded to nearest; *bad when it exceeds 2^39 units
+__device__ __forceinline__ long long pk_fix(float x, int E, bool* bad) {
+    const int b = __float_as_int(x), e = b >> 23 & 0xff;
+    const long long m = (b & 0x7fffff) | (e ? 0x800000 : 0);
+    const int s = max(e, 1) - 150 - E + 34;  // m 2^(e - 150)
+    *bad = e == 255 || s > 15;
+    const long long t = s >= 0 ? m << min(s, 15) : (s > -40 ? (m + ((1ll << -s) >> 1)) >> -s : 0ll);
+    return b < 0 ? -t : t;
+}
+__device__ __forceinline__ float pk_value(long long t, int E) { return ldexpf(__ll2float_rn(t), E - 34); }
+constexpr int kPkDrop32 = 10, kPkDrop64 = 14;  // exponents a sum may fall below the previous one
+
+// hi 2^40 + lo as a 62-bit magnitude and a shift
+__device__ __forceinline__ unsigned long long pk_magnitude(long long hi, long long lo, bool* neg, int* shift) {
+    const __int128 t = ((__int128)hi << 40) + lo;
+    *neg = t < 0;
+    unsigned __int128 u = *neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
+    *shift = 0;
     const unsigned long long top = (unsigned long long)(u >> 62);  // |t| < 2^96
     if (top) {
-        k = 64 - __clzll((long long)top);
-        u >>= k;
+        *shift = 64 - __clzll((long long)top);
+        u >>= *shift;
     }
-    const double d = fx_value((long long)(unsigned long long)u, (unsigned)(E - 67 + k + 1075 + 4096) , 4096);
+    return (unsigned long long)u;
+}
+__device__ __forceinline__ double pk_value(long long hi, long long lo, int E) {
+    bool neg;
+    int k;
+    const unsigned long long u = pk_magnitude(hi, lo, &neg, &k);
+    const double d = fx_value((long long)u, (unsigned)(E - 67 + k + 1075 + 4096), 4096);
     return neg ? -d : d;
 }
 
-// per-thread state of the packed reductions of one set of values (warp 0: lane
-// k serves value k, or word k of the FP64 values)
+// per-thread state of the packed reductions of one set of values
 struct PkState {
     unsigned long long last[2] = {0ull, 0ull};
-    int E = kPkUnknown;
+    int E = kPkUnknown;  // lane k (FP32), lanes 2 k and 2 k + 1 (FP64): exponent of value k's last sum
     unsigned epoch = 0;
     bool known = false;  // uniform over the grid
 };
+// one word of a reduction: adds, waits; 0: *diff holds what the blocks added, 1: to be repeated, 2: watchdog
+__device__ __forceinline__ int pk_exchange(const PackedAR& g, unsigned epoch, unsigned long long (&last)[2], int word,
+                                           long long t, bool fits, unsigned long long* diff) {
+    unsigned long long* p = g.w + (epoch & 1) * kPkWords + word;
+    red_relaxed_add_u64(p, pk_word(t, !fits));
+    if (!pk_wait(p, epoch & 1 ? last[1] : last[0], g.status, diff)) return 2;
+    return pk_misfit(*diff) ? 1 : 0;
+}
 
 // Sums of NV <= 8 values over the grid, as grid_allreduce.  publish: the
 // blocks' earlier writes are visible to every block afterwards.
 template <int NV>
 __device__ bool packed_allreduce(const PackedAR& g, PkState& pk, const GridAR& slow, unsigned long long& slow_epoch,
                                  const float (&v)[NV], float (&out)[NV], bool publish) {
+    static_assert(NV <= 8, "two words per value");
     __shared__ float red[NV][32];
     __shared__ float res[NV];
     __shared__ int state;  // 0: done, 1: repeat, 2: watchdog
@@ -649,21 +668,18 @@ __device__ bool packed_allreduce(const PackedAR& g, PkState& pk, const GridAR& s
                 for (int ww = 0; ww < nw; ++ww) x += red[lane][ww];
             if (publish) __threadfence();
             if (lane < NV) {
-                unsigned long long* p = g.w + (pk.epoch & 1) * kPkWords + lane;
                 bool bad;
                 const long long t = pk_fix(x, pk.E, &bad);
-                red_relaxed_add_u64(p, pk_word(t, bad));
                 unsigned long long diff = 0;
-                if (!pk_wait(p, pk.epoch & 1 ? pk.last[1] : pk.last[0], g.status, &diff)) st = 2;
-                else if (pk_misfit(diff)) st = 1;
+                st = pk_exchange(g, pk.epoch, pk.last, lane, t, !bad, &diff);
                 x = pk_value(pk_sum(diff), pk.E);
                 res[lane] = x;
                 const int e = pk_exp(x);
-                if (e == kPkUnknown) st = max(st, x == 0.f ? 0 : 1);
-                else pk.E = e;
+                if (e < pk.E - kPkDrop32) st = max(st, 1);
+                pk.E = e;
             }
             if (publish) fence_acquire_gpu();
-            st = __reduce_max_sync(0xffffffffu, st);
+            st = (int)__reduce_max_sync(0xffffffffu, (unsigned)st);
             if (lane == 0) state = st;
         }
         ++pk.epoch;
@@ -723,7 +739,6 @@ __device__ bool packed_allreduce(const PackedAR& g, PkState& pk, const GridAR& s
         if (lane == 0) redb[w] = bad;
         __syncthreads();
         if (w == 0) {
-            int st = 0;
             long long t = 0;
             bool fits = !__any_sync(0xffffffffu, lane < nw && redb[lane]);
 #pragma unroll
@@ -738,26 +753,25 @@ __device__ bool packed_allreduce(const PackedAR& g, PkState& pk, const GridAR& s
                     fits &= f;
                 }
             }
+            int st = 0;
             if (publish) __threadfence();
             long long s = 0;
             if (lane < 2 * NV) {
-                unsigned long long* p = g.w + (pk.epoch & 1) * kPkWords + lane;
-                red_relaxed_add_u64(p, pk_word(t, !fits));
                 unsigned long long diff = 0;
-                if (!pk_wait(p, pk.epoch & 1 ? pk.last[1] : pk.last[0], g.status, &diff)) st = 2;
-                else if (pk_misfit(diff)) st = 1;
+                st = pk_exchange(g, pk.epoch, pk.last, lane, t, fits, &diff);
                 s = lane & 1 ? (long long)(diff >> 16) : pk_sum(diff);  // low parts are not negative
             }
             const long long lo = __shfl_down_sync(0xffffffffu, s, 1);
             if (lane < 2 * NV && !(lane & 1)) {
                 const double x = pk_value(s, lo, pk.E);
                 const int e = pk_exp(x);
-                if (e != kPkUnknown) pk.E = e;
+                if (e < pk.E - kPkDrop64) st = max(st, 1);
+                pk.E = e;
                 res[lane >> 1] = x;
-                sE[lane >> 1] = pk.E;
+                sE[lane >> 1] = e;
             }
             if (publish) fence_acquire_gpu();
-            st = __reduce_max_sync(0xffffffffu, st);
+            st = (int)__reduce_max_sync(0xffffffffu, (unsigned)st);
             if (lane == 0) state = st;
         }
         ++pk.epoch;
@@ -905,9 +919,9 @@ __device__ __forceinline__ int64_t balanced_part_start(const int32_t* __restrict
     return lo;
 }
 
-template <int NW, class T>
+template <int NW, class T, int MAXS = kBalMaxSlices>
 struct BalShared {
-    int32_t P[kBalMaxSlices + 1];
+    int32_t P[MAXS + 1];
     T tail[NW][32];
 };
 
@@ -938,8 +952,8 @@ __device__ __forceinline__ void sell_block_plan(BalShared<NW, T>& sh, const int3
 // The product over planned slices (sh.P holds the prefix of [s0, s0 + S)):
 // row(slice, c0, n) returns one lane's partial sum over the slice columns
 // [c0, c0 + n); T needs T(0) and +.
-template <int NW, class T, class ROW, class EMIT>
-__device__ __forceinline__ void sell_block_walk_fn(BalShared<NW, T>& sh, int64_t s0, int S, ROW row, EMIT emit) {
+template <int NW, class T, int MAXS, class ROW, class EMIT>
+__device__ __forceinline__ void sell_block_walk_fn(BalShared<NW, T, MAXS>& sh, int64_t s0, int S, ROW row, EMIT emit) {
     const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
     const int32_t Tot = sh.P[S];
     const int32_t g0 = (int32_t)((int64_t)j * Tot / NW), g1 = (int32_t)((int64_t)(j + 1) * Tot / NW);
@@ -990,7 +1004,7 @@ __device__ __forceinline__ void sell_block_walk(BalShared<NW, T>& sh, const int3
                                                 int64_t s0, int S, XL xload, EMIT emit,
                                                 const SellCache<T>& cache = SellCache<T>()) {
     const int lane = threadIdx.x & 31;
-    sell_block_walk_fn<NW, T>(
+    sell_block_walk_fn(
         sh, s0, S,
         [&](int64_t s, int32_t c0, int32_t n) { return sell_row_range<T>(ptr, col, val, s, lane, c0, n, xload, cache); },
         emit);
@@ -1003,6 +1017,34 @@ __device__ __forceinline__ void sell_block_balanced(BalShared<NW, T>& sh, const 
                                                     const SellCache<T>& cache = SellCache<T>()) {
     sell_block_plan<NW, T>(sh, ptr, s0, S);
     sell_block_walk<NW, T>(sh, ptr, col, val, s0, S, xload, emit, cache);
+}
+
+// n columns of one slot row: translated columns cp[32 k] (shared memory),
+// values vp[32 k] (shared memory when vsh, else global), vector xs (shared
+// memory).  The columns and values of the next eight are loaded while the
+// gathers of the current eight are in flight.  Terms are summed in column order.
+template <class T>
+__device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* __restrict__ vp, bool vsh, int32_t n,
+                                     const T* __restrict__ xs) {
+    constexpr int U = 8;
+    T acc = T(0);
+    for (int32_t k = 0; k < n; k += U) {
+        T xv[U], vv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (k + u < n) {
+                vv[u] = vsh ? vp[32 * (k + u)] : __ldg(vp + 32 * (k + u));
+                xv[u] = xs[cp[32 * (k + u)]];
+            } else {
+                vv[u] = T(0);
+                xv[u] = T(0);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u < n) acc += vv[u] * xv[u];
+    }
+    return acc;
 }
 
 #define TF_SLICE_LOOP(nslices, s)                                                    \

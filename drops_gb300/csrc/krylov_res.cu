@@ -95,34 +95,6 @@ __device__ __forceinline__ T res_u(const V& v, T al, T be) {
     return mul_rn(r, v.w);
 }
 
-// n columns of one slot row: translated columns cp[32 k] (shared memory),
-// values vp[32 k] (shared memory when vsh, else global), vector xs (shared
-// memory).  The columns and values of the next eight are loaded while the
-// gathers of the current eight are in flight.  Terms are summed in column order.
-template <class T>
-__device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* __restrict__ vp, bool vsh, int32_t n,
-                                     const T* __restrict__ xs) {
-    constexpr int U = 8;
-    T acc = T(0);
-    for (int32_t k = 0; k < n; k += U) {
-        T xv[U], vv[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (k + u < n) {
-                vv[u] = vsh ? vp[32 * (k + u)] : __ldg(vp + 32 * (k + u));
-                xv[u] = xs[cp[32 * (k + u)]];
-            } else {
-                vv[u] = T(0);
-                xv[u] = T(0);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (k + u < n) acc += vv[u] * xv[u];
-    }
-    return acc;
-}
-
 template <class T>
 struct PcgResArgs {
     using V = typename ResState<T>::V;
@@ -301,7 +273,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
         // the slice offsets of the run come from the plan in shared memory:
         // ptr[sb0 + i] - pb = 32 * bsh.P[i]
         auto walk = [&](auto emit) {
-            sell_block_walk_fn<NW, T>(
+            sell_block_walk_fn(
                 bsh, sb0, S,
                 [&](int64_t s, int32_t c0, int32_t n) {
                     const int i = (int)(s - sb0);
@@ -495,7 +467,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
     // q = A Ps over the run; returns this thread's part of <q, Ps>
     auto walk = [&]() -> double {
         double pq = 0.;
-        sell_block_walk_fn<NW, double>(
+        sell_block_walk_fn(
             bsh, sb0, S,
             [&](int64_t s, int32_t c0, int32_t n) {
                 const int i = (int)(s - sb0);
