@@ -925,6 +925,13 @@ struct BalShared {
     T tail[NW][32];
 };
 
+// A warp's part of the planned columns: slices [lo, hi) of which the first began
+// in warp ja when ja >= 0.
+struct WalkRange {
+    int32_t g0, g1;  // columns
+    int lo, hi, ja;
+};
+
 // The column prefix of the slices [s0, s0 + S) into sh.P (one block
 // barrier); a block that walks the same slices repeatedly plans once.
 template <int NW, class T>
@@ -949,53 +956,88 @@ __device__ __forceinline__ void sell_block_plan(BalShared<NW, T>& sh, const int3
     __syncthreads();
 }
 
-// The product over planned slices (sh.P holds the prefix of [s0, s0 + S)):
-// row(slice, c0, n) returns one lane's partial sum over the slice columns
-// [c0, c0 + n); T needs T(0) and +.
-template <int NW, class T, int MAXS, class ROW, class EMIT>
-__device__ __forceinline__ void sell_block_walk_fn(BalShared<NW, T, MAXS>& sh, int64_t s0, int S, ROW row, EMIT emit) {
-    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+// The part of this thread's warp: binary searches, 0.2 to 0.5 us of shared memory
+// latency, so a block that walks the same slices repeatedly keeps it (in shared
+// memory: a register array of it spills in the resident solvers).
+template <int NW, class T, int MAXS>
+__device__ __forceinline__ WalkRange sell_block_range(const BalShared<NW, T, MAXS>& sh, int S) {
+    const int j = threadIdx.x >> 5;
     const int32_t Tot = sh.P[S];
-    const int32_t g0 = (int32_t)((int64_t)j * Tot / NW), g1 = (int32_t)((int64_t)(j + 1) * Tot / NW);
+    WalkRange r;
+    r.g0 = (int32_t)((int64_t)j * Tot / NW);
+    r.g1 = (int32_t)((int64_t)(j + 1) * Tot / NW);
     // first slice that overlaps [g0, ..) or starts at g0 (zero width included)
     int lo = 0, hi = S;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (sh.P[mid + 1] > g0 || sh.P[mid] >= g0) hi = mid;
+        if (sh.P[mid + 1] > r.g0 || sh.P[mid] >= r.g0) hi = mid;
         else lo = mid + 1;
     }
+    r.lo = lo;
+    // first slice beyond: it starts at g1 or later (the last warp takes the empty slices at the end)
+    hi = S;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (!(sh.P[mid] < r.g1 || (j == NW - 1 && sh.P[mid] == Tot))) hi = mid;
+        else lo = mid + 1;
+    }
+    r.hi = lo;
+    r.ja = -1;
+    if (r.lo < r.hi && sh.P[r.lo] < r.g0) {
+        int ja = j - 1;
+        while (ja > 0 && (int32_t)((int64_t)ja * Tot / NW) > sh.P[r.lo]) --ja;
+        r.ja = ja;
+    }
+    return r;
+}
+
+// The product over planned slices (sh.P holds the prefix of [s0, s0 + S)):
+// row(slice, c0, n) returns one lane's partial sum over the slice columns
+// [c0, c0 + n); T needs T(0) and +.
+template <int NW, class T, int MAXS, class ROW, class EMIT>
+__device__ __forceinline__ void sell_block_walk_range(BalShared<NW, T, MAXS>& sh, int64_t s0, int S, const WalkRange& wr,
+                                                      ROW row, EMIT emit) {
+    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+    const int32_t g0 = wr.g0, g1 = wr.g1;
+    const int lo = wr.lo, hi = wr.hi;
     T head = T(0);
-    int hslice = -1;
-    for (int i = lo; i < S; ++i) {
-        const int32_t pa = sh.P[i], pb = sh.P[i + 1];
-        if (!(pa < g1 || (j == NW - 1 && pa == Tot))) break;
-        const int32_t c0 = g0 > pa ? g0 - pa : 0;
-        const int32_t c1 = (g1 < pb ? g1 : pb) - pa;
-        const T acc = row(s0 + i, c0, c1 > c0 ? c1 - c0 : 0);
-        const bool starts = pa >= g0, ends = pb <= g1;
-        if (starts && ends) {
-            emit(s0 + i, acc);
-        } else if (ends) {
-            head = acc;
-            hslice = i;
-        } else {
-            sh.tail[j][lane] = acc;
+    bool end = false;  // the first slice began in another warp and ends here
+    if (lo < hi) {
+        int32_t pa = sh.P[lo];
+        for (int i = lo; i < hi; ++i) {
+            const int32_t pb = sh.P[i + 1];
+            const int32_t c0 = g0 > pa ? g0 - pa : 0;
+            const int32_t c1 = (g1 < pb ? g1 : pb) - pa;
+            const T acc = row(s0 + i, c0, c1 > c0 ? c1 - c0 : 0);
+            const bool starts = pa >= g0, ends = pb <= g1;
+            if (starts && ends) {
+                emit(s0 + i, acc);
+            } else if (ends) {
+                head = acc;
+                end = true;
+            } else {
+                sh.tail[j][lane] = acc;
+            }
+            pa = pb;
         }
     }
     __syncthreads();
-    if (hslice >= 0) {
+    if (end) {
         // warps from the one holding the slice's first column up to this one
-        const int32_t pa = sh.P[hslice];
-        int ja = j - 1;
-        while (ja > 0 && (int32_t)((int64_t)ja * Tot / NW) > pa) --ja;
+        const int32_t Tot = sh.P[S];
         T sum = T(0);
-        for (int jj = ja; jj < j; ++jj) {
+        for (int jj = wr.ja; jj < j; ++jj) {
             const int32_t a0 = (int32_t)((int64_t)jj * Tot / NW), a1 = (int32_t)((int64_t)(jj + 1) * Tot / NW);
             if (a1 > a0) sum = sum + sh.tail[jj][lane];
         }
-        emit(s0 + hslice, sum + head);
+        emit(s0 + lo, sum + head);
     }
     __syncthreads();  // emits visible to the block; sh.tail free for the next call
+}
+
+template <int NW, class T, int MAXS, class ROW, class EMIT>
+__device__ __forceinline__ void sell_block_walk_fn(BalShared<NW, T, MAXS>& sh, int64_t s0, int S, ROW row, EMIT emit) {
+    sell_block_walk_range(sh, s0, S, sell_block_range(sh, S), row, emit);
 }
 
 template <int NW, class T, class XL, class EMIT>
@@ -1021,8 +1063,7 @@ __device__ __forceinline__ void sell_block_balanced(BalShared<NW, T>& sh, const 
 
 // n columns of one slot row: translated columns cp[32 k] (shared memory),
 // values vp[32 k] (shared memory when vsh, else global), vector xs (shared
-// memory).  The columns and values of the next eight are loaded while the
-// gathers of the current eight are in flight.  Terms are summed in column order.
+// memory).  Terms are summed in column order.
 template <class T>
 __device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* __restrict__ vp, bool vsh, int32_t n,
                                      const T* __restrict__ xs) {

@@ -186,6 +186,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
     }
     sell_block_plan<NW, T>(bsh, a.ptr, sb0, S);
     sell_block_plan<NW, double>(bshd, a.ptr, sb0, S);  // ends with a block barrier
+    __shared__ WalkRange wrs[NW];
+    if (lane == 0) wrs[wid] = sell_block_range(bsh, S);
+    __syncwarp();
 
     const int max_iter = a.max_iter;
     const double tol = a.tol;
@@ -273,8 +276,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
         // the slice offsets of the run come from the plan in shared memory:
         // ptr[sb0 + i] - pb = 32 * bsh.P[i]
         auto walk = [&](auto emit) {
-            sell_block_walk_fn(
-                bsh, sb0, S,
+            sell_block_walk_range(
+                bsh, sb0, S, wrs[wid],
                 [&](int64_t s, int32_t c0, int32_t n) {
                     const int i = (int)(s - sb0);
                     const int32_t p0 = 32 * (bsh.P[i] + c0) + lane;
@@ -464,11 +467,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
         if (k < a.vcap) cval[k] = __ldg(a.val + pb + k);
     }
     sell_block_plan<NW, double>(bsh, a.ptr, sb0, S);  // ends with a block barrier
+    __shared__ WalkRange wrs[NW];
+    if (lane == 0) wrs[threadIdx.x >> 5] = sell_block_range(bsh, S);
+    __syncwarp();
     // q = A Ps over the run; returns this thread's part of <q, Ps>
     auto walk = [&]() -> double {
         double pq = 0.;
-        sell_block_walk_fn(
-            bsh, sb0, S,
+        sell_block_walk_range(
+            bsh, sb0, S, wrs[threadIdx.x >> 5],
             [&](int64_t s, int32_t c0, int32_t n) {
                 const int i = (int)(s - sb0);
                 const int32_t p0 = 32 * (bsh.P[i] + c0) + lane;
