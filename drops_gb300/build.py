@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT, "libtracefem.so")
-UNITS = ["common.cu", "mesh_levelset.cu", "dofs.cu", "assemble.cu", "krylov.cu", "krylov_res.cu", "ch.cu", "capi.cu", "noalloc.cu", "batch.cu", "mlp.cu", "learned.cu", "gmres.cu", "gmres2.cu", "tune.cu", "quaqua.cu", "order.cu", "refine.cu", "refine_par.cu"]
+UNITS = ["common.cu", "mesh_levelset.cu", "dofs.cu", "assemble.cu", "krylov.cu", "krylov_res.cu", "pcg_cluster.cu", "ch.cu", "capi.cu", "noalloc.cu", "batch.cu", "mlp.cu", "learned.cu", "gmres.cu", "gmres2.cu", "tune.cu", "quaqua.cu", "order.cu", "refine.cu", "refine_par.cu"]
 NO_FMA = {"mesh_levelset.cu", "learned.cu", "refine.cu", "refine_par.cu"}
 # host arithmetic that must round like the reference's (no fused multiply-add)
 HOST_NO_CONTRACT = {"refine.cu", "refine_par.cu"}

@@ -547,19 +547,12 @@ static std::vector<int64_t> batch_key(Context* c, const std::vector<int64_t>& nn
     return k;
 }
 
-static int batch_workspace(Context* c, CSR& A, bool mixed) {
+static int batch_workspace(Context* c, CSR& A) {
     const int n = c->batch_count;
     TF_TRY(ensure(c, c->batch_queue, 1));
     TF_TRY(ensure(c, c->batch_iters, (size_t)n));
     TF_TRY(ensure(c, c->batch_resid, (size_t)n));
     TF_TRY(ensure(c, c->batch_order, (size_t)n));
-    if (mixed) {
-        TF_TRY(ensure_csr_f32(c, A));
-        TF_TRY(ensure(c, c->kry32, (size_t)6 * A.m + 1));
-    } else {
-        TF_TRY(ensure(c, c->kry64, (size_t)6 * A.m + 1));
-    }
-    TF_TRY(ensure(c, c->batch_xtmp, (size_t)A.m + 1));
     if (!c->h_batch_out) {
         TF_CUDA(c, cudaMallocHost((void**)&c->h_batch_out, sizeof(double) * 2 * kMaxBatchInstances));
     }
@@ -586,6 +579,17 @@ static int batch_workspace(Context* c, CSR& A, bool mixed) {
     return TF_OK;
 }
 
+// what k_batch_pcg needs besides
+static int batch_lanes_workspace(Context* c, CSR& A, bool mixed) {
+    if (mixed) {
+        TF_TRY(ensure_csr_f32(c, A));
+        TF_TRY(ensure(c, c->kry32, (size_t)6 * A.m + 1));
+    } else {
+        TF_TRY(ensure(c, c->kry64, (size_t)6 * A.m + 1));
+    }
+    return ensure(c, c->batch_xtmp, (size_t)A.m + 1);
+}
+
 static int batch_launch(Context* c, const BatchSetup& s, const double* b, double* x, int max_iter, double tol, int rel) {
     BatchPcgArgs a = s.a;
     a.b = b;
@@ -605,7 +609,8 @@ static int batch_launch(Context* c, const BatchSetup& s, const double* b, double
 // number of iterations (tolerance 0, scratch iterate) and keeps the fastest.
 int batch_tune(Context* c, CSR& A, const double* b, bool mixed, int* lanes_out, int* threads_out) {
     TF_TRY(batch_ranges(c));
-    TF_TRY(batch_workspace(c, A, mixed));
+    TF_TRY(batch_workspace(c, A));
+    TF_TRY(batch_lanes_workspace(c, A, mixed));
     static const int kLanes[] = {2, 4, 8, 16};
     static const int kThreads[] = {128, 256, 512, 1024};
     constexpr int kTuneIters = 12;
@@ -675,17 +680,25 @@ int batch_pcg(Context* c, CSR& A, const double* b, double* x, int precision, int
     if (A.m != c->n_dofs) return set_err(c, TF_ERR_BAD_INPUT, "batch_pcg: matrix does not match the numbering");
     const int n = c->batch_count;
     if (n > kMaxBatchInstances) return set_err(c, TF_ERR_CAPACITY, "batch_pcg: too many instances");
-    TF_TRY(batch_workspace(c, A, mixed));
-    if (c->batch_fixed_lanes == 0 && (c->batch_lanes == 0 || c->batch_tuned_key != batch_key(c, c->h_batch_nnz, mixed)))
+    TF_TRY(batch_workspace(c, A));
+    BatchCluster bc;
+    bool cluster = false;
+    if (mixed && c->pcg_cluster != 0 && c->batch_fixed_lanes == 0) TF_TRY(batch_cluster_prepare(c, A, &bc, &cluster));
+    if (!cluster) TF_TRY(batch_lanes_workspace(c, A, mixed));
+    if (!cluster && c->batch_fixed_lanes == 0 && (c->batch_lanes == 0 || c->batch_tuned_key != batch_key(c, c->h_batch_nnz, mixed)))
         TF_TRY(batch_tune(c, A, b, mixed, nullptr, nullptr));
     const int G = c->batch_fixed_lanes ? c->batch_fixed_lanes : c->batch_lanes;
     const int T = c->batch_fixed_lanes ? c->batch_fixed_threads : c->batch_threads;
-    BatchSetup s;
-    TF_TRY(batch_prepare(c, A, mixed, G, T, &s));
+    BatchSetup s{};
+    if (!cluster) TF_TRY(batch_prepare(c, A, mixed, G, T, &s));
+    auto launch = [&]() {
+        return cluster ? batch_cluster_launch(c, bc, b, x, max_iter, tol, rel)
+                       : batch_launch(c, s, b, x, max_iter, tol, rel);
+    };
     TimedLaunch tl(c, TF_K_BATCH);
     if (!c->batch_use_graph) {
         drop_batch_graph(c);
-        TF_TRY(batch_launch(c, s, b, x, max_iter, tol, rel));
+        TF_TRY(launch());
         TF_CUDA(c, cudaMemcpyAsync(c->h_batch_out, c->batch_iters.p, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream));
         TF_CUDA(c, cudaMemcpyAsync(c->h_batch_out + kMaxBatchInstances, c->batch_resid.p, sizeof(double) * n,
                                    cudaMemcpyDeviceToHost, c->stream));
@@ -693,13 +706,15 @@ int batch_pcg(Context* c, CSR& A, const double* b, double* x, int precision, int
         union { double d; int64_t i; } tb;
         tb.d = tol;
         const std::vector<int64_t> key = {(int64_t)(intptr_t)b, (int64_t)(intptr_t)x, (int64_t)(intptr_t)A.vals,
-                                          A.pattern_gen, mixed, max_iter, tb.i, rel, G, T, s.grid,
+                                          A.pattern_gen, mixed, max_iter, tb.i, rel, cluster ? -bc.ctas : G,
+                                          cluster ? bc.grid : T, s.grid, (int64_t)(intptr_t)bc.scratch,
+                                          (int64_t)(intptr_t)bc.z, (int64_t)(intptr_t)c->cl_slots.p,
                                           (int64_t)(intptr_t)s.a.work, (int64_t)(intptr_t)s.a.val32};
         if (!c->batch_exec || key != c->batch_graph_key) {
             drop_batch_graph(c);
             cudaGraph_t g = nullptr;
             TF_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            int st = batch_launch(c, s, b, x, max_iter, tol, rel);
+            int st = launch();
             if (st == TF_OK &&
                 cudaMemcpyAsync(c->h_batch_out, c->batch_iters.p, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream) !=
                     cudaSuccess)

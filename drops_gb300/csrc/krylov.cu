@@ -1240,6 +1240,9 @@ void release_solver_workspace(Context* c) {
     release(c->kry_resid);
     release(c->kry_bar);
     release(c->kry_packed);
+    release(c->cl_z);
+    release(c->cl_slots);
+    release(c->cl_scratch);
     release(c->kry_iters);
 }
 
@@ -1401,6 +1404,15 @@ int pcg_mixed_kind(Context* c, CSR& A, const double* b, double* x, int kind, int
 
 int pcg_jacobi(Context* c, CSR& A, const double* b, double* x, int precision, int* max_iter, double* tol, int rel) {
     if (!A.vals || A.m <= 0) return set_err(c, TF_ERR_BAD_INPUT, "pcg: empty matrix");
+    if (precision == TF_PREC_MIXED || c->pcg_fp64_kernel == TF_PCG_FP64_CLASSIC) {
+        if (const int C = pcg_cluster_ctas(c, A)) {
+            TimedLaunch tl(c, TF_K_PCG);
+            bool applied = false;
+            const int st = precision == TF_PREC_MIXED ? pcg_cluster<float>(c, A, C, b, x, max_iter, tol, rel, &applied)
+                                                      : pcg_cluster<double>(c, A, C, b, x, max_iter, tol, rel, &applied);
+            if (applied || st != TF_OK) return st;
+        }
+    }
     TF_TRY(ensure_diag(c, A));
     TF_TRY(ensure_sell(c, A, precision == TF_PREC_MIXED));
     const int64_t m = A.m;

@@ -249,6 +249,7 @@ struct TuneEntry {
 struct CSR {
     int64_t m = 0, nnz = 0;
     int64_t pattern_gen = 0;    // bumps whenever the pattern changes
+    int64_t cluster_gen = -1;   // pattern of the last solve on a cluster
     Sell sell;
     int32_t* rowptr = nullptr;  // m+1 (device)
     int32_t* colind = nullptr;  // nnz
@@ -314,6 +315,9 @@ struct Context {
     DBuf<float> kry32;
     DBuf<unsigned> kry_bar;
     DBuf<unsigned long long> kry_packed;  // words of the packed reductions
+    DBuf<double> cl_z;        // cluster PCG: z per cluster
+    DBuf<int32_t> cl_slots;   // cluster slot of every row
+    DBuf<unsigned char> cl_scratch;  // what the CTAs' shared memory does not hold
     DBuf<int> kry_iters;
     // scratch
     DBuf<unsigned char> scratch;
@@ -347,6 +351,7 @@ struct Context {
     DBuf<int32_t> sell_cols[TF_NUM_MATS];  // GMRES: SELL columns as slots
     int64_t sell_cols_gen[TF_NUM_MATS] = {-1, -1, -1, -1, -1, -1, -1, -1};
     DBuf<uint16_t> sell_coltr[TF_NUM_MATS];
+    int pcg_cluster = -1;       // PCG of small systems and mixed batches on clusters (-1: by rule, 0: never, else CTAs)
     bool pcg_resident = true;   // PCG: block share of the system resident in shared memory where it fits
     bool autotune = true;       // measured launch shapes per matrix structure (tune.cu)
     bool spmv_shape_fixed = false, pcg_shape_fixed = false;  // set by the environment switches
@@ -534,6 +539,18 @@ int pcg_jacobi(Context* c, CSR& A, const double* b, double* x, int precision, in
 template <class T>
 int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);
 int packed_words(Context* c, int n, unsigned long long** w);
+int pcg_cluster_ctas(const Context* c, const CSR& A);
+template <class V>
+int pcg_cluster(Context* c, CSR& A, int ctas, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);
+// one prepared launch of the cluster PCG over the batch (pcg_cluster.cu)
+struct BatchCluster {
+    alignas(16) unsigned char blob[512];
+    int grid = 0, ctas = 0;
+    void* scratch = nullptr;
+    void* z = nullptr;
+};
+int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok);
+int batch_cluster_launch(Context* c, const BatchCluster& bc, const double* b, double* x, int max_iter, double tol, int rel);
 int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);
 // kinds of the single-barrier mixed PCG (autotuned per matrix structure, tune.cu)
 constexpr int kPcgResident = 0, kPcgCg1_512 = 1, kPcgCg1_256 = 2;
