@@ -105,37 +105,79 @@ __device__ __noinline__ ff ff_rhs(const RhsPar& R, const ff x[3]) {
 
 // The pair forms' per-tet data, one thread per tet: the tet geometry
 // (GetTrafoTr and the level set's vertex gradients), the patch on the
-// order-2 lattice and (P1, LIN) the linear-level-set test and its constants,
-// with the arithmetic of warp_tet_geometry, warp_patch and the P1 kernel's
-// linear path done serially.  The FP64 work of a tet is then one thread's
+// order-2 lattice, with the arithmetic of warp_tet_geometry and warp_patch
+// done serially.  The FP64 work of a tet is then one thread's
 // instead of a warp's with 4 to 25 lanes active, so that every FP64 warp
 // instruction works for 32 tets (GB300 runs FP64 at 1/64 of the FP32 rate).
 struct TetPrep {
     ff gl[4][3], G[4][3], X[4][3];
     ff fb[16][3][4], fw[16];
-    double lin_sg[4][3], lin_G[10], lin_dn[4];
     double absdet;
     ff absdet_ff;
-    int nf, lin;
+    int nf;
 };
 constexpr int64_t kPrepChunk = 1 << 18;  // tets per prep pass (about 0.6 GB of records)
 
-template <bool LIN>
+// Sign of a lattice value from its bits (a comparison holds the FP64 pipe 64 cycles): -1, 0, 1; 0 for NaN.
+__device__ __forceinline__ int lat_sign(double x) {
+    const long long b = __double_as_longlong(x);
+    const unsigned long long m = (unsigned long long)b & 0x7fffffffffffffffull;
+    return m == 0ull || m > 0x7ff0000000000000ull ? 0 : b < 0 ? -1 : 1;
+}
+
+// the lattice's negative and positive values as bits
+__device__ __forceinline__ void lat_signs(const double lat[10], unsigned& neg, unsigned& pos) {
+    neg = pos = 0u;
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+        const int s = lat_sign(lat[k]);
+        neg |= (s < 0 ? 1u : 0u) << k;
+        pos |= (s > 0 ? 1u : 0u) << k;
+    }
+}
+// sign pattern of a sub-tet: sum (s_k + 1) 3^k
+__device__ __forceinline__ int lat_pattern(int sub, unsigned neg, unsigned pos) {
+    int pat = 0;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+        const int v = cT.lat_t[sub][k];
+        pat = 3 * pat + 1 + (int)(pos >> v & 1u) - (int)(neg >> v & 1u);
+    }
+    return pat;
+}
+
+// the same for a sub-tet that differs between lanes
+__device__ __forceinline__ int lat_pattern_tab(const Tables* __restrict__ T, int sub, unsigned neg, unsigned pos) {
+    int pat = 0;
+#pragma unroll
+    for (int k = 3; k >= 0; --k) {
+        const int v = __ldg(&T->lat_t[sub][k]);
+        pat = 3 * pat + 1 + (int)(pos >> v & 1u) - (int)(neg >> v & 1u);
+    }
+    return pat;
+}
+// cut_point of a lattice edge that differs between lanes
+__device__ __forceinline__ void cut_point_tab(const Tables* __restrict__ T, const double lat[10], int k, double out[4]) {
+    const int a = __ldg(&T->edge_a[k]), b = __ldg(&T->edge_b[k]);
+    const double la = lat[a], t = __ddiv_rn(la, __dsub_rn(la, lat[b])), s = __dsub_rn(1.0, t);
+    for (int c = 0; c < 4; ++c)
+        out[c] = __dadd_rn(__dmul_rn(s, __ldg(&T->lat_v[a][c])), __dmul_rn(t, __ldg(&T->lat_v[b][c])));
+}
+
+// The loops over lattice edges, sub-tets, facets and vertices stay rolled in
+// the kernels below: unrolled, 150 to 190 KB of code ran from L2.
 __global__ void __launch_bounds__(128) k_prep_tets(AsmArgs A) {
     TetPrep* const out = reinterpret_cast<TetPrep*>(A.prep);
-    const int64_t n = A.c1 - A.c0;
+    const int64_t n = A.prep_count ? *A.prep_count : A.c1 - A.c0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = A.c0 + (A.prep_order ? A.prep_order[i] : i);
         TetPrep& Q = out[r - A.c0];
         const int32_t t = A.active[r];
         int32_t v[4], e[6];
-        mesh_tet(A.M, t, v, e);
         TetGeom g;
         double ls10[10];
-        for (int k = 0; k < 4; ++k) {
-            mesh_coord(A.M, v[k], g.X[k]);
-            ls10[k] = A.lsv[v[k]];
-        }
+        mesh_tet_points(A.M, t, v, e, g.X);
+        for (int k = 0; k < 4; ++k) ls10[k] = A.lsv[v[k]];
         for (int k = 0; k < 6; ++k) ls10[4 + k] = A.lse[e[k]];
         // warp_tet_geometry, lane by lane
         double Ms[9], Cs[9];
@@ -169,104 +211,69 @@ __global__ void __launch_bounds__(128) k_prep_tets(AsmArgs A) {
         // warp_patch, lane by lane: cut points of the lattice edges, the sub-tets' facets in order
         double lat[10];
         for (int k = 0; k < 10; ++k) lat[cP2OnLat[k]] = ls10[k];
+        unsigned neg, pos;
+        lat_signs(lat, neg, pos);
+        // every lane walks its own list of cut edges, then of facets (bit 2 s + f: facet f of sub-tet s), so lanes
+        // with different patterns stay in step
         double cut[25][4];
+        unsigned cuts = 0u;
+#pragma unroll
         for (int k = 0; k < 25; ++k) {
             const int a = cT.edge_a[k], b = cT.edge_b[k];
-            const double va = lat[a], vb = lat[b];
-            if ((va > 0. && vb < 0.) || (va < 0. && vb > 0.)) cut_point(lat, a, b, cut[k]);
+            cuts |= (((neg >> a & pos >> b) | (pos >> a & neg >> b)) & 1u) << k;
+        }
+#pragma unroll 1
+        for (unsigned m = cuts; m; m &= m - 1u) {
+            const int k = __ffs((int)m) - 1;
+            cut_point_tab(A.tab, lat, k, cut[k]);
+        }
+        unsigned facets = 0u;
+#pragma unroll 1
+        for (int sub = 0; sub < 8; ++sub) {
+            const int nfs = __ldg(&A.tab->pat_nf[lat_pattern(sub, neg, pos)]);
+            if (nfs < 0) set_status(A.status, TF_ERR_ZERO_PATTERN, t);
+            facets |= (nfs > 1 ? 3u : nfs > 0 ? 1u : 0u) << (2 * sub);
         }
         int nf = 0;
-        for (int sub = 0; sub < 8; ++sub) {
-            int pat = 0;
-            for (int k = 0; k < 4; ++k) {
-                const double val = lat[cT.lat_t[sub][k]];
-                pat += ((val > 0.) - (val < 0.) + 1) * (k == 0 ? 1 : k == 1 ? 3 : k == 2 ? 9 : 27);
-            }
-            int nfs = cT.pat_nf[pat];
-            if (nfs < 0) {
-                set_status(A.status, TF_ERR_ZERO_PATTERN, t);
-                nfs = 0;
-            }
-            for (int f = 0; f < nfs && nf < 16; ++f, ++nf) {
-                double w[3][3];
-                for (int j = 0; j < 3; ++j) {
-                    const int ext = cT.pat_f[pat][f][j];
-                    double b[4];
-                    if (ext < 4) {
-                        const int Lv = cT.lat_t[sub][ext];
-                        for (int c = 0; c < 4; ++c) b[c] = cT.lat_v[Lv][c];
-                    } else {
-                        const int id = cT.ledge[sub][ext - 4];
-                        for (int c = 0; c < 4; ++c) b[c] = cut[id][c];
-                    }
-                    for (int c = 0; c < 4; ++c) Q.fb[nf][j][c] = ff_split(b[c]);
-                    for (int rr = 0; rr < 3; ++rr)
-                        w[j][rr] = g.X[0][rr] * b[0] + g.X[1][rr] * b[1] + g.X[2][rr] * b[2] + g.X[3][rr] * b[3];
+#pragma unroll 1
+        for (unsigned m = facets; m; m &= m - 1u, ++nf) {
+            const int sub = (__ffs((int)m) - 1) >> 1, f = (__ffs((int)m) - 1) & 1;
+            const int pat = lat_pattern_tab(A.tab, sub, neg, pos);
+            double w[3][3];
+#pragma unroll 1
+            for (int j = 0; j < 3; ++j) {
+                const int ext = __ldg(&A.tab->pat_f[pat][f][j]);
+                double b[4];
+                if (ext < 4) {
+                    const int Lv = __ldg(&A.tab->lat_t[sub][ext]);
+                    for (int c = 0; c < 4; ++c) b[c] = __ldg(&A.tab->lat_v[Lv][c]);
+                } else {
+                    const int id = __ldg(&A.tab->ledge[sub][ext - 4]);
+                    for (int c = 0; c < 4; ++c) b[c] = cut[id][c];
                 }
-                double u[3], vq[3];
-                for (int rr = 0; rr < 3; ++rr) {
-                    u[rr] = w[1][rr] - w[0][rr];
-                    vq[rr] = w[2][rr] - w[0][rr];
-                }
-                const double c0 = u[1] * vq[2] - u[2] * vq[1], c1 = u[2] * vq[0] - u[0] * vq[2],
-                             c2 = u[0] * vq[1] - u[1] * vq[0];
-                Q.fw[nf] = ff_split(sqrt(c0 * c0 + c1 * c1 + c2 * c2) * (cT.pat_bnd[pat] ? 0.5 : 1.0));
+                for (int c = 0; c < 4; ++c) Q.fb[nf][j][c] = ff_split(b[c]);
+                for (int rr = 0; rr < 3; ++rr)
+                    w[j][rr] = g.X[0][rr] * b[0] + g.X[1][rr] * b[1] + g.X[2][rr] * b[2] + g.X[3][rr] * b[3];
             }
+            double u[3], vq[3];
+            for (int rr = 0; rr < 3; ++rr) {
+                u[rr] = w[1][rr] - w[0][rr];
+                vq[rr] = w[2][rr] - w[0][rr];
+            }
+            const double c0 = u[1] * vq[2] - u[2] * vq[1], c1 = u[2] * vq[0] - u[0] * vq[2],
+                         c2 = u[0] * vq[1] - u[1] * vq[0];
+            Q.fw[nf] = ff_split(sqrt(c0 * c0 + c1 * c1 + c2 * c2) * (__ldg(&A.tab->pat_bnd[pat]) ? 0.5 : 1.0));
         }
         Q.nf = nf;
-        // linear level set on the tet: every edge value the mean of its end values, bit for bit
-        bool lin = LIN;
-        for (int k = 0; LIN && k < 6; ++k) {
-            const double mean = __dmul_rn(0.5, __dadd_rn(ls10[ev0(k)], ls10[ev1(k)]));
-            lin = lin && __double_as_longlong(mean) == __double_as_longlong(ls10[4 + k]);
-        }
-        Q.lin = lin;
-        if (lin) {
-            const double bc[4] = {0.25, 0.25, 0.25, 0.25};
-            double n[3];
-            unit_normal(g, bc, n);
-            for (int vv = 0; vv < 4; ++vv) {
-                const double ng = n[0] * g.gl[vv][0] + n[1] * g.gl[vv][1] + n[2] * g.gl[vv][2];
-                for (int c = 0; c < 3; ++c) Q.lin_sg[vv][c] = g.gl[vv][c] - ng * n[c];
-            }
-            for (int k = 0; k < 10; ++k) {
-                int i, j;
-                sym_entry(4, k, i, j);
-                Q.lin_G[k] = Q.lin_sg[j][0] * Q.lin_sg[i][0] + Q.lin_sg[j][1] * Q.lin_sg[i][1] +
-                             Q.lin_sg[j][2] * Q.lin_sg[i][2];
-            }
-            for (int i = 0; i < 4; ++i) Q.lin_dn[i] = n[0] * g.gl[i][0] + n[1] * g.gl[i][1] + n[2] * g.gl[i][2];
-        }
         Q.absdet = g.absdet;
         Q.absdet_ff = ff_split(g.absdet);
+#pragma unroll 1
         for (int vv = 0; vv < 4; ++vv)
             for (int c = 0; c < 3; ++c) {
                 Q.gl[vv][c] = ff_split(g.gl[vv][c]);
                 Q.G[vv][c] = ff_split(g.G[vv][c]);
                 Q.X[vv][c] = ff_split(g.X[vv][c]);
             }
-    }
-}
-
-// Sort key of a tet for k_prep_tets: the signs (-, 0, +) of its 10 lattice
-// values in base 3.  They fix every branch of the prep (which lattice edges
-// are cut, each sub-tet's pattern and facets).  Signs from the bits: -0 and
-// +0 are zero, NaN counts by its sign bit (the key only orders the threads).
-constexpr int kPrepKeyBits = 16;  // 3^10 = 59,049 < 2^16
-__global__ void k_prep_key(AsmArgs A, uint32_t* __restrict__ key, int32_t* __restrict__ idx) {
-    const int64_t n = A.c1 - A.c0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        int32_t v[4], e[6];
-        mesh_tet(A.M, A.active[A.c0 + i], v, e);
-        uint32_t k = 0;
-        for (int j = 0; j < 10; ++j) {
-            const unsigned long long b =
-                (unsigned long long)__double_as_longlong(j < 4 ? A.lsv[v[j]] : A.lse[e[j - 4]]);
-            const uint32_t sg = (b << 1) == 0ull ? 1u : (b >> 63) ? 0u : 2u;
-            k = 3u * k + sg;
-        }
-        key[i] = k;
-        idx[i] = (int32_t)i;
     }
 }
 
@@ -416,11 +423,9 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p2_pair(AsmArgs A) 
 
 // ---------------------------------------------------------------------------
 // P1 forms M, A, C_n and the load vector in pair arithmetic (k_assemble_p1_pair).
-// The structure of k_assemble<4>: on a tet whose level set is linear (every
-// edge value the mean of its end values, bit for bit) the normal and the hat
-// functions' surface gradients are constant, A = (sum_p w_p) sg_i.sg_j and
-// C_n = |det| (sum_q w_q) dn_i dn_j from FP64 per-tet constants; otherwise the
-// normal, the projected gradients and the 15-point volume rule run per point.
+// The tets whose level set is not linear: the normal, the projected gradients
+// and the 15-point volume rule run per point; a warp takes a tet of the list
+// that k_assemble_p1_linear left.
 // Per point (node, weight and its square root, normal, gradients, load
 // function) and every sum over points run in pair arithmetic; the point
 // groups of the sums are those of k_assemble<4> (entries on 3 groups of
@@ -434,8 +439,7 @@ struct AsmPair1Smem {
     AsmPair1Pts p;
     ff gl[4][3], G[4][3], X[4][3];
     ff fb[16][3][4], fw[16];
-    ff wt[32], fx[32];  // w_p; sqrt(w) f(x_p)
-    double lin_sg[4][3], lin_G[10], lin_dn[4];
+    ff fx[32];  // sqrt(w) f(x_p)
 };
 
 __device__ __forceinline__ ff ff_shfl_down(ff a, int d) {
@@ -462,15 +466,13 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1_pair(AsmArgs A) 
     const bool wantC = A.forms & (1u << TF_FORM_CN);
     const bool wantF = A.rhs.kind != TF_RHS_NONE;
     const int64_t nwarps = (int64_t)gridDim.x * kAsmWarps;
-    double s3 = 0.;  // the 15-point rule's weight sum (linear level set: n . grad(phi_i) is constant)
-    for (int pp = 0; pp < 15; ++pp) s3 += cT.q3_w[pp];
-
     const TetPrep* const prep = reinterpret_cast<const TetPrep*>(A.prep);
-    for (int64_t r = A.c0 + (int64_t)blockIdx.x * kAsmWarps + wib; r < A.c1; r += nwarps) {
+    const int64_t n = *A.prep_count;
+    for (int64_t i = (int64_t)blockIdx.x * kAsmWarps + wib; i < n; i += nwarps) {
+        const int64_t r = A.c0 + A.prep_order[i];
         // the tet's record (k_prep_tets) into shared memory
         const TetPrep& Q = prep[r - A.c0];
         const int nf = Q.nf;
-        const bool lin = Q.lin != 0;
         const double absdet = Q.absdet;
         for (int k = lane; k < 36; k += 32) {
             const int m = k / 12, v3 = (k % 12) / 3, c = k % 3;
@@ -483,15 +485,6 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1_pair(AsmArgs A) 
             else
                 S.fb[f][j >> 2][j & 3] = Q.fb[f][j >> 2][j & 3];
         }
-        if (lin)
-            for (int k = lane; k < 26; k += 32) {
-                if (k < 12)
-                    S.lin_sg[k / 3][k % 3] = Q.lin_sg[k / 3][k % 3];
-                else if (k < 22)
-                    S.lin_G[k - 12] = Q.lin_G[k - 12];
-                else
-                    S.lin_dn[k - 22] = Q.lin_dn[k - 22];
-            }
         __syncwarp();
         AsmPair1Pts& P = S.p;
 
@@ -510,16 +503,13 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1_pair(AsmArgs A) 
                                   ff_fma(S.fb[f][1][c], cTF.q2_node[q][1], ff_mul(S.fb[f][0][c], cTF.q2_node[q][0])));
                 const ff w = ff_mul(S.fw[f], cTF.q2_w[q]);
                 const ff sw = ff_sqrt(w);
-                S.wt[lane] = w;
                 for (int i = 0; i < 4; ++i) P.phi[lane][i] = ff_mul(sw, b[i]);
-                if (!lin) {
-                    ff n[3];
-                    ff_normal1(S.G, b, n);
+                ff n[3];
+                ff_normal1(S.G, b, n);
 #pragma unroll 1
-                    for (int k = 0; k < 4; ++k) {
-                        const ff ng = ff_dot3(n, S.gl[k]);
-                        for (int c = 0; c < 3; ++c) P.sg[lane][3 * k + c] = ff_mul(sw, ff_sub(S.gl[k][c], ff_mul(ng, n[c])));
-                    }
+                for (int k = 0; k < 4; ++k) {
+                    const ff ng = ff_dot3(n, S.gl[k]);
+                    for (int c = 0; c < 3; ++c) P.sg[lane][3 * k + c] = ff_mul(sw, ff_sub(S.gl[k][c], ff_mul(ng, n[c])));
                 }
                 if (wantF) {
                     ff x[3];
@@ -535,13 +525,9 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1_pair(AsmArgs A) 
                 for (int pp = grp; pp < cnt; pp += 3) {
                     if (wantM) accM.add_prod(P.phi[pp][ej], P.phi[pp][ei]);
                     if (wantA) {
-                        if (lin) {
-                            accA.add(S.wt[pp]);
-                        } else {
-                            accA.add_prod(P.sg[pp][3 * ej], P.sg[pp][3 * ei]);
-                            accA.add_prod(P.sg[pp][3 * ej + 1], P.sg[pp][3 * ei + 1]);
-                            accA.add_prod(P.sg[pp][3 * ej + 2], P.sg[pp][3 * ei + 2]);
-                        }
+                        accA.add_prod(P.sg[pp][3 * ej], P.sg[pp][3 * ei]);
+                        accA.add_prod(P.sg[pp][3 * ej + 1], P.sg[pp][3 * ei + 1]);
+                        accA.add_prod(P.sg[pp][3 * ej + 2], P.sg[pp][3 * ei + 2]);
                     }
                 }
             }
@@ -558,35 +544,411 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1_pair(AsmArgs A) 
         vF = ff_add(vF, ff_shfl_down(vF, 4));
         double outC = 0.;
         if (wantC) {
-            if (lin) {
-                outC = (s3 * (S.lin_dn[ej] * S.lin_dn[ei])) * absdet;
-            } else {
-                __syncwarp();
-                if (lane < 15) {
-                    ff b[4];
-                    for (int c = 0; c < 4; ++c) b[c] = cTF.q3_node[lane][c];
-                    ff n[3];
-                    ff_normal1(S.G, b, n);
-                    for (int k = 0; k < 4; ++k) P.phi[lane][k] = ff_mul(cTF.q3_sw[lane], ff_dot3(n, S.gl[k]));
-                }
-                __syncwarp();
-                ffacc accC;
-                if (grp < 3)
-                    for (int pp = grp; pp < 15; pp += 3) accC.add_prod(P.phi[pp][ej], P.phi[pp][ei]);
-                ff vC = accC.value();
-                vC = ff_add(ff_add(vC, ff_shfl_down(vC, 10)), ff_shfl_down(vC, 20));
-                outC = ff_to_double(vC) * absdet;
+            __syncwarp();
+            if (lane < 15) {
+                ff b[4];
+                for (int c = 0; c < 4; ++c) b[c] = cTF.q3_node[lane][c];
+                ff n[3];
+                ff_normal1(S.G, b, n);
+                for (int k = 0; k < 4; ++k) P.phi[lane][k] = ff_mul(cTF.q3_sw[lane], ff_dot3(n, S.gl[k]));
             }
+            __syncwarp();
+            ffacc accC;
+            if (grp < 3)
+                for (int pp = grp; pp < 15; pp += 3) accC.add_prod(P.phi[pp][ej], P.phi[pp][ei]);
+            ff vC = accC.value();
+            vC = ff_add(ff_add(vC, ff_shfl_down(vC, 10)), ff_shfl_down(vC, 20));
+            outC = ff_to_double(vC) * absdet;
         }
         if (lane < NSYM) {
             if (wantM) A.elem[((int64_t)TF_FORM_M * A.n_active + r) * NSYM + lane] = ff_to_double(vM);
-            if (wantA) {
-                const double a = ff_to_double(vA);
-                A.elem[((int64_t)TF_FORM_A * A.n_active + r) * NSYM + lane] = lin ? a * S.lin_G[lane] : a;
-            }
+            if (wantA) A.elem[((int64_t)TF_FORM_A * A.n_active + r) * NSYM + lane] = ff_to_double(vA);
             if (wantC) A.elem[((int64_t)TF_FORM_CN * A.n_active + r) * NSYM + lane] = outC;
         }
         if (wantF && lane < NL) A.elem_rhs[r * NL + lane] = ff_to_double(vF);
         __syncwarp();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// P1 forms M, A, C_n and the load vector on tets whose level set is linear
+// (every edge value the mean of its end values, bit for bit): G lanes per tet.
+//
+// The normal and the hat functions' surface gradients are constant, so
+//   A_ij = |cut| sg_i . sg_j,  C_ij = |det| (sum_q w_q) dn_i dn_j,
+// the hat functions are linear on the cut, so M is exact in closed form,
+//   int phi_i phi_j = |facet| / 12 (S_i S_j + sum_k phi_i(v_k) phi_j(v_k)),
+// S_i = sum_k phi_i(v_k), and a constant load's vector |facet| / 3 S_i: all on the
+// cut of the whole tet, one or two triangles, where the quadrature took 7 points on
+// each of up to 16 facets of the order-2 lattice.  Other loads keep that rule, the
+// points of a facet summed into the moments sum_q w_q N_k(q) f(x_q) before they meet
+// the basis.  Every lane walks the lists of its own tet's cut edges and facets, so
+// lanes with different sign patterns stay in step.  Facets lie in the plane of normal
+// n, and n . (u x v) = det sum_c dn_c (du x dv)_c from barycentric differences du, dv
+// needs no square root.  Geometry, cut points and areas are FP64, everything per point
+// and all sums pairs.
+//
+// Bound by the FP64 pipe (about 380 instructions per warp of 32 tets with a constant
+// load, 600 with points, 64 cycles each; 49% busy) and, with points, the pair
+// arithmetic.  Forms M, A, C_n of 126,800 cut tets (P1 sphere 128^3, prep and sort
+// included): 868 -> 147 us with a constant load, 1,017 -> 374 with the closest-point
+// load; 1,920 tets 143 -> 41 and 145 -> 73.  The warp per tet before formed 42 points on
+// 64 lanes and its sums on 10 to 30 lanes, from 1.9 KB records of FP64 work unrolled to
+// 152 KB of code.
+//
+// Tets whose level set is not linear go to `rest` (counted in *nrest, in the
+// order of the threads up to the order of the warps' atomics).
+// ---------------------------------------------------------------------------
+// the closest-point load c y0 y1 y2 at centre + d: y = centre + R d / |d|
+__device__ __forceinline__ ff ff_rhs_sphere(const ff ctr[3], ff R, ff amp, const ff d[3]) {
+    ffacc n2;
+    for (int r = 0; r < 3; ++r) n2.add_prod(d[r], d[r]);
+    const ff s = ff_mul(R, ff_rsqrt(n2.value()));
+    ff y[3];
+    for (int r = 0; r < 3; ++r) y[r] = ff_fma(s, d[r], ctr[r]);
+    return ff_mul(ff_mul(ff_mul(amp, y[0]), y[1]), y[2]);
+}
+
+// pair -> double with one FP64 instruction: both parts widened on the integer pipe
+__device__ __forceinline__ double widen_f32(float x) {
+    const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
+    if (e - 1u >= 254u) return (b << 1) == 0u ? 0.0 : (double)x;
+    return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20 | (b & 0x7fffffu) >> 3)), (int)(b << 29));
+}
+__device__ __forceinline__ double ff_widen(ff a) { return __dadd_rn(widen_f32(a.h), widen_f32(a.l)); }
+
+template <int G>
+__device__ __forceinline__ ff lane_group_sum(ff a) {
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1)
+        a = ff_add(a, ff{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)});
+    return a;
+}
+
+// |u x w| of the facet's edges, where the level set's gradient is too small or large to give the plane's normal
+__device__ __noinline__ double p1_area2(const double (&X)[4][3], const double (&du)[3], const double (&dv)[3]) {
+    double u[3], w[3];
+    for (int rr = 0; rr < 3; ++rr) {
+        u[rr] = du[0] * (X[1][rr] - X[0][rr]) + du[1] * (X[2][rr] - X[0][rr]) + du[2] * (X[3][rr] - X[0][rr]);
+        w[rr] = dv[0] * (X[1][rr] - X[0][rr]) + dv[1] * (X[2][rr] - X[0][rr]) + dv[2] * (X[3][rr] - X[0][rr]);
+    }
+    const double c0 = u[1] * w[2] - u[2] * w[1], c1 = u[2] * w[0] - u[0] * w[2], c2 = u[0] * w[1] - u[1] * w[0];
+    return sqrt(c0 * c0 + c1 * c1 + c2 * c2);
+}
+
+// linear level set on the tet: every edge value the mean of its end values, bit for bit
+__device__ __forceinline__ bool p1_linear_ls(const double (&ls10)[10]) {
+    bool lin = true;
+    for (int k = 0; k < 6; ++k) {
+        const double mean = __dmul_rn(0.5, __dadd_rn(ls10[ev0(k)], ls10[ev1(k)]));
+        lin = lin && __double_as_longlong(mean) == __double_as_longlong(ls10[4 + k]);
+    }
+    return lin;
+}
+__device__ __forceinline__ bool p1_linear_tet(const AsmArgs& A, int32_t t, double (&lat)[10]) {
+    int32_t v[4], e[6];
+    mesh_tet(A.M, t, v, e);
+    double ls10[10];
+    for (int k = 0; k < 10; ++k) ls10[k] = k < 4 ? A.lsv[v[k]] : A.lse[e[k - 4]];
+    for (int k = 0; k < 10; ++k) lat[cP2OnLat[k]] = ls10[k];
+    return p1_linear_ls(ls10);
+}
+
+// lattice edges that a linear level set cuts at most (every sign pattern whose edge midpoints take the sign of
+// equal ends; a value that rounds to zero only takes cuts away)
+constexpr int kLinCuts = 13;
+
+template <int G, int B>
+__global__ void __launch_bounds__(128, B) k_assemble_p1_linear(AsmArgs A, int32_t* __restrict__ rest, int* __restrict__ nrest) {
+    constexpr int NSYM = 10;
+    const bool wantM = A.forms & (1u << TF_FORM_M), wantA = A.forms & (1u << TF_FORM_A);
+    const bool wantC = A.forms & (1u << TF_FORM_CN);
+    const bool wantF = A.rhs.kind != TF_RHS_NONE, constF = A.rhs.kind == TF_RHS_CONST;
+    const int lane = threadIdx.x & 31, sub = lane % G;
+    const int64_t n = A.c1 - A.c0;
+    double s3 = 0.;  // the 15-point rule's weight sum
+    for (int q = 0; q < 15; ++q) s3 += cT.q3_w[q];
+    // tets for the general kernels; whole warps call
+    auto leave = [&](bool yes, int32_t rel) {
+        const unsigned m = __ballot_sync(0xffffffffu, yes);
+        if (!m) return;
+        int at = 0;
+        if (lane == 0) at = atomicAdd(nrest, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (yes) rest[at + __popc(m & ((1u << lane) - 1u))] = rel;
+    };
+    // Blocks of kTets tets.  With a point rule the block's tets are taken in the order of their facet counts: the
+    // lanes of a warp walk their facets in step, and the longest list sets the warp's time.
+    constexpr int kTets = 128 / G;
+    __shared__ int32_t order[kTets];
+    __shared__ int bin[17];
+    for (int64_t i0 = (int64_t)blockIdx.x * kTets; i0 < n; i0 += (int64_t)gridDim.x * kTets) {
+        const int m = (int)(n - i0 < kTets ? n - i0 : kTets);
+        if (wantF && !constF) {
+            __syncthreads();
+            if (threadIdx.x < 17) bin[threadIdx.x] = 0;
+            __syncthreads();
+            int nf = 0, at = 0;
+            bool linear = false;
+            if ((int)threadIdx.x < m) {
+                double lat[10];
+                linear = p1_linear_tet(A, A.active[A.c0 + i0 + threadIdx.x], lat);
+                unsigned neg, pos;
+                lat_signs(lat, neg, pos);
+#pragma unroll 1
+                for (int s8 = 0; s8 < 8; ++s8) nf += max(0, (int)__ldg(&A.tab->pat_nf[lat_pattern(s8, neg, pos)]));
+                at = atomicAdd(&bin[nf], 1);
+            }
+            __syncthreads();
+            if ((int)threadIdx.x < m) {
+                for (int k = 0; k < nf; ++k) at += bin[k];
+                order[at] = linear ? (int32_t)threadIdx.x : ~(int32_t)threadIdx.x;
+            }
+            __syncthreads();
+        }
+        const int slot = threadIdx.x / G;
+        const int at = slot >= m ? -1 : wantF && !constF ? order[slot] : slot;
+        const bool valid = at >= 0;
+        if (wantF && !constF) leave(slot < m && at < 0 && sub == 0, (int32_t)i0 + ~at);
+        const int32_t rel = !valid ? 0 : (int32_t)i0 + at;
+        const int64_t r = A.c0 + rel;
+        const int32_t t = valid ? A.active[r] : 0;
+        double X[4][3], lat[10];
+        bool lin = valid;
+        if (valid) {
+            int32_t v[4], e[6];
+            mesh_tet_points(A.M, t, v, e, X);
+            double ls10[10];
+            for (int k = 0; k < 10; ++k) ls10[k] = k < 4 ? A.lsv[v[k]] : A.lse[e[k - 4]];
+            if (!(wantF && !constF)) lin = p1_linear_ls(ls10);
+            for (int k = 0; k < 10; ++k) lat[cP2OnLat[k]] = ls10[k];
+        }
+        if (!(wantF && !constF)) leave(valid && !lin && sub == 0, rel);
+        double gl[4][3], dn[4], absdet, ddn[3], inv_g = 0.;
+        bool plane = false;
+        if (lin) {
+            double Ms[9], Cs[9];
+            for (int l = 0; l < 9; ++l) Ms[l] = X[l % 3 + 1][l / 3] - X[0][l / 3];
+            for (int l = 0; l < 9; ++l) {
+                const int rr = l / 3, c = l % 3;
+                const int r1 = (rr + 1) % 3, r2 = (rr + 2) % 3, c1 = (c + 1) % 3, c2 = (c + 2) % 3;
+                Cs[l] = Ms[3 * r1 + c1] * Ms[3 * r2 + c2] - Ms[3 * r1 + c2] * Ms[3 * r2 + c1];
+            }
+            const double d = Ms[0] * Cs[0] + Ms[1] * Cs[1] + Ms[2] * Cs[2];
+            const double inv = 1.0 / d;
+            absdet = fabs(d);
+            for (int vv = 1; vv < 4; ++vv)
+                for (int rr = 0; rr < 3; ++rr) gl[vv][rr] = Cs[3 * rr + vv - 1] * inv;
+            for (int rr = 0; rr < 3; ++rr) gl[0][rr] = (-gl[1][rr] - gl[2][rr]) - gl[3][rr];
+            // the level set's gradient from the vertex values
+            const double l0 = lat[cP2OnLat[0]];
+            double g[3] = {0., 0., 0.};
+            for (int vv = 1; vv < 4; ++vv) {
+                const double dl = lat[cP2OnLat[vv]] - l0;
+                for (int rr = 0; rr < 3; ++rr) g[rr] += dl * gl[vv][rr];
+            }
+            const double g2 = g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
+            const unsigned ge = (unsigned)(__double2hiint(g2) >> 20);
+            plane = ge > 123u && ge < 1923u;  // 2^-900 < |g|^2 < 2^900: n is a unit vector
+            inv_g = rsqrt_fp64(g2);
+            for (int rr = 0; rr < 3; ++rr) g[rr] *= inv_g;
+            for (int vv = 0; vv < 4; ++vv) dn[vv] = g[0] * gl[vv][0] + g[1] * gl[vv][1] + g[2] * gl[vv][2];
+            for (int c = 0; c < 3; ++c) ddn[c] = d * dn[c + 1];
+            // A needs the projected gradients' products
+            if (wantA && sub == 0)
+                for (int vv = 0; vv < 4; ++vv)
+                    for (int c = 0; c < 3; ++c) gl[vv][c] -= dn[vv] * g[c];
+        }
+        // twice the area of a facet of barycentric corners b (components 1..3), as a pair
+        auto area2 = [&](const double (&b)[3][3], float scale) {
+            double du[3], dv[3], m[3];
+            for (int c = 0; c < 3; ++c) {
+                du[c] = b[1][c] - b[0][c];
+                dv[c] = b[2][c] - b[0][c];
+            }
+            for (int c = 0; c < 3; ++c) m[c] = du[(c + 1) % 3] * dv[(c + 2) % 3] - du[(c + 2) % 3] * dv[(c + 1) % 3];
+            double a2 = fabs(m[0] * ddn[0] + m[1] * ddn[1] + m[2] * ddn[2]);
+            if (!plane) a2 = p1_area2(X, du, dv);
+            return ff_scale(ff_split(a2), scale);
+        };
+        unsigned neg = 0u, pos = 0u;
+        ffacc accF[4];
+        if (lin && sub == 0) {
+            // M, A, C_n and a constant load: the cut of the whole tet, at most two triangles
+            lat_signs(lat, neg, pos);
+            int pat = 0;
+            for (int k = 3; k >= 0; --k) pat = 3 * pat + 1 + (int)(pos >> cP2OnLat[k] & 1u) - (int)(neg >> cP2OnLat[k] & 1u);
+            const int nf = __ldg(&A.tab->pat_nf[pat]);
+            const float scale = __ldg(&A.tab->pat_bnd[pat]) ? 0.5f : 1.0f;
+            if (nf < 0) set_status(A.status, TF_ERR_ZERO_PATTERN, t);
+            ffacc accM[NSYM], accA;
+#pragma unroll 1
+            for (int f = 0; f < nf; ++f) {
+                double b[3][3];
+                ff p[4][4];
+#pragma unroll 1
+                for (int j = 0; j < 3; ++j) {
+                    const int ext = __ldg(&A.tab->pat_f[pat][f][j]);
+                    int va = ext, vb = ext;
+                    double st = 1.0, tt = 0.0;
+                    if (ext >= 4) {
+                        va = ev0(ext - 4);
+                        vb = ev1(ext - 4);
+                        const double la = lat[cP2OnLat[va]], lb = lat[cP2OnLat[vb]];
+                        tt = __ddiv_rn(la, __dsub_rn(la, lb));
+                        st = __dsub_rn(1.0, tt);
+                    }
+                    const ff sf = ff_split(st), tf = ff_split(tt);
+                    for (int c = 0; c < 4; ++c) {
+                        p[j][c] = c == va ? sf : c == vb ? tf : ff_of(0.f);
+                        if (c > 0) b[j][c - 1] = c == va ? st : c == vb ? tt : 0.0;
+                    }
+                }
+                const ff fw = area2(b, scale);
+                accA.add(fw);
+                for (int c = 0; c < 4; ++c) p[3][c] = ff_add(ff_add(p[0][c], p[1][c]), p[2][c]);
+                if (constF)
+                    for (int c = 0; c < 4; ++c) accF[c].add_prod(fw, p[3][c]);
+#pragma unroll 1
+                for (int j = 0; j < 4; ++j) {
+                    ff q[4];
+                    for (int c = 0; c < 4; ++c) q[c] = p[j][c];
+                    int k = 0;  // entry (a, c), a <= c, row by row
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        const ff tq = ff_mul(fw, q[a]);
+#pragma unroll
+                        for (int c = a; c < 4; ++c) accM[k++].add_prod(tq, q[c]);
+                    }
+                }
+            }
+            const int64_t e = r * (NSYM / 2), form = A.n_active * (NSYM / 2);
+            double2* const el = reinterpret_cast<double2*>(A.elem);
+            if (wantM) {
+#pragma unroll
+                for (int k = 0; k < NSYM; k += 2)
+                    el[TF_FORM_M * form + e + k / 2] = make_double2(ff_widen(accM[k].value()) * (1.0 / 24.0),
+                                                                    ff_widen(accM[k + 1].value()) * (1.0 / 24.0));
+            }
+            if (wantA) {
+                const double area = 0.5 * ff_widen(accA.value());
+                double w[NSYM];
+                int k = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = i; j < 4; ++j)
+                        w[k++] = area * (gl[j][0] * gl[i][0] + gl[j][1] * gl[i][1] + gl[j][2] * gl[i][2]);
+#pragma unroll
+                for (int k = 0; k < NSYM; k += 2) el[TF_FORM_A * form + e + k / 2] = make_double2(w[k], w[k + 1]);
+            }
+            if (wantC) {
+                const double s3d = s3 * absdet;
+                double w[NSYM];
+                int k = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = i; j < 4; ++j) w[k++] = s3d * (dn[j] * dn[i]);
+#pragma unroll
+                for (int k = 0; k < NSYM; k += 2) el[TF_FORM_CN * form + e + k / 2] = make_double2(w[k], w[k + 1]);
+            }
+        }
+        if (lin && wantF && !constF) {
+            // other loads: the 7-point rule on the facets of the order-2 lattice
+            const ff ctr[3] = {ff_split(A.rhs.p[0]), ff_split(A.rhs.p[1]), ff_split(A.rhs.p[2])};
+            const ff R = ff_split(A.rhs.p[3]), amp = ff_split(A.rhs.p[4]);
+            ff Xf[4][3];
+#pragma unroll 1
+            for (int vv = 0; vv < 4; ++vv)
+                for (int c = 0; c < 3; ++c) Xf[vv][c] = ff_sub(ff_split(X[vv][c]), ctr[c]);
+            if (G > 1) lat_signs(lat, neg, pos);
+            // the lattice edges cut and their points in this order; every lane walks its own list, so lanes with
+            // different patterns stay in step
+            unsigned cuts = 0u;
+#pragma unroll
+            for (int k = 0; k < 25; ++k) {
+                const int a = cT.edge_a[k], b = cT.edge_b[k];
+                cuts |= (((neg >> a & pos >> b) | (pos >> a & neg >> b)) & 1u) << k;
+            }
+            double cut[kLinCuts][4];
+            int ncut = 0;
+#pragma unroll 1
+            for (unsigned m = cuts; m && ncut < kLinCuts; m &= m - 1u, ++ncut) {
+                cut_point_tab(A.tab, lat, __ffs((int)m) - 1, cut[ncut]);
+            }
+            // the facets: bit 2 s + f is facet f of sub-tet s
+            unsigned facets = 0u;
+#pragma unroll 1
+            for (int s8 = 0; s8 < 8; ++s8) {
+                const int nfs = __ldg(&A.tab->pat_nf[lat_pattern(s8, neg, pos)]);
+                if (nfs < 0) set_status(A.status, TF_ERR_ZERO_PATTERN, t);
+                facets |= (nfs > 1 ? 3u : nfs > 0 ? 1u : 0u) << (2 * s8);
+            }
+            // a lane takes every G-th of them
+            auto drop = [](unsigned m, int k) {
+                for (; k > 0; --k) m &= m - 1u;
+                return m;
+            };
+#pragma unroll 1
+            for (unsigned m = drop(facets, sub); m; m = drop(m, G)) {
+                const int s8 = (__ffs((int)m) - 1) >> 1, f = (__ffs((int)m) - 1) & 1;
+                const int pat = lat_pattern_tab(A.tab, s8, neg, pos);
+                const float scale = __ldg(&A.tab->pat_bnd[pat]) ? 0.5f : 1.0f;
+                // corners: barycentric, as pairs p[j], and world coordinates from the centre Y[j]
+                double b[3][3];
+                ff p[3][4], Y[3][3];
+#pragma unroll 1
+                for (int j = 0; j < 3; ++j) {
+                    const int ext = __ldg(&A.tab->pat_f[pat][f][j]);
+                    double v[4];
+                    if (ext < 4) {
+                        const int lv = __ldg(&A.tab->lat_t[s8][ext]);
+                        for (int c = 0; c < 4; ++c) v[c] = __ldg(&A.tab->lat_v[lv][c]);
+                    } else {
+                        const int id = __ldg(&A.tab->ledge[s8][ext - 4]);
+                        const int at = min(__popc(cuts & ((1u << id) - 1u)), kLinCuts - 1);
+                        for (int c = 0; c < 4; ++c) v[c] = cut[at][c];
+                    }
+                    ff pj[4];
+                    for (int c = 0; c < 4; ++c) {
+                        pj[c] = ff_split(v[c]);
+                        p[j][c] = pj[c];
+                        if (c > 0) b[j][c - 1] = v[c];
+                    }
+                    for (int c = 0; c < 3; ++c) {
+                        ffacc y;
+                        for (int k = 0; k < 4; ++k) y.add_prod(pj[k], Xf[k][c]);
+                        Y[j][c] = y.value();
+                    }
+                }
+                const ff fw = area2(b, scale);
+                ffacc mom[3];
+#pragma unroll 1
+                for (int q = 0; q < 7; ++q) {
+                    ff d[3];
+                    for (int c = 0; c < 3; ++c) {
+                        ffacc x;
+                        for (int j = 0; j < 3; ++j) x.add_prod(Y[j][c], cTF.q2_node[q][j]);
+                        d[c] = x.value();
+                    }
+                    const ff wf = ff_mul(cTF.q2_w[q], ff_rhs_sphere(ctr, R, amp, d));
+                    for (int j = 0; j < 3; ++j) mom[j].add_prod(wf, cTF.q2_node[q][j]);
+                }
+                for (int j = 0; j < 3; ++j) {
+                    const ff w = ff_mul(fw, mom[j].value());
+                    for (int c = 0; c < 4; ++c) accF[c].add_prod(w, p[j][c]);
+                }
+            }
+        }
+        ff vF[4];
+        for (int k = 0; k < 4; ++k) vF[k] = lane_group_sum<G>(accF[k].value());
+        if (!lin || sub != 0) continue;
+        if (wantF) {
+            const double c = constF ? A.rhs.p[0] * (1.0 / 6.0) : 1.0;
+            double2* const o = reinterpret_cast<double2*>(A.elem_rhs + r * 4);
+            o[0] = make_double2(c * ff_widen(vF[0]), c * ff_widen(vF[1]));
+            o[1] = make_double2(c * ff_widen(vF[2]), c * ff_widen(vF[3]));
+        }
     }
 }

@@ -22,7 +22,6 @@
 #include <climits>
 #include <cstring>
 
-#include <cub/device/device_radix_sort.cuh>
 
 #include "ff.cuh"
 #include "tf_internal.cuh"
@@ -528,6 +527,8 @@ struct AsmArgs {
     void* prep;
     int64_t c0, c1;
     const int32_t* prep_order;  // prep thread i takes active tet c0 + prep_order[i] (null: c0 + i)
+    const int* prep_count;      // entries of prep_order (null: c1 - c0)
+    const Tables* tab;          // cT in global memory: indexes that differ between lanes are replayed in the constant bank
 };
 
 template <int NL>
@@ -798,28 +799,21 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble(AsmArgs A) {
 
 #include "asm_pair.cuh"
 
-// The order of the prep threads over active tets [A.c0, A.c1): by the sign
-// pattern of each tet's lattice values (k_prep_key), so that a warp's tets
-// take the same branches.  Every thread still writes its own tet's record.
-static int prep_order(Context* c, AsmArgs& A, int64_t chunk) {
-    A.prep_order = nullptr;
-    if (!c->prep_sort) return TF_OK;
-    const int64_t n = A.c1 - A.c0;
-    TF_TRY(ensure(c, c->prep_key, (size_t)(2 * chunk)));
-    TF_TRY(ensure(c, c->prep_idx, (size_t)(2 * chunk)));
-    uint32_t* key = c->prep_key.p;
-    int32_t* idx = c->prep_idx.p;
-    k_prep_key<<<grid_for(c, n, 256), 256, 0, c->stream>>>(A, key, idx);
-    ++c->launches;
-    TF_CUDA(c, cudaGetLastError());
-    size_t bytes = 0;
-    TF_CUDA(c, cub::DeviceRadixSort::SortPairs(nullptr, bytes, key, key + chunk, idx, idx + chunk, (int)n, 0,
-                                                kPrepKeyBits, c->stream));
-    TF_TRY(ensure(c, c->prep_tmp, bytes + 1));
-    TF_CUDA(c, cub::DeviceRadixSort::SortPairs(c->prep_tmp.p, bytes, key, key + chunk, idx, idx + chunk, (int)n, 0,
-                                                kPrepKeyBits, c->stream));
-    A.prep_order = idx + chunk;
-    return TF_OK;
+// The linear tets of a chunk.  Four lanes per tet while that is at most one block
+// per SM (latency: the facets of a tet in a quarter of the steps), else one; 160
+// registers while all blocks are resident at three per SM, else 128 and four.
+// A load with a point rule, us: 1,920 tets 111 / 73 on 1 / 4 lanes, 4,458 112 / 74, 13,010
+// 112 / 171; 28,800 tets 143 / 149 on three / four blocks per SM, 71,300 289 / 222,
+// 126,800 448 / 374.
+static void launch_p1_linear(Context* c, const AsmArgs& A, int64_t n, int32_t* rest, int* nrest) {
+    const bool points = A.rhs.kind != TF_RHS_NONE && A.rhs.kind != TF_RHS_CONST;
+    if (points && (n + 31) / 32 <= c->num_sms) {
+        k_assemble_p1_linear<4, 3><<<(unsigned)((n + 31) / 32), 128, 0, c->stream>>>(A, rest, nrest);
+        return;
+    }
+    const unsigned blocks = (unsigned)((n + 127) / 128);
+    if ((int64_t)blocks <= 3 * (int64_t)c->num_sms) k_assemble_p1_linear<1, 3><<<blocks, 128, 0, c->stream>>>(A, rest, nrest);
+    else k_assemble_p1_linear<1, 4><<<blocks, 128, 0, c->stream>>>(A, rest, nrest);
 }
 
 // ---------------------------------------------------------------------------
@@ -1150,6 +1144,7 @@ int setup_fe_system(Context* c, unsigned forms, int rhs_kind, const double* rhs_
                           (rhs_kind == TF_RHS_NONE || rhs_kind == TF_RHS_CONST || rhs_kind == TF_RHS_SPHERE_XYZ);
         if (pair) {
             TF_TRY(ensure_tables_ff(c));
+            TF_CUDA(c, cudaGetSymbolAddress((void**)&A.tab, cT));
             const size_t sm = sizeof(AsmPairSmem) * kAsmWarps;
             TF_CUDA(c, cudaFuncSetAttribute(k_assemble_p2_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             // per chunk of active tets: the per-tet records (one thread per tet), then the forms (warp per tet)
@@ -1160,8 +1155,7 @@ int setup_fe_system(Context* c, unsigned forms, int rhs_kind, const double* rhs_
                 A.c0 = c0;
                 A.c1 = std::min<int64_t>(na, c0 + chunk);
                 const int64_t n = A.c1 - A.c0;
-                TF_TRY(prep_order(c, A, chunk));
-                k_prep_tets<false><<<grid_for(c, n, 128), 128, 0, c->stream>>>(A);
+                k_prep_tets<<<grid_for(c, n, 128), 128, 0, c->stream>>>(A);
                 k_assemble_p2_pair<<<grid_for(c, (n + kAsmWarps - 1) / kAsmWarps, 1, 8), 32 * kAsmWarps, sm,
                                      c->stream>>>(A);
                 c->launches += 2;
@@ -1170,21 +1164,29 @@ int setup_fe_system(Context* c, unsigned forms, int rhs_kind, const double* rhs_
         } else if (!p2 && !c->asm_fp64 && !(forms & ~((1u << TF_FORM_M) | (1u << TF_FORM_A) | (1u << TF_FORM_CN))) &&
                    (rhs_kind == TF_RHS_NONE || rhs_kind == TF_RHS_CONST || rhs_kind == TF_RHS_SPHERE_XYZ)) {
             TF_TRY(ensure_tables_ff(c));
+            TF_CUDA(c, cudaGetSymbolAddress((void**)&A.tab, cT));
             const size_t sm = sizeof(AsmPair1Smem) * kAsmWarps;
             TF_CUDA(c, cudaFuncSetAttribute(k_assemble_p1_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            // per chunk of active tets: the per-tet records (one thread per tet), then the forms (warp per tet)
+            // per chunk of active tets: the linear ones, then the records of the others and their forms (warp per tet)
             const int64_t chunk = std::min<int64_t>(na, kPrepChunk);
             TF_TRY(ensure(c, c->prep1, (size_t)chunk * sizeof(TetPrep)));
+            TF_TRY(ensure(c, c->prep_rest, (size_t)chunk + 1));
             A.prep = c->prep1.p;
+            int32_t* const rest = c->prep_rest.p + 1;
+            int* const nrest = c->prep_rest.p;
             for (int64_t c0 = 0; c0 < na; c0 += chunk) {
                 A.c0 = c0;
                 A.c1 = std::min<int64_t>(na, c0 + chunk);
                 const int64_t n = A.c1 - A.c0;
-                TF_TRY(prep_order(c, A, chunk));
-                k_prep_tets<true><<<grid_for(c, n, 128), 128, 0, c->stream>>>(A);
+                A.prep_count = nullptr;
+                TF_CUDA(c, cudaMemsetAsync(nrest, 0, sizeof(int), c->stream));
+                launch_p1_linear(c, A, n, rest, nrest);
+                A.prep_order = rest;
+                A.prep_count = nrest;
+                k_prep_tets<<<grid_for(c, n, 128), 128, 0, c->stream>>>(A);
                 k_assemble_p1_pair<<<grid_for(c, (n + kAsmWarps - 1) / kAsmWarps, 1, 8), 32 * kAsmWarps, sm,
                                      c->stream>>>(A);
-                c->launches += 2;
+                c->launches += 3;
             }
             --c->launches;  // counted per chunk above
         } else if (p2) {

@@ -110,11 +110,11 @@ __device__ __forceinline__ ff ff_rsqrt(ff s) {
 // FP32 normal range (the result is then below 2^-50)
 __device__ __forceinline__ ff ff_sqrt(ff s) { return s.h > 7.8886091e-31f ? ff_mul(s, ff_rsqrt(s)) : ff_of(0.f); }
 
-// double -> pair.  Integer path (no conversion, which GB300 runs on its
+// double -> pair without an FP64 instruction (GB300 runs conversions on its
 // narrow FP64 pipe): hi = the top 24 significand bits (truncated), lo = the
-// remaining 29 bits normalised and truncated to 24, |x - hi - lo| <= 2^-47 |x|;
-// valid while lo is a normal float (|x| in [2^-74, 2^100]).  Outside that
-// range (and for non-finite x) the conversions of the FP64 pipe.
+// remaining 29 bits, an integer, rounded to a float and scaled by a power of
+// two, |x - hi - lo| <= 2^-48 |x|; valid while lo is a normal float (|x| in
+// [2^-74, 2^100]).  Outside that range (and for non-finite x) the conversions.
 __device__ __forceinline__ ff ff_split(double x) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     if ((b << 1) == 0ull) return ff{0.f, 0.f};
@@ -126,14 +126,9 @@ __device__ __forceinline__ ff ff_split(double x) {
     const unsigned long long mant = b & 0xfffffffffffffull;
     const unsigned hb = sgn | ((e - 896u) << 23) | (unsigned)(mant >> 29);
     const unsigned rem = (unsigned)(mant & 0x1fffffffu);
-    unsigned lb = 0u;
-    if (rem) {
-        const int lz = __clz((int)rem);          // >= 3
-        const unsigned p = 31u - (unsigned)lz;   // leading bit of rem
-        const unsigned m23 = (unsigned)((((unsigned long long)rem << (lz + 1)) & 0xffffffffull) >> 9);
-        lb = sgn | ((p + e - 948u) << 23) | m23;  // rem * 2^(e - 1075)
-    }
-    return ff{__int_as_float((int)hb), __int_as_float((int)lb)};
+    // rem * 2^(e - 1075), signed
+    const float lo = __fmul_rn(__uint2float_rn(rem), __int_as_float((int)(sgn | ((e - 948u) << 23))));
+    return ff{__int_as_float((int)hb), lo};
 }
 
 // pair -> double (two conversions and an add on the FP64 pipe)

@@ -14,7 +14,7 @@
 // residual algorithms", 2021).  An Arnoldi step is
 //   1. w = B v_i on the block's rows, dots of w and of v_i with every basis
 //      vector (row i of L comes from the same read of the basis); reduction of
-//      2 i + 1 values;
+//      2 i + 2 values;
 //   2. h by forward substitution in every block, w -= V h, |w|^2; reduction of
 //      one value, which is also the barrier before others gather w; Givens
 //      rotation and stopping test in every block on identical values.

@@ -200,6 +200,26 @@ __device__ inline void mesh_coord(const MeshView& M, int32_t v, double x[3]) {
     brick_coord(M.b, v, x);
 }
 
+// mesh_tet and mesh_coord of its vertices: one search of the batch for all of
+// them, and one copy of the index arithmetic (the four inlined copies of
+// mesh_coord are 40 KB of code in a kernel that runs once per tet).
+__device__ inline void mesh_tet_points(const MeshView& M, int64_t t, int32_t v[4], int32_t e[6], double X[4][3]) {
+    if (M.explicit_mesh) {
+        for (int k = 0; k < 4; ++k) v[k] = M.tet_v[4 * t + k];
+        for (int k = 0; k < 6; ++k) e[k] = M.tet_e[6 * t + k];
+        for (int k = 0; k < 4; ++k)
+            for (int c = 0; c < 3; ++c) X[k][c] = M.coords[3 * (int64_t)v[k] + c];
+        return;
+    }
+    const BatchBrick* I = nullptr;
+    if (M.nbatch) I = M.batch + batch_find(M.tstart, M.nbatch, t);
+    const Brick& B = I ? I->b : M.b;
+    const int32_t v0 = I ? I->v0 : 0;
+    brick_tet(B, I ? t - I->t0 : t, v0, I ? I->e0 : 0, v, e);
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) brick_coord(B, v[k] - v0, X[k]);
+}
+
 // ---------------------------------------------------------------------------
 // device buffers
 // ---------------------------------------------------------------------------
@@ -407,10 +427,7 @@ struct Context {
     DBuf<double> qq_grad;  // isoparametric P2: recovered level-set gradient per interface DOF
     DBuf<double> qq_base;   // isoparametric P2: per cut tet its data, per quadrature point the base point and the point data
     DBuf<int32_t> qq_idx;   // isoparametric P2: points per tet, their offsets, each point's tet
-    DBuf<uint32_t> prep_key;      // pair forms: sort keys of the prep threads (2 x chunk)
-    DBuf<int32_t> prep_idx;       // and their tets (2 x chunk)
-    DBuf<unsigned char> prep_tmp;
-    bool prep_sort = true;        // prep threads ordered by the tets' sign patterns
+    DBuf<int32_t> prep_rest;      // P1 pair forms: count and list of a chunk's tets with a level set that is not linear
     DBuf<unsigned char> prep1;  // P1 pair forms: per-tet records of one chunk of active tets
     DBuf<double> ch_prev, ch_x1, ch_x2;  // adaptive BDF1/BDF2: chi_prev, BDF1 and BDF2 states
     DBuf<float> ch_xyz, ch_nrm, ch_Y, ch_pred;
