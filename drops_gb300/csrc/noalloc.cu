@@ -21,17 +21,22 @@
 
 #include <mutex>
 
-#include "../../include/tracefem.h"
+#include "krylov_dev.cuh"
 
 namespace {
 
-// work vectors r, z, p0, p1, q, diag (6 per row), per-block partials, control words
-constexpr int kThreads = 256;
-constexpr int kMaxBlocksPerSm = 8;
-constexpr int kMaxSms = 256;
+using tf::GridAR;
+using tf::PackedAR;
+using tf::PkState;
+
+// control words, words of the packed reductions, the partials of grid_allreduce, work vectors r, z, p0, p1, q,
+// 1 / diag (6 per row)
+constexpr int kThreads = 512;
+constexpr int kMaxBlocks = tf::kPkMaxBlocks;
 constexpr int64_t kCtrlDoubles = 64;
-constexpr int64_t kPartDoubles = (int64_t)kMaxSms * kMaxBlocksPerSm * 3 * 2;
-constexpr int64_t kScratchDoubles = kCtrlDoubles + kPartDoubles + 6 * (int64_t)TF_NOALLOC_MAX_ROWS;
+constexpr int64_t kWordDoubles = 2 * 2 * tf::kPkWords;
+constexpr int64_t kPartDoubles = 2 * (int64_t)kMaxBlocks * tf::kArMax;
+constexpr int64_t kScratchDoubles = kCtrlDoubles + kWordDoubles + kPartDoubles + 6 * (int64_t)TF_NOALLOC_MAX_ROWS;
 
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
@@ -53,14 +58,8 @@ int scratch_for_current_device(double** out) {
     return TF_OK;
 }
 
-// ---- warp sums and a bounded grid barrier -----------------------------------------
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 struct Ctrl {
-    unsigned count, gen;
+    unsigned long long count;
     int status, iters;
     double resid;
     int converged;
@@ -73,75 +72,6 @@ __device__ void finish(Ctrl* ctl, int iters, double resid, bool converged) {
         ctl->resid = resid;
         ctl->converged = converged ? 1 : 0;
     }
-}
-
-__device__ bool barrier(Ctrl* ctl) {
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned* vgen = &ctl->gen;
-        const unsigned my = *vgen;
-        __threadfence();
-        if (atomicAdd(&ctl->count, 1u) == gridDim.x - 1) {
-            ctl->count = 0;
-            __threadfence();
-            atomicAdd(&ctl->gen, 1u);
-        } else {
-            long long spins = 0;
-            while (*vgen == my) {
-                if (++spins > 20000000LL) {
-                    atomicCAS(&ctl->status, 0, TF_ERR_WATCHDOG);
-                    break;
-                }
-                if (spins > 64) __nanosleep(64);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return *((volatile int*)&ctl->status) == 0;
-}
-
-template <int NV>
-__device__ void partials(double (&v)[NV], double* part) {
-    __shared__ double red[NV][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = 0; k < NV; ++k) {
-        const double x = warp_sum(v[k]);
-        if (lane == 0) red[k][w] = x;
-    }
-    __syncthreads();
-    if (w == 0)
-        for (int k = 0; k < NV; ++k) {
-            double x = lane < nw ? red[k][lane] : 0.;
-            x = warp_sum(x);
-            if (lane == 0) part[(size_t)blockIdx.x * NV + k] = x;
-        }
-    __syncthreads();
-}
-
-// every block sums all partials in the same fixed order
-template <int NV>
-__device__ void reduce_all(const double* part, double (&out)[NV]) {
-    __shared__ double red[NV][32];
-    __shared__ double res[NV];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int k = 0; k < NV; ++k) {
-        double x = 0.;
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) x += __ldcg(part + (size_t)b * NV + k);
-        x = warp_sum(x);
-        if (lane == 0) red[k][w] = x;
-    }
-    __syncthreads();
-    if (w == 0)
-        for (int k = 0; k < NV; ++k) {
-            double x = lane < nw ? red[k][lane] : 0.;
-            x = warp_sum(x);
-            if (lane == 0) res[k] = x;
-        }
-    __syncthreads();
-    for (int k = 0; k < NV; ++k) out[k] = res[k];
-    __syncthreads();
 }
 
 // ---- persistent PCG on CSR, G lanes per row ---------------------------------------
@@ -158,87 +88,122 @@ struct Args {
     int rel;
 };
 
+// The rows go round-robin over the blocks, a warp's share at a time (small systems
+// use every SM); a lane keeps eight entries in flight.  p = z + beta p is formed in
+// the gathers, so an iteration has two grid steps, both packed integer reductions
+// (krylov_dev.cuh).  Bound by latency below some 20,000 rows (two reductions, about
+// 3 us, and the dependent trips to L2), by the FP64 pipe above: 21 instructions per
+// row of a 7-point matrix on one lane, where G = 8 lanes issued their butterfly sums
+// for 4 rows at a time.  Per iteration of a 7-point matrix, call included: 512 rows
+// 16.1 -> 8.5 us, 8,000 23.0 -> 8.8, 65,231 34.4 -> 10.7, 238,328 70.4 -> 20.1 (before: 8
+// lanes per row, up to 8 blocks of 256 per SM, counter barriers and FP64 tree sums).
 template <int G>
-__global__ void __launch_bounds__(kThreads) k_pcg_noalloc(Args a) {
+__global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(Args a) {
     const int64_t m = a.m;
     Ctrl* ctl = reinterpret_cast<Ctrl*>(a.scratch);
-    // Partials alternate between two buffers, one per reduction in turn (set-up: B;
-    // each iteration: A then B).  A block may only rewrite a buffer after every
-    // block has passed the barrier that follows its last read of that buffer.
-    double* partA = a.scratch + kCtrlDoubles;
-    double* partB = partA + (size_t)gridDim.x * 3;
-    double* r = a.scratch + kCtrlDoubles + kPartDoubles;
+    unsigned long long* const words = reinterpret_cast<unsigned long long*>(a.scratch + kCtrlDoubles);
+    const GridAR g{&ctl->count, nullptr, a.scratch + kCtrlDoubles + kWordDoubles, &ctl->status};
+    const PackedAR pa{words, &ctl->status}, pb{words + 2 * tf::kPkWords, &ctl->status};
+    PkState ka, kb;
+    unsigned long long epoch = 0;
+    double* r = a.scratch + kCtrlDoubles + kWordDoubles + kPartDoubles;
     double* z = r + m;
     double* p0 = z + m;
     double* p1 = p0 + m;
     double* q = p1 + m;
     double* d = q + m;
     const int lane = threadIdx.x & 31, sub = lane & (G - 1);
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarp = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
+    const int64_t first = ((threadIdx.x >> 5) * (int64_t)gridDim.x + blockIdx.x) * (32 / G) + lane / G;
+    const int64_t step = (int64_t)gridDim.x * kThreads / G;
+    __shared__ double sh[3];
+
+    // sum over the entries of a row of f(column, value), all lanes of the warp
+    auto row_sum = [&](int64_t row, auto load, auto term) {
+        constexpr int U = 8;
+        double acc = 0.;
+        int32_t s = 0, e = 0;
+        if (row < m) {
+            s = __ldg(a.rowptr + row) + sub;
+            e = __ldg(a.rowptr + row + 1);
+        }
+        for (int32_t k = s; k < e; k += U * G) {
+            int32_t c[U];
+            double v[U];
+            decltype(load(0)) x[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool in = k + u * G < e;
+                c[u] = in ? __ldg(a.colind + k + u * G) : 0;
+                v[u] = in ? __ldg(a.vals + k + u * G) : 0.;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k + u * G < e) x[u] = load(c[u]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k + u * G < e) acc = term(acc, c[u], v[u], x[u]);
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
+        return acc;
+    };
+    const int64_t rounds = (m + step - 1) / step;  // the warps of a block make the same number of passes
 
     // diagonal (row scan, SolveGSstep<PB_JAC0>), r = b - A x, z = r/d, p0 = z
     {
         double v[3] = {0., 0., 0.};
-        for (int64_t base = warp * (32 / G); base < m; base += nwarp * (32 / G)) {
-            const int64_t row = base + lane / G;
-            int32_t s = 0, e = 0;
-            if (row < m) {
-                s = a.rowptr[row];
-                e = a.rowptr[row + 1];
-            }
-            double acc = 0., dg = 0.;
-            for (int32_t k = s + sub; k < e; k += G) {
-                const int32_t c = a.colind[k];
-                acc += a.vals[k] * __ldcg(a.x + c);
-                if (c == row) dg = a.vals[k];
-            }
-            for (int o = G / 2; o > 0; o >>= 1) {
-                acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
-                dg += __shfl_xor_sync(0xffffffffu, dg, o, G);
-            }
+        for (int64_t k = 0; k < rounds; ++k) {
+            const int64_t row = first + k * step;
+            double dg = 0.;
+            const double acc = row_sum(
+                row, [&](int32_t c) { return __ldcg(a.x + c); },
+                [&](double s, int32_t c, double av, double x) {
+                    if (c == row) dg = av;
+                    return s + av * x;
+                });
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, o, G);
             if (sub == 0 && row < m) {
-                const double ri = a.b[row] - acc, zi = ri / dg;
-                d[row] = dg;
+                const double bi = a.b[row], ri = bi - acc, di = 1.0 / dg, zi = ri * di;
+                d[row] = di;
                 r[row] = ri;
                 z[row] = zi;
                 p0[row] = zi;
                 v[0] += ri * ri;
-                v[1] += a.b[row] * a.b[row];
+                v[1] += bi * bi;
                 v[2] += zi * ri;
             }
         }
-        partials<3>(v, partB);
+        double o[3];
+        if (!tf::grid_allreduce<double, 3>(g, epoch, v, o)) return;
+        if (threadIdx.x == 0) {
+            double nb = sqrt(o[1]);
+            if (nb == 0.0 || !a.rel) nb = 1.0;
+            sh[0] = nb;
+            sh[1] = sqrt(o[0]) / nb;
+            sh[2] = o[2];
+        }
+        __syncthreads();
     }
-    if (!barrier(ctl)) return;
-    double s0[3];
-    reduce_all<3>(partB, s0);
-    double normb = sqrt(s0[1]);
-    if (normb == 0.0 || !a.rel) normb = 1.0;
-    double resid = sqrt(s0[0]) / normb, rho = s0[2], beta = 0.;
+    const double normb = sh[0];
+    double resid = sh[1], rho = sh[2], beta = 0.;
     if (resid <= a.tol || a.max_iter == 0) {
         finish(ctl, 0, resid, resid <= a.tol);
         return;
     }
+    struct Pair {
+        double z, p;
+    };
     double* pc = p0;
     double* pn = p1;
     for (int it = 1; it <= a.max_iter; ++it) {
         {
-            double v[1] = {0.};
-            for (int64_t base = warp * (32 / G); base < m; base += nwarp * (32 / G)) {
-                const int64_t row = base + lane / G;
-                int32_t s = 0, e = 0;
-                if (row < m) {
-                    s = a.rowptr[row];
-                    e = a.rowptr[row + 1];
-                }
-                double acc = 0.;
-                for (int32_t k = s + sub; k < e; k += G) {
-                    const int32_t c = a.colind[k];
-                    acc += a.vals[k] * (__ldcg(z + c) + beta * __ldcg(pc + c));
-                }
-                for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
+            double v[1] = {0.}, o[1];
+            for (int64_t k = 0; k < rounds; ++k) {
+                const int64_t row = first + k * step;
+                const double acc = row_sum(
+                    row, [&](int32_t c) { return Pair{__ldcg(z + c), __ldcg(pc + c)}; },
+                    [&](double s, int32_t, double av, const Pair& x) { return s + av * (x.z + beta * x.p); });
                 if (sub == 0 && row < m) {
                     const double pi = __ldcg(z + row) + beta * __ldcg(pc + row);
                     pn[row] = pi;
@@ -246,36 +211,41 @@ __global__ void __launch_bounds__(kThreads) k_pcg_noalloc(Args a) {
                     v[0] += acc * pi;
                 }
             }
-            partials<1>(v, partA);
+            if (!tf::packed_allreduce<1>(pa, ka, g, epoch, v, o, false)) return;
+            if (threadIdx.x == 0) sh[0] = rho / o[0];
+            __syncthreads();
         }
-        if (!barrier(ctl)) return;
-        double lam[1];
-        reduce_all<1>(partA, lam);
-        const double alpha = rho / lam[0];
+        const double alpha = sh[0];
         {
-            double v[2] = {0., 0.};
-            for (int64_t i = tid; i < m; i += nth) {
-                a.x[i] += alpha * __ldcg(pn + i);
-                const double ri = r[i] + (-alpha) * __ldcg(q + i);
-                const double zi = ri / __ldcg(d + i);
-                r[i] = ri;
-                z[i] = zi;
-                v[0] += ri * ri;
-                v[1] += zi * ri;
+            // the rows of the product, by the same threads
+            double v[2] = {0., 0.}, o[2];
+            for (int64_t k = 0; k < rounds; ++k) {
+                const int64_t row = first + k * step;
+                if (sub == 0 && row < m) {
+                    a.x[row] += alpha * pn[row];
+                    const double ri = r[row] - alpha * q[row];
+                    const double zi = ri * d[row];
+                    r[row] = ri;
+                    z[row] = zi;
+                    v[0] += ri * ri;
+                    v[1] += zi * ri;
+                }
             }
-            partials<2>(v, partB);
+            if (!tf::packed_allreduce<2>(pb, kb, g, epoch, v, o, true)) return;
+            if (threadIdx.x == 0) {
+                sh[1] = sqrt(o[0]) / normb;
+                sh[2] = o[1];
+                sh[0] = o[1] / rho;
+            }
+            __syncthreads();
         }
-        if (!barrier(ctl)) return;
-        double s2[2];
-        reduce_all<2>(partB, s2);
-        resid = sqrt(s2[0]) / normb;
+        resid = sh[1];
         if (resid <= a.tol || it == a.max_iter) {
             finish(ctl, it, resid, resid <= a.tol);
             return;
         }
-        const double rho1 = rho;
-        rho = s2[1];
-        beta = rho / rho1;
+        rho = sh[2];
+        beta = sh[0];
         double* t = pc;
         pc = pn;
         pn = t;
@@ -301,19 +271,17 @@ extern "C" int tf_pcg_jacobi_noalloc(int64_t m, const int32_t* rowptr, const int
         cudaStreamSynchronize(s) != cudaSuccess)
         return TF_ERR_CUDA;
     const double avg = (double)nnz / (double)m;
-    const int G = avg <= 6 ? 4 : avg <= 12 ? 8 : avg <= 24 ? 16 : 32;
-    const void* fn = G == 4 ? (const void*)k_pcg_noalloc<4> : G == 8 ? (const void*)k_pcg_noalloc<8>
-                   : G == 16 ? (const void*)k_pcg_noalloc<16> : (const void*)k_pcg_noalloc<32>;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, 0) != cudaSuccess || per_sm < 1)
-        return TF_ERR_CUDA;
-    if (per_sm > kMaxBlocksPerSm) per_sm = kMaxBlocksPerSm;
-    if (sms > kMaxSms) sms = kMaxSms;
-    int64_t want = (m * G + kThreads - 1) / kThreads;
-    int blocks = (int)(want < (int64_t)per_sm * sms ? want : (int64_t)per_sm * sms);
+    // long rows are spread over lanes; 152 x 512 lanes hold 77,824 rows
+    const int G = avg <= 32 ? 1 : avg <= 128 ? 8 : 32;
+    const void* fn = G == 1 ? (const void*)k_pcg_noalloc<1> : G == 8 ? (const void*)k_pcg_noalloc<8>
+                                                                     : (const void*)k_pcg_noalloc<32>;
+    if (sms > kMaxBlocks) sms = kMaxBlocks;
+    // at least four warps per block
+    const int64_t want = (m * G + 127) / 128;
+    int blocks = (int)(want < sms ? want : sms);
     if (blocks < 1) blocks = 1;
     // the control words must start at zero; everything else is written before it is read
-    if (cudaMemsetAsync(scratch, 0, sizeof(double) * kCtrlDoubles, s) != cudaSuccess) return TF_ERR_CUDA;
+    if (cudaMemsetAsync(scratch, 0, sizeof(double) * (kCtrlDoubles + kWordDoubles), s) != cudaSuccess) return TF_ERR_CUDA;
     Args a{m, rowptr, colind, vals, b, x, scratch, *max_iter, *tol, rel};
     void* args[] = {&a};
     if (cudaLaunchCooperativeKernel(fn, blocks, kThreads, args, 0, s) != cudaSuccess) return TF_ERR_CUDA;
