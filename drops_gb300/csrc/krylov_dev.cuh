@@ -1035,9 +1035,51 @@ __device__ __forceinline__ void sell_block_walk_range(BalShared<NW, T, MAXS>& sh
     __syncthreads();  // emits visible to the block; sh.tail free for the next call
 }
 
+// The same for a single walk: without the searches for the end of the range.
 template <int NW, class T, int MAXS, class ROW, class EMIT>
 __device__ __forceinline__ void sell_block_walk_fn(BalShared<NW, T, MAXS>& sh, int64_t s0, int S, ROW row, EMIT emit) {
-    sell_block_walk_range(sh, s0, S, sell_block_range(sh, S), row, emit);
+    const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
+    const int32_t Tot = sh.P[S];
+    const int32_t g0 = (int32_t)((int64_t)j * Tot / NW), g1 = (int32_t)((int64_t)(j + 1) * Tot / NW);
+    // first slice that overlaps [g0, ..) or starts at g0 (zero width included)
+    int lo = 0, hi = S;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (sh.P[mid + 1] > g0 || sh.P[mid] >= g0) hi = mid;
+        else lo = mid + 1;
+    }
+    T head = T(0);
+    int hslice = -1;
+    for (int i = lo; i < S; ++i) {
+        const int32_t pa = sh.P[i], pb = sh.P[i + 1];
+        if (!(pa < g1 || (j == NW - 1 && pa == Tot))) break;
+        const int32_t c0 = g0 > pa ? g0 - pa : 0;
+        const int32_t c1 = (g1 < pb ? g1 : pb) - pa;
+        const T acc = row(s0 + i, c0, c1 > c0 ? c1 - c0 : 0);
+        const bool starts = pa >= g0, ends = pb <= g1;
+        if (starts && ends) {
+            emit(s0 + i, acc);
+        } else if (ends) {
+            head = acc;
+            hslice = i;
+        } else {
+            sh.tail[j][lane] = acc;
+        }
+    }
+    __syncthreads();
+    if (hslice >= 0) {
+        // warps from the one holding the slice's first column up to this one
+        const int32_t pa = sh.P[hslice];
+        int ja = j - 1;
+        while (ja > 0 && (int32_t)((int64_t)ja * Tot / NW) > pa) --ja;
+        T sum = T(0);
+        for (int jj = ja; jj < j; ++jj) {
+            const int32_t a0 = (int32_t)((int64_t)jj * Tot / NW), a1 = (int32_t)((int64_t)(jj + 1) * Tot / NW);
+            if (a1 > a0) sum = sum + sh.tail[jj][lane];
+        }
+        emit(s0 + hslice, sum + head);
+    }
+    __syncthreads();  // emits visible to the block; sh.tail free for the next call
 }
 
 template <int NW, class T, class XL, class EMIT>
