@@ -609,14 +609,6 @@ __device__ __forceinline__ ff ff_rhs_sphere(const ff ctr[3], ff R, ff amp, const
     return ff_mul(ff_mul(ff_mul(amp, y[0]), y[1]), y[2]);
 }
 
-// pair -> double with one FP64 instruction: both parts widened on the integer pipe
-__device__ __forceinline__ double widen_f32(float x) {
-    const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
-    if (e - 1u >= 254u) return (b << 1) == 0u ? 0.0 : (double)x;
-    return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20 | (b & 0x7fffffu) >> 3)), (int)(b << 29));
-}
-__device__ __forceinline__ double ff_widen(ff a) { return __dadd_rn(widen_f32(a.h), widen_f32(a.l)); }
-
 template <int G>
 __device__ __forceinline__ ff lane_group_sum(ff a) {
 #pragma unroll

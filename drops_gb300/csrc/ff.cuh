@@ -134,4 +134,20 @@ __device__ __forceinline__ ff ff_split(double x) {
 // pair -> double (two conversions and an add on the FP64 pipe)
 __device__ __forceinline__ double ff_to_double(ff a) { return __dadd_rn((double)a.h, (double)a.l); }
 
+// float -> double on the integer pipe (the conversion instruction holds the FP64 pipe)
+__device__ __forceinline__ double widen_f32(float x) {
+    const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
+    if (e - 1u >= 254u) return (b << 1) == 0u ? 0.0 : (double)x;
+    return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20 | (b & 0x7fffffu) >> 3)), (int)(b << 29));
+}
+// pair -> double with one FP64 instruction
+__device__ __forceinline__ double ff_widen(ff a) { return __dadd_rn(widen_f32(a.h), widen_f32(a.l)); }
+
+// x 2^e, exact where the result is normal
+__device__ __forceinline__ double scale_pow2(double x, int e) {
+    const int hi = __double2hiint(x), ex = hi >> 20 & 0x7ff, to = ex + e;
+    if (ex == 0 || ex == 2047 || to <= 0 || to >= 2047) return scalbn(x, e);
+    return __hiloint2double(hi + (e << 20), __double2loint(x));
+}
+
 }  // namespace tf

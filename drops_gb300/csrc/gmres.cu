@@ -162,7 +162,8 @@ __device__ void ls_sum_parts(const V* part, int n, V* grp, V* tot) {
     __syncthreads();
 }
 
-template <class V>
+// SMEM: the block's parts of w and v_i lie in shared memory (a pointer to either would make every access generic)
+template <class V, bool SMEM>
 __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
     constexpr bool kMixed = sizeof(V) == 4;
     extern __shared__ __align__(16) unsigned char ls_dyn[];
@@ -176,13 +177,17 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
     const int64_t s1 = (int64_t)(blockIdx.x + 1) * a.nslices / gridDim.x;
     const int64_t base = s0 * 32;
     const int nl = (int)(s1 - s0) * 32;
-    const bool smem = a.nloc > 0;
     const int R = a.R;
     unsigned long long epoch = 0;
     int it = 0, cycles = 0;  // Arnoldi steps, cycles
     // a run of at most kBalMaxSlices slices plans its column split once
     const bool planned = s1 - s0 <= kBalMaxSlices;
-    if (planned) sell_block_plan<kLsWarps, V>(bsh, a.ptr, s0, (int)(s1 - s0));
+    __shared__ WalkRange wrs[kLsWarps];
+    if (planned) {
+        sell_block_plan<kLsWarps, V>(bsh, a.ptr, s0, (int)(s1 - s0));
+        if (lane == 0) wrs[warp] = sell_block_range(bsh, (int)(s1 - s0));
+        __syncwarp();
+    }
 
     // one reduction: the block's n partials are in part[epoch & 1][block]
     auto reduce = [&](int n) -> bool {
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                             }
                         }
                         V0[(s - s0) * 32 + lane] = (V)r;
-                        if (smem) sbuf[(s - s0) * 32 + lane] = (V)r;
+                        if (SMEM) sbuf[(s - s0) * 32 + lane] = (V)r;
                         v[0] += r * r;
                         if (first) v[1] += bi * bi;
                     });
@@ -260,19 +265,27 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
         const int steps = kMixed ? R : R - 1;
         bool done = false;
         int i = 0;
-        V* ws = smem ? sbuf + a.nloc : nullptr;  // this block's part of w, then of the next v_i
-        V* vs = smem ? sbuf : nullptr;           // of v_i
+        V* ws = SMEM ? sbuf + a.nloc : nullptr;  // this block's part of w, then of the next v_i
+        V* vs = SMEM ? sbuf : nullptr;           // of v_i
         while (i < steps && it < a.max_iter) {
             const V* const Vi = a.basis + (size_t)i * a.ld;
             V* const W = a.basis + (size_t)(i + 1) * a.ld;
             const V sci = q.scl[i];
-            V* const wl = smem ? ws : W + base;
-            const V* const vl = smem ? vs : Vi + base;
+            V* const wl = SMEM ? ws : W + base;
+            const V* const vl = SMEM ? vs : Vi + base;
             for (int64_t c0 = s0; c0 < s1; c0 += kBalMaxSlices) {
                 const int S = (int)(s1 - c0 < kBalMaxSlices ? s1 - c0 : kBalMaxSlices);
-                if (!planned) sell_block_plan<kLsWarps, V>(bsh, a.ptr, c0, S);
-                sell_block_walk<kLsWarps, V>(
-                    bsh, a.ptr, a.cols, a.bval, c0, S, [&](int32_t j) { return kld(Vi + j); },
+                if (!planned) {
+                    sell_block_plan<kLsWarps, V>(bsh, a.ptr, c0, S);
+                    if (lane == 0) wrs[warp] = sell_block_range(bsh, S);
+                    __syncwarp();
+                }
+                sell_block_walk_range(
+                    bsh, c0, S, wrs[warp],
+                    [&](int64_t s, int32_t k, int32_t n) {
+                        return sell_row_range<V>(a.ptr, a.cols, a.bval, s, lane, k, n, [&](int32_t j) { return kld(Vi + j); },
+                                                 SellCache<V>());
+                    },
                     [&](int64_t s, V acc) { wl[(s - s0) * 32 + lane] = sci * acc; });
             }
             // Dots of w and v_i with the basis: a warp takes four basis vectors and, while there are
@@ -442,7 +455,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                 for (; k <= i; ++k) acc[k & 3] -= q.coef[k] * kld(vk + (size_t)k * a.ld);
                 const V w = (acc[0] + acc[1]) + (acc[2] + acc[3]);
                 W[base + e] = w;
-                if (smem) ws[e] = w;
+                if (SMEM) ws[e] = w;
                 nrm[0] += w * w;
             }
             V o[1];
@@ -480,7 +493,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
             resid = q.resid;
             done = q.flag != 0;
             ++i;
-            if (smem) {
+            if (SMEM) {
                 V* t = ws;
                 ws = vs;
                 vs = t;
@@ -584,7 +597,7 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     const V* bval = nullptr;
     TF_TRY(gmres_operator<V>(c, A, left, &bval));
     TimedLaunch tl(c, TF_K_GMRES);
-    const int64_t ns = A.sell.nslices, ld = ns * 32;
+    const int64_t ns = A.sell.used, ld = ns * 32;
     // at least two slices per block: a block's share of the reductions (its
     // partials are read by every other block) outweighs less work per block
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(c->num_sms, kPkMaxBlocks), ns / 2));
@@ -599,10 +612,9 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
     unsigned long long* pw = nullptr;
     TF_TRY(packed_words(c, 2, &pw));
-    const void* fn = (const void*)k_gmres_ls<V>;
     cudaFuncAttributes fa{};
     int optin = 0;
-    TF_CUDA(c, cudaFuncGetAttributes(&fa, fn));
+    TF_CUDA(c, cudaFuncGetAttributes(&fa, (const void*)k_gmres_ls<V, true>));
     TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     const int64_t room = (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024;
     const size_t small = (sizeof(LsSmall<V>) + 15) & ~(size_t)15;
@@ -610,6 +622,7 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     const int64_t both = (int64_t)small + 2 * run * (int64_t)sizeof(V);
     const bool smem = both <= room;  // else w and v_i are read from the basis
     const size_t dyn = smem ? (size_t)both : small;
+    const void* fn = smem ? (const void*)k_gmres_ls<V, true> : (const void*)k_gmres_ls<V, false>;
     TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     int per_sm = 0;
     TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLsThreads, dyn));

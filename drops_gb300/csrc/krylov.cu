@@ -145,6 +145,7 @@ int ensure_sell(Context* c, CSR& A, bool fp32) {
         ++c->launches;
         TF_CUDA(c, cudaGetLastError());
         S.nslices = ns;
+        S.used = (A.m + 31) / 32;
         S.npad = npad;
         S.perm = c->sell_perm[id].p;
         S.ptr = c->sell_ptr[id].p;
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_spmv_bal(int64_t nslices, con
 }
 
 void launch_spmv_shape(Context* c, const CSR& A, const double* x, double* y, int threads, int per_sm) {
-    const int64_t ns = A.sell.nslices;
+    const int64_t ns = A.sell.used;
     int64_t nb = (int64_t)c->num_sms * per_sm;
     if (nb > ns) nb = ns;
     if (nb < 1) nb = 1;
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                 },
                 [&](int64_t s, Pair2 q) {
                     const int32_t row = __ldg(perm + s * 32 + lane);
-                    if (row >= 0) y[row] = ((double)q.h + (double)q.l) * pow2(__ldg(rexp + s * 32 + lane));
+                    if (row >= 0) y[row] = scale_pow2(ff_widen(ff{q.h, q.l}), __ldg(rexp + s * 32 + lane));
                 });
         }
     }
@@ -461,7 +462,7 @@ int spmv(Context* c, const CSR& Ac, const double* x, double* y) {
         TF_TRY(ensure(c, c->x_pairs, (size_t)(A.m > 0 ? A.m : 1)));
         TF_CUDA(c, cudaMemsetAsync(c->status.p + 2, 0, sizeof(int), c->stream));
         k_split_x_int<<<grid_for(c, A.m), kBlock, 0, c->stream>>>(A.m, x, c->x_pairs.p, c->status.p + 2);
-        const int64_t ns = A.sell.nslices;
+        const int64_t ns = A.sell.used;
         int64_t nb = (int64_t)c->num_sms * 2;
         if (nb > ns) nb = ns;
         if (nb < 1) nb = 1;

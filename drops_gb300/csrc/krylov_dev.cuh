@@ -2,6 +2,7 @@
 // barriers, fixed-order reductions, the scalar state of a solve and the
 // SELL row product.
 #pragma once
+#include "ff.cuh"
 #include "tf_internal.cuh"
 
 namespace tf {
@@ -1104,10 +1105,10 @@ __device__ __forceinline__ void sell_block_balanced(BalShared<NW, T>& sh, const 
 }
 
 // n columns of one slot row: translated columns cp[32 k] (shared memory),
-// values vp[32 k] (shared memory when vsh, else global), vector xs (shared
-// memory).  Terms are summed in column order.
-template <class T>
-__device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* __restrict__ vp, bool vsh, int32_t n,
+// values vp[32 k] (shared memory when VSH, else global: a pointer to either makes
+// every load generic), vector xs (shared memory).  Terms are summed in column order.
+template <bool VSH, class T>
+__device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* __restrict__ vp, int32_t n,
                                      const T* __restrict__ xs) {
     constexpr int U = 8;
     T acc = T(0);
@@ -1116,7 +1117,7 @@ __device__ __forceinline__ T res_row(const uint16_t* __restrict__ cp, const T* _
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (k + u < n) {
-                vv[u] = vsh ? vp[32 * (k + u)] : __ldg(vp + 32 * (k + u));
+                vv[u] = VSH ? vp[32 * (k + u)] : __ldg(vp + 32 * (k + u));
                 xv[u] = xs[cp[32 * (k + u)]];
             } else {
                 vv[u] = T(0);

@@ -282,7 +282,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
                     const int i = (int)(s - sb0);
                     const int32_t p0 = 32 * (bsh.P[i] + c0) + lane;
                     const bool vsh = 32 * bsh.P[i + 1] <= a.vcap;
-                    return res_row<T>(ccol + p0, vsh ? cval + p0 : a.val + pb + p0, vsh, n, Us);
+                    return vsh ? res_row<true, T>(ccol + p0, cval + p0, n, Us)
+                               : res_row<false, T>(ccol + p0, a.val + pb + p0, n, Us);
                 },
                 [&](int64_t s, T val) { emit((int)(s - sb0) * 32 + lane, val); });
         };
@@ -479,7 +480,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
                 const int i = (int)(s - sb0);
                 const int32_t p0 = 32 * (bsh.P[i] + c0) + lane;
                 const bool vsh = 32 * bsh.P[i + 1] <= a.vcap;
-                return res_row<double>(ccol + p0, vsh ? cval + p0 : a.val + pb + p0, vsh, n, Ps);
+                return vsh ? res_row<true, double>(ccol + p0, cval + p0, n, Ps)
+                           : res_row<false, double>(ccol + p0, a.val + pb + p0, n, Ps);
             },
             [&](int64_t s, double val) {
                 const int ls = (int)(s - sb0) * 32 + lane;
@@ -701,7 +703,7 @@ int ensure_res_plan(Context* c, CSR& A, int blocks) {
         TF_CUDA(c, cudaMemsetAsync(c->kry_iters.p, 0, 4 * sizeof(int), c->stream));
         const size_t hsm = sizeof(int32_t) * (kHashSlots + kHaloMax);
         TF_CUDA(c, cudaFuncSetAttribute((const void*)k_res_halo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
-        k_res_halo<<<blocks, 512, hsm, c->stream>>>(S.ptr, S.nslices, S.col, S.iperm, S.col_tr, S.halo_slots, S.halo_n,
+        k_res_halo<<<blocks, 512, hsm, c->stream>>>(S.ptr, S.used, S.col, S.iperm, S.col_tr, S.halo_slots, S.halo_n,
                                                     c->kry_iters.p);
         ++c->launches;
         TF_CUDA(c, cudaGetLastError());
@@ -720,7 +722,7 @@ int ensure_res_plan(Context* c, CSR& A, int blocks) {
 // Blocks of a resident solve: one per SM, and at least two slices each (a
 // smaller share saves less than another block adds to the reductions).
 int res_blocks(const Context* c, const CSR& A) {
-    return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(c->num_sms, kPkMaxBlocks), A.sell.nslices / 2));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(c->num_sms, kPkMaxBlocks), A.sell.used / 2));
 }
 
 // shared memory a block of fn can use besides its static part
@@ -802,7 +804,7 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     PcgResArgs<T> g;
     g.pk = PackedAR{pw, c->status.p};
     g.m = m;
-    g.nslices = S.nslices;
+    g.nslices = S.used;
     g.perm = S.perm;
     g.ptr = S.ptr;
     g.col = S.col;
@@ -888,7 +890,7 @@ int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter
     g.pk1 = PackedAR{pw, c->status.p};
     g.pk2 = PackedAR{pw + 2 * kPkWords, c->status.p};
     g.m = m;
-    g.nslices = S.nslices;
+    g.nslices = S.used;
     g.perm = S.perm;
     g.ptr = S.ptr;
     g.col_tr = S.col_tr;

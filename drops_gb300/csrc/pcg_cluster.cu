@@ -112,12 +112,7 @@ __device__ __forceinline__ void cl_store(const double* p, unsigned rank, double 
 __device__ __forceinline__ void cl_store(const int* p, unsigned rank, int v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cl_map(p, rank)), "r"(v) : "memory");
 }
-// float to double on the integer pipe (the conversion instruction holds the FP64 pipe)
-__device__ __forceinline__ double cl_widen(float x) {
-    const unsigned b = __float_as_uint(x), e = b >> 23 & 0xffu;
-    if (e - 1u >= 254u) return (b << 1) == 0u ? 0.0 : (double)x;
-    return __hiloint2double((int)((b & 0x80000000u) | ((e + 896u) << 20 | (b & 0x7fffffu) >> 3)), (int)(b << 29));
-}
+__device__ __forceinline__ double cl_widen(float x) { return widen_f32(x); }
 __device__ __forceinline__ double cl_widen(double x) { return x; }
 
 __host__ __device__ inline size_t cl_up(size_t b) { return (b + 127) & ~(size_t)127; }
@@ -430,7 +425,7 @@ __global__ void __launch_bounds__(kClThreads<V>, 1) k_pcg_cluster(ClArgs a) {
                     const int so = soff[s];
                     if (so >= 0) {
                         const int e = so + 32 * c0 + lane;
-                        return res_row<V>(scol + e, sval + e, true, nn, p);
+                        return res_row<true, V>(scol + e, sval + e, nn, p);
                     }
                     const int e = 32 * (bsh.P[s] + c0) + lane;
                     return cl_row<V>(gcol() + e, gval() + e, nn, p);
