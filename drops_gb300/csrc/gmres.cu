@@ -75,6 +75,7 @@ struct GmLsArgs {
     GridAR g;
     PackedAR pkd, pkn;     // dots, norm
     int R, max_iter, rel, left, nloc;  // nloc: slots of the largest run held in shared memory (0: none)
+    int ccap;              // entries of the block's part of B kept in shared memory
     double tol, inner_floor;
     int* out_iter;
     double* out_resid;
@@ -188,6 +189,19 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
         if (lane == 0) wrs[warp] = sell_block_range(bsh, (int)(s1 - s0));
         __syncwarp();
     }
+    // the head of the block's part of B in shared memory: its slices [0, cs)
+    int cs = 0;
+    V* const cval = sbuf + 2 * a.nloc;
+    int32_t* const ccol = reinterpret_cast<int32_t*>(cval + a.ccap);
+    if (SMEM && planned) {
+        const int S = (int)(s1 - s0);
+        while (cs < S && 32 * bsh.P[cs + 1] <= a.ccap) ++cs;
+        const int32_t pb = __ldg(a.ptr + s0);
+        for (int k = threadIdx.x; k < 32 * bsh.P[cs]; k += kLsThreads) {
+            cval[k] = __ldg(a.bval + pb + k);
+            ccol[k] = __ldg(a.cols + pb + k);
+        }
+    }
 
     // one reduction: the block's n partials are in part[epoch & 1][block]
     auto reduce = [&](int n) -> bool {
@@ -283,8 +297,12 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
                 sell_block_walk_range(
                     bsh, c0, S, wrs[warp],
                     [&](int64_t s, int32_t k, int32_t n) {
-                        return sell_row_range<V>(a.ptr, a.cols, a.bval, s, lane, k, n, [&](int32_t j) { return kld(Vi + j); },
-                                                 SellCache<V>());
+                        auto gather = [&](int32_t j) { return kld(Vi + j); };
+                        if (SMEM && s - s0 < cs) {
+                            const int e = 32 * (bsh.P[s - s0] + k) + lane;
+                            return sell_row_walk<true, V>(ccol + e, cval + e, n, gather);
+                        }
+                        return sell_row_range<V>(a.ptr, a.cols, a.bval, s, lane, k, n, gather);
                     },
                     [&](int64_t s, V acc) { wl[(s - s0) * 32 + lane] = sci * acc; });
             }
@@ -621,7 +639,11 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     const int64_t run = 32 * ((ns + blocks - 1) / blocks);  // slots of the largest run
     const int64_t both = (int64_t)small + 2 * run * (int64_t)sizeof(V);
     const bool smem = both <= room;  // else w and v_i are read from the basis
-    const size_t dyn = smem ? (size_t)both : small;
+    // what is left keeps the head of every block's part of B (at most the largest run, guessed at 9/8 of the mean)
+    const int64_t mean = A.sell.npad / blocks;
+    int64_t ccap = smem ? std::min((room - both) / (int64_t)(sizeof(V) + 4), mean + mean / 8 + 1024) & ~(int64_t)31 : 0;
+    if (ccap < 0) ccap = 0;
+    const size_t dyn = smem ? (size_t)(both + ccap * (int64_t)(sizeof(V) + 4)) : small;
     const void* fn = smem ? (const void*)k_gmres_ls<V, true> : (const void*)k_gmres_ls<V, false>;
     TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     int per_sm = 0;
@@ -655,6 +677,7 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     g.rel = rel;
     g.left = left;
     g.nloc = smem ? (int)run : 0;
+    g.ccap = (int)ccap;
     g.tol = *tol;
     g.inner_floor = 1e-5;
     g.out_iter = c->kry_iters.p;

@@ -96,3 +96,22 @@ def test_mixed_iterations_near_the_attainable_residual(ctx):
         its[prec] = it
     print(its)
     assert its[tf.PREC_MIXED].sum() <= 1.25 * its[tf.PREC_FP64].sum()
+
+
+@pytest.mark.parametrize("precision", [tf.PREC_FP64, tf.PREC_MIXED])
+def test_uneven_rows_beyond_the_cached_part_of_the_matrix(precision):
+    """Blocks whose share of the matrix is several times the mean keep only its head in shared memory."""
+    from tests.test_gpu_pcg_cluster import mul, spd
+
+    m = 12000
+    A = spd(m, lambda i: 30 if i < m // 10 else 0, seed=11)
+    b = A[3]
+    with tf.TraceFEM(0) as ctx:
+        ctx.matrix_upload(*A[:3])
+        ctx.vec_upload(tf.VEC_B, b)
+        ctx.vec_upload(tf.VEC_X, np.zeros(m))
+        st, it, res = ctx.gmres_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, restart=50, tol=1e-10, precision=precision)
+        assert st == tf.OK and res <= 1e-10
+        r = b - mul(A, ctx.vec_download(tf.VEC_X))
+    # the FP64 solver stops on the rotated residual, which follows the true one of a well conditioned system closely
+    assert np.linalg.norm(r) <= 1.01e-10 * np.linalg.norm(b)
