@@ -38,9 +38,11 @@
 // Bound: latency (grid round trips, FP64 instructions in chains).  Per Arnoldi
 // step on GB300, mean over a solve, before (one reduction per projection in
 // FP64, CGS2 with three grid steps in FP32) and now: Cahn-Hilliard block system
-// of the 128^3 torus (119,752 rows) in FP32 40.8 -> 18.9 us, of the 40^3 torus
-// (11,928 rows) in FP64 153 -> 21.4 us.  The 18.9 us: product 4.6, dots 2.8,
-// reduction 4.6 (2.9 of it the wait), coefficients 1.0, update 2.5, norm 3.3.
+// of the 128^3 torus (119,752 rows) in FP32 40.8 -> 15.6 us, of the 40^3 torus
+// (11,928 rows) in FP64 153 -> 17.3 us.  With counter reductions it was 18.9 and 21.4:
+// product 4.6, dots 2.8, reduction 4.6 (2.9 of it the wait), coefficients 1.0, update
+// 2.5, norm 3.3; packed sums took 2.4 off (FP32), the head of B in shared memory,
+// shared memory loads and kept warp ranges the rest.
 #include <algorithm>
 #include <cmath>
 

@@ -39,7 +39,12 @@
 // shared memory; 11.3 us with the packed reduction and the room given to matrix
 // values (a block whose last slices' values came from L2 walked 6.2 us instead of
 // 4.4); 9.3 us with the states in slot order and ascending halo lists (the block
-// with the largest halo loaded it in 2.6 us against 1.2 in the mean).
+// with the largest halo loaded it in 2.6 us against 1.2 in the mean); 6.8 us with
+// loads that are known to be shared (a pointer that may be either is a generic load:
+// the product took 3.9 us, now 2.9), the warps' ranges kept, and without the last
+// window's empty slices (one warp of the last block did them all while the others
+// waited, 1.4 us).  The product is now bound by shared memory: 2.9 bank conflicts per
+// gather, 5.4 cycles per 32 entries.
 //
 // Applicability is decided on the host: every block's run (slot rows, halo,
 // translated columns) must fit the shared memory and its vector 16-bit
