@@ -160,8 +160,14 @@ __device__ __forceinline__ int lat_pattern_tab(const Tables* __restrict__ T, int
 __device__ __forceinline__ void cut_point_tab(const Tables* __restrict__ T, const double lat[10], int k, double out[4]) {
     const int a = __ldg(&T->edge_a[k]), b = __ldg(&T->edge_b[k]);
     const double la = lat[a], t = __ddiv_rn(la, __dsub_rn(la, lat[b])), s = __dsub_rn(1.0, t);
-    for (int c = 0; c < 4; ++c)
-        out[c] = __dadd_rn(__dmul_rn(s, __ldg(&T->lat_v[a][c])), __dmul_rn(t, __ldg(&T->lat_v[b][c])));
+    // lattice coordinates are 0, 1/2 and 1: the products are s, s/2, t, t/2 and 0, exactly, and at most two
+    // coordinates have both (12 FP64 operations as a plain combination)
+    const double hs = 0.5 * s, ht = 0.5 * t;
+    for (int c = 0; c < 4; ++c) {
+        const int ia = __double2hiint(__ldg(&T->lat_v[a][c])), ib = __double2hiint(__ldg(&T->lat_v[b][c]));
+        const double u = ia == 0 ? 0. : ia == 0x3ff00000 ? s : hs, v = ib == 0 ? 0. : ib == 0x3ff00000 ? t : ht;
+        out[c] = ia != 0 && ib != 0 ? __dadd_rn(u, v) : ia != 0 ? u : v;
+    }
 }
 
 // The loops over lattice edges, sub-tets, facets and vertices stay rolled in
@@ -583,16 +589,15 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p1_pair(AsmArgs A) 
 // each of up to 16 facets of the order-2 lattice.  Other loads keep that rule, the
 // points of a facet summed into the moments sum_q w_q N_k(q) f(x_q) before they meet
 // the basis.  Every lane walks the lists of its own tet's cut edges and facets, so
-// lanes with different sign patterns stay in step.  Facets lie in the plane of normal
-// n, and n . (u x v) = det sum_c dn_c (du x dv)_c from barycentric differences du, dv
-// needs no square root.  Geometry, cut points and areas are FP64, everything per point
+// lanes with different sign patterns stay in step.  Facets lie in one plane, so a facet's
+// area is a constant of the tet times one 2 x 2 minor of barycentric differences.  Geometry, cut points and areas are FP64, everything per point
 // and all sums pairs.
 //
 // Bound by the FP64 pipe (about 380 instructions per warp of 32 tets with a constant
 // load, 600 with points, 64 cycles each; 49% busy) and, with points, the pair
 // arithmetic.  Forms M, A, C_n of 126,800 cut tets (P1 sphere 128^3, prep and sort
-// included): 868 -> 147 us with a constant load, 1,017 -> 374 with the closest-point
-// load; 1,920 tets 143 -> 41 and 145 -> 73.  The warp per tet before formed 42 points on
+// included): 868 -> 147 us with a constant load, 1,017 -> 354 with the closest-point
+// load; 1,920 tets 143 -> 41 and 145 -> 71.  The warp per tet before formed 42 points on
 // 64 lanes and its sums on 10 to 30 lanes, from 1.9 KB records of FP64 work unrolled to
 // 152 KB of code.
 //
@@ -716,7 +721,8 @@ __global__ void __launch_bounds__(128, B) k_assemble_p1_linear(AsmArgs A, int32_
             for (int k = 0; k < 10; ++k) lat[cP2OnLat[k]] = ls10[k];
         }
         if (!(wantF && !constF)) leave(valid && !lin && sub == 0, rel);
-        double gl[4][3], dn[4], absdet, ddn[3], inv_g = 0.;
+        double gl[4][3], dn[4], absdet, per_minor = 0.;  // twice a facet's area per minor (c1, c2)
+        int c1 = 1, c2 = 2;
         bool plane = false;
         if (lin) {
             double Ms[9], Cs[9];
@@ -734,18 +740,26 @@ __global__ void __launch_bounds__(128, B) k_assemble_p1_linear(AsmArgs A, int32_
             for (int rr = 0; rr < 3; ++rr) gl[0][rr] = (-gl[1][rr] - gl[2][rr]) - gl[3][rr];
             // the level set's gradient from the vertex values
             const double l0 = lat[cP2OnLat[0]];
-            double g[3] = {0., 0., 0.};
+            double g[3] = {0., 0., 0.}, dl[3];
             for (int vv = 1; vv < 4; ++vv) {
-                const double dl = lat[cP2OnLat[vv]] - l0;
-                for (int rr = 0; rr < 3; ++rr) g[rr] += dl * gl[vv][rr];
+                dl[vv - 1] = lat[cP2OnLat[vv]] - l0;
+                for (int rr = 0; rr < 3; ++rr) g[rr] += dl[vv - 1] * gl[vv][rr];
             }
             const double g2 = g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
             const unsigned ge = (unsigned)(__double2hiint(g2) >> 20);
             plane = ge > 123u && ge < 1923u;  // 2^-900 < |g|^2 < 2^900: n is a unit vector
-            inv_g = rsqrt_fp64(g2);
+            const double inv_g = rsqrt_fp64(g2);
             for (int rr = 0; rr < 3; ++rr) g[rr] *= inv_g;
             for (int vv = 0; vv < 4; ++vv) dn[vv] = g[0] * gl[vv][0] + g[1] * gl[vv][1] + g[2] * gl[vv][2];
-            for (int c = 0; c < 3; ++c) ddn[c] = d * dn[c + 1];
+            // du x dv (of the coordinates 1..3) is parallel to the differences dl of the level set, and the area is
+            // |d sum_c dn_c (du x dv)_c|: from the largest component alone, (du x dv)_k |d| |g| / |dl_k|, as
+            // sum_c dn_c dl_c = |g|
+            const double a0 = fabs(dl[0]), a1 = fabs(dl[1]), a2 = fabs(dl[2]);
+            const long long i0 = __double_as_longlong(a0), i1 = __double_as_longlong(a1), i2 = __double_as_longlong(a2);
+            const int k = i0 >= i1 && i0 >= i2 ? 0 : i1 >= i2 ? 1 : 2;
+            c1 = k == 0 ? 1 : k == 1 ? 2 : 0;
+            c2 = k == 0 ? 2 : k == 1 ? 0 : 1;
+            per_minor = absdet * (g2 * inv_g) / (k == 0 ? a0 : k == 1 ? a1 : a2);
             // A needs the projected gradients' products
             if (wantA && sub == 0)
                 for (int vv = 0; vv < 4; ++vv)
@@ -753,15 +767,19 @@ __global__ void __launch_bounds__(128, B) k_assemble_p1_linear(AsmArgs A, int32_
         }
         // twice the area of a facet of barycentric corners b (components 1..3), as a pair
         auto area2 = [&](const double (&b)[3][3], float scale) {
-            double du[3], dv[3], m[3];
-            for (int c = 0; c < 3; ++c) {
-                du[c] = b[1][c] - b[0][c];
-                dv[c] = b[2][c] - b[0][c];
+            if (!plane) {
+                double du[3], dv[3];
+                for (int c = 0; c < 3; ++c) {
+                    du[c] = b[1][c] - b[0][c];
+                    dv[c] = b[2][c] - b[0][c];
+                }
+                return ff_scale(ff_split(p1_area2(X, du, dv)), scale);
             }
-            for (int c = 0; c < 3; ++c) m[c] = du[(c + 1) % 3] * dv[(c + 2) % 3] - du[(c + 2) % 3] * dv[(c + 1) % 3];
-            double a2 = fabs(m[0] * ddn[0] + m[1] * ddn[1] + m[2] * ddn[2]);
-            if (!plane) a2 = p1_area2(X, du, dv);
-            return ff_scale(ff_split(a2), scale);
+            // the minor of the two coordinates c1, c2
+            auto pick = [](const double (&v)[3], int c) { return c == 0 ? v[0] : c == 1 ? v[1] : v[2]; };
+            const double p0 = pick(b[0], c1), q0 = pick(b[0], c2);
+            const double m = (pick(b[1], c1) - p0) * (pick(b[2], c2) - q0) - (pick(b[1], c2) - q0) * (pick(b[2], c1) - p0);
+            return ff_scale(ff_split(fabs(m * per_minor)), scale);
         };
         unsigned neg = 0u, pos = 0u;
         ffacc accF[4];
