@@ -48,7 +48,7 @@ static int ensure_tables_ff(Context* c) {
 
 // Per warp.  The FP64 per-tet scratch (geometry, patch) is dead once split
 // into pairs, so it shares storage with the point rows.  Point rows are padded
-// to an odd number of pairs per lane (11 and 31): a lane's row starts 22 or 62
+// to an odd number of pairs per lane (11 and 21): a lane's row starts 22 or 42
 // words after its neighbour's, so the lanes' 64-bit stores of one column fall
 // in distinct banks, and the contraction's reads of one row (one point, ten
 // columns) do too.
@@ -60,7 +60,7 @@ struct AsmPairFp64 {
 };
 struct AsmPairPts {
     ff phi[32][11];  // sqrt(w) phi_i; n . grad(phi_i) sqrt(w) for the volume rule
-    ff sg[32][31];   // [3 i + c]: sqrt(w) (I - n n^T) grad(phi_i)
+    ff sg[32][21];   // [2 i + c]: sqrt(w) grad(phi_i) in an orthonormal basis of the tangent plane
 };
 struct AsmPairSmem {
     union {
@@ -75,13 +75,39 @@ struct AsmPairSmem {
 // the unit normal grad(phi_h) / |grad(phi_h)| at barycentric b
 __device__ __noinline__ void ff_normal(const AsmPairSmem& S, const ff b[4], ff n[3]) {
     ff v[3];
+    ffacc nn;
     for (int r = 0; r < 3; ++r) {
-        v[r] = ff_mul(b[0], S.G[0][r]);
-        for (int k = 1; k < 4; ++k) v[r] = ff_fma(b[k], S.G[k][r], v[r]);
+        ffacc q;
+        for (int k = 0; k < 4; ++k) q.add_prod(b[k], S.G[k][r]);
+        v[r] = q.value();
+        nn.add_prod(v[r], v[r]);
     }
-    const ff nn = ff_fma(v[2], v[2], ff_fma(v[1], v[1], ff_mul(v[0], v[0])));
-    const ff inv = ff_rsqrt(nn);
+    const ff inv = ff_rsqrt(nn.value());
     for (int r = 0; r < 3; ++r) n[r] = ff_mul(v[r], inv);
+}
+
+// a . b through one accumulator (42 operations where chained pair sums take 64)
+__device__ __forceinline__ ff ff_dot3a(const ff a[3], const ff b[3]) {
+    ffacc q;
+    for (int c = 0; c < 3; ++c) q.add_prod(a[c], b[c]);
+    return q.value();
+}
+
+// An orthonormal basis (t0, t1) of the plane of unit normal n (Duff, Burgess, Christensen, Hery, Kensler, Liani, Villemin,
+// "Building an orthonormal basis, revisited", 2017): one reciprocal, 1 / (1 + |n_z|), in pairs by a Newton step.
+__device__ __forceinline__ void ff_tangents(const ff n[3], ff t0[3], ff t1[3]) {
+    const float sg = copysignf(1.f, n[2].h);
+    const ff d = ff_add_f(ff_scale(n[2], sg), 1.f);
+    const float r0 = __frcp_rn(d.h);
+    const ff q = ff_mul_f(d, r0);
+    const ff a = ff_scale(ff_fast_two_sum(r0, __fmul_rn(r0, __fsub_rn(__fsub_rn(1.f, q.h), q.l))), -sg);
+    const ff xa = ff_mul(n[0], a), b = ff_mul(xa, n[1]);
+    t0[0] = ff_add_f(ff_scale(ff_mul(xa, n[0]), sg), 1.f);
+    t0[1] = ff_scale(b, sg);
+    t0[2] = ff_scale(n[0], -sg);
+    t1[0] = b;
+    t1[1] = ff_add_f(ff_mul(ff_mul(n[1], a), n[1]), sg);
+    t1[2] = ff_neg(n[1]);
 }
 
 __device__ __forceinline__ ff ff_dot3(const ff a[3], const ff b[3]) {
@@ -322,20 +348,28 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p2_pair(AsmArgs A) 
             if (p < npts) {
                 const int f = p / 7, q = p - 7 * (p / 7);
                 ff b[4];
-                for (int c = 0; c < 4; ++c)
-                    b[c] = ff_fma(S.fb[f][2][c], cTF.q2_node[q][2],
-                                  ff_fma(S.fb[f][1][c], cTF.q2_node[q][1], ff_mul(S.fb[f][0][c], cTF.q2_node[q][0])));
+                for (int c = 0; c < 4; ++c) {
+                    ffacc v;
+                    for (int j = 0; j < 3; ++j) v.add_prod(S.fb[f][j][c], cTF.q2_node[q][j]);
+                    b[c] = v.value();
+                }
                 const ff sw = ff_sqrt(ff_mul(S.fw[f], cTF.q2_w[q]));
                 ff n[3];
                 ff_normal(S, b, n);
                 // The basis loops are kept rolled (their operands in L1-resident local
                 // memory): unrolled, the per-point pair code overflows the instruction cache.
-                ff pg[4][3], q4[4];
+                // The projected gradients lie in the tangent plane: two components in a basis of it
+                // instead of three take a third off the A sums and the gradient rows.
+                ff pg[4][2], q4[4];
+                {
+                    ff t0[3], t1[3];
+                    ff_tangents(n, t0, t1);
 #pragma unroll 1
-                for (int k = 0; k < 4; ++k) {
-                    const ff ng = ff_dot3(n, S.gl[k]);
-                    for (int c = 0; c < 3; ++c) pg[k][c] = ff_mul(sw, ff_sub(S.gl[k][c], ff_mul(ng, n[c])));
-                    q4[k] = ff_scale(b[k], 4.f);
+                    for (int k = 0; k < 4; ++k) {
+                        pg[k][0] = ff_mul(sw, ff_dot3a(S.gl[k], t0));
+                        pg[k][1] = ff_mul(sw, ff_dot3a(S.gl[k], t1));
+                        q4[k] = ff_scale(b[k], 4.f);
+                    }
                 }
 #pragma unroll 1
                 for (int i = 0; i < 10; ++i) {
@@ -345,16 +379,18 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p2_pair(AsmArgs A) 
                     const ff ph = i < 4 ? ff_mul(b[a], ff_add_f(ff_scale(b[a], 2.f), -1.f)) : ff_mul(q4[a], b[c2]);
                     P.phi[lane][i] = ff_mul(sw, ph);
                     const ff fa = i < 4 ? ff_add_f(q4[a], -1.f) : q4[c2];
-                    for (int c = 0; c < 3; ++c) {
+                    for (int c = 0; c < 2; ++c) {
                         const ff t = ff_mul(fa, pg[a][c]);
-                        P.sg[lane][3 * i + c] = i < 4 ? t : ff_fma(q4[a], pg[c2][c], t);
+                        P.sg[lane][2 * i + c] = i < 4 ? t : ff_fma(q4[a], pg[c2][c], t);
                     }
                 }
                 if (wantF) {
                     ff x[3];
-                    for (int c = 0; c < 3; ++c)
-                        x[c] = ff_fma(b[3], S.X[3][c],
-                                      ff_fma(b[2], S.X[2][c], ff_fma(b[1], S.X[1][c], ff_mul(b[0], S.X[0][c]))));
+                    for (int c = 0; c < 3; ++c) {
+                        ffacc v;
+                        for (int k = 0; k < 4; ++k) v.add_prod(b[k], S.X[k][c]);
+                        x[c] = v.value();
+                    }
                     S.fx[lane] = ff_mul(sw, ff_rhs(A.rhs, x));
                 }
             }
@@ -370,9 +406,9 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p2_pair(AsmArgs A) 
                     accM[1].add_prod(P.phi[pp][j1], P.phi[pp][i1]);
                 }
                 if (wantA)
-                    for (int c = 0; c < 3; ++c) {
-                        accA[0].add_prod(P.sg[pp][3 * j0 + c], P.sg[pp][3 * i0 + c]);
-                        accA[1].add_prod(P.sg[pp][3 * j1 + c], P.sg[pp][3 * i1 + c]);
+                    for (int c = 0; c < 2; ++c) {
+                        accA[0].add_prod(P.sg[pp][2 * j0 + c], P.sg[pp][2 * i0 + c]);
+                        accA[1].add_prod(P.sg[pp][2 * j1 + c], P.sg[pp][2 * i1 + c]);
                     }
             }
             if (wantF && lane < 30) {  // 10 rows x 3 point groups (combined after the last chunk)
