@@ -293,7 +293,10 @@ int tf_assemble_options(tf_context* ctx, int kernel);
  * x (vec_x) is the initial guess and the result; max_iter and tol are in/out
  * (used iterations / reached residual).  TF_PREC_MIXED runs FP32 PCG sweeps
  * inside FP64 iterative refinement with the same stopping test on the FP64
- * residual.  Returns TF_ERR_NOT_CONVERGED where the reference returns false.  */
+ * residual.  Returns TF_ERR_NOT_CONVERGED where the reference returns false.
+ * The first solve on a pattern of at most 32,768 non-zeros runs on one
+ * thread-block cluster, which needs no layout of the matrix; later solves build
+ * the grid-wide kernels' layout once (and tune their shapes, below).           */
 int tf_pcg_jacobi(tf_context* ctx, int mat, int vec_b, int vec_x, int precision, int* max_iter, double* tol,
                   int rel);
 /* FP64 kernel of tf_pcg_jacobi (TF_PREC_FP64).  No counterpart in the
@@ -367,14 +370,18 @@ int tf_batch_lincomb(tf_context* ctx, int nterms, const int* forms, const double
  * TF_PREC_MIXED: FP32 iterations with FP64 iterate and FP64 residual
  * replacement.  iters[count] and resids[count] (may be NULL) receive each
  * instance's iterations and reached residual; TF_ERR_NOT_CONVERGED when any
- * instance missed tol.  Unless tf_batch_config fixed them, the lanes per row
- * and CTA size come from tf_batch_tune, run on the first solve of a pattern,
- * and the launch sequence is captured once as a CUDA graph and replayed while
- * matrix, vectors and parameters stay the same.                                */
+ * instance missed tol.  TF_PREC_MIXED solves every instance on a thread-block
+ * cluster of 1 to 8 CTAs, their number chosen from the batch's row counts,
+ * unless tf_batch_config fixed lanes or an instance does not fit.  Otherwise one
+ * CTA solves an instance, and unless fixed the lanes per row and CTA size come
+ * from tf_batch_tune, run on the first solve of a pattern.  The launch sequence
+ * is captured once as a CUDA graph and replayed while matrix, vectors and
+ * parameters stay the same.                                                    */
 int tf_batch_pcg_jacobi(tf_context* ctx, int mat, int vec_b, int vec_x, int precision, int max_iter, double tol,
                         int rel, int* iters, double* resids);
-/* Autotuner: times every (lanes per row in {2,4,8,16}, CTA size in
- * {128,256,512,1024}) candidate on this batch and keeps the fastest.           */
+/* Autotuner of the CTA-per-instance form: times every (lanes per row in
+ * {2,4,8,16}, CTA size in {128,256,512,1024}) candidate on this batch and keeps
+ * the fastest.                                                                 */
 int tf_batch_tune(tf_context* ctx, int mat, int vec_b, int precision, int* lanes, int* threads);
 /* lanes = 0: autotune; else fixed lanes per row and CTA size.  use_graph = 0
  * launches the solve directly instead of replaying a CUDA graph.               */
