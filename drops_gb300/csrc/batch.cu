@@ -683,7 +683,8 @@ int batch_pcg(Context* c, CSR& A, const double* b, double* x, int precision, int
     TF_TRY(batch_workspace(c, A));
     BatchCluster bc;
     bool cluster = false;
-    if (mixed && c->pcg_cluster != 0 && c->batch_fixed_lanes == 0) TF_TRY(batch_cluster_prepare(c, A, &bc, &cluster));
+    if (c->pcg_cluster != 0 && c->batch_fixed_lanes == 0)
+        TF_TRY(mixed ? batch_cluster_prepare<float>(c, A, &bc, &cluster) : batch_cluster_prepare<double>(c, A, &bc, &cluster));
     if (!cluster) TF_TRY(batch_lanes_workspace(c, A, mixed));
     if (!cluster && c->batch_fixed_lanes == 0 && (c->batch_lanes == 0 || c->batch_tuned_key != batch_key(c, c->h_batch_nnz, mixed)))
         TF_TRY(batch_tune(c, A, b, mixed, nullptr, nullptr));

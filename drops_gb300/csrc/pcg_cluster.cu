@@ -1,5 +1,5 @@
 // Jacobi-PCG of one system per CTA or thread-block cluster (num/krylovsolver.h:
-// 107-189): the mixed form of the batched solver and small single systems.
+// 107-189): the batched solver and small single systems.
 //
 // A cluster of C CTAs (1 to 8) solves a system; its rows are split into C
 // contiguous ranges.  A CTA sorts its rows by length, so that its slices of 32
@@ -24,7 +24,8 @@
 // 20th iteration); p and r 0.9.  k_batch_pcg took 34.6 at 8,180 rows where this takes
 // 25.6, 15.0, 9.4, 7.1 on 1, 2, 4, 8 CTAs; the whole batch took 33.7 ms and takes 13.0.
 // 1,024 threads (64 registers, spills to an L1 of a few KB) took 15.6 ms, two CTAs of
-// 256 threads per SM 16.3.
+// 256 threads per SM 16.3.  FP64 is bound by the FP64 pipe of its SMs: 8,180 rows 102 ->
+// 27.9, 18.2, 13.7 on 2, 4, 8 CTAs.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -776,12 +777,13 @@ int pcg_cluster(Context* c, CSR& A, int C, const double* b, double* x, int* max_
 template int pcg_cluster<float>(Context*, CSR&, int, const double*, double*, int*, double*, int, bool*);
 template int pcg_cluster<double>(Context*, CSR&, int, const double*, double*, int*, double*, int, bool*);
 
-// The mixed batch (launch only, capturable once prepared): rows and nnz per instance on the host.
+// The batch (launch only, capturable once prepared): rows and nnz per instance on the host.
+template <class V>
 int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok) {
     *ok = false;
     const int n = c->batch_count;
     int64_t room = 0, rmax = 0, nmax = 0;
-    TF_TRY(cl_room<float>(c, &room));
+    TF_TRY(cl_room<V>(c, &room));
     for (int i = 0; i < n; ++i) {
         rmax = std::max<int64_t>(rmax, c->h_batch_rows[i + 1] - c->h_batch_rows[i]);
         nmax = std::max(nmax, c->h_batch_nnz[i]);
@@ -793,16 +795,21 @@ int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok) {
     // the rows, and the launch ends with the longest system or with the queue.  Whole solves on 1, 2, 4, 8 CTAs
     // (ms): 256 ellipsoids of 16^3 to 64^3 cubes - / 13.1 / 16.8 / 30.9 (k_batch_pcg 33.0), 200 of 24^3 to 40^3
     // 21.1 / 20.1 / 23.0 / 31.2 (with assembly), 100 of 10^3 to 60^3 - / 22.0 / 17.4 / 21.0, 40 of 20^3 to 60^3
-    // - / 16.1 / 11.8 / 10.6.
+    // - / 16.1 / 11.8 / 10.6.  FP64: 6.3 us plus 5.3 ns a row of the share (the FP64 pipe) and 0.25 ns a row of the system
+    // (p); solver alone in ms, k_batch_pcg and 1, 2, 4, 8 CTAs (-: does not fit): 256 of 16^3 to 64^3 91.1, - / - / - / 48.9;
+    // 200 of 24^3 to 40^3 24.2, - / 8.4 / 12.2 / 22.2; 40 of 20^3 to 60^3 75.7, - / - / - / 7.9; 16 of 8^3 to 20^3 2.6,
+    // 1.5 / 1.2 / 0.9 / 0.8.
     int C = 0;
     double best = 0.;
     for (int k = 1; k <= kClMaxCtas; k *= 2) {
-        if (!cl_fits<float>(rmax, k, room)) continue;
+        if (!cl_fits<V>(rmax, k, room)) continue;
         const double clusters = std::min(n, c->num_sms / k);
         double sum = 0., top = 0.;
         for (int i = 0; i < n; ++i) {
             const double rows = (double)(c->h_batch_rows[i + 1] - c->h_batch_rows[i]);
-            const double t = std::sqrt(rows) * (5.3 + (k > 1 ? 1. : 0.) + 2.5e-3 * std::max(0., rows / k - 700.));
+            const double us = sizeof(V) == 4 ? 5.3 + (k > 1 ? 1. : 0.) + 2.5e-3 * std::max(0., rows / k - 700.)
+                                             : 6.3 + 5.3e-3 * rows / k + (k > 1 ? 0.25e-3 * rows : 0.);
+            const double t = std::sqrt(rows) * us;
             sum += t;
             top = std::max(top, t);
         }
@@ -812,13 +819,13 @@ int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok) {
             best = est;
         }
     }
-    if (c->pcg_cluster > 0) C = cl_fits<float>(rmax, c->pcg_cluster, room) ? c->pcg_cluster : 0;
+    if (c->pcg_cluster > 0) C = cl_fits<V>(rmax, c->pcg_cluster, room) ? c->pcg_cluster : 0;
     if (C == 0) return TF_OK;
     TF_TRY(ensure(c, c->cl_slots, (size_t)A.m));
     static_assert(sizeof(bc->blob) >= sizeof(ClPlan) + sizeof(ClArgs), "batch cluster blob");
     ClPlan pl;
     ClArgs a{};
-    TF_TRY(cl_plan<float>(c, C, n, rmax, nmax, room, &pl, &a, ok));
+    TF_TRY(cl_plan<V>(c, C, n, rmax, nmax, room, &pl, &a, ok));
     if (!*ok) return TF_OK;
     a.count = n;
     a.order = c->batch_order.p;
@@ -834,6 +841,7 @@ int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok) {
     std::memcpy(bc->blob, &pl, sizeof(pl));
     std::memcpy(bc->blob + sizeof(pl), &a, sizeof(a));
     bc->grid = (int)pl.cfg.gridDim.x;
+    bc->mixed = sizeof(V) == 4;
     bc->ctas = C;
     bc->scratch = a.scratch;
     bc->z = a.z;
@@ -852,7 +860,9 @@ int batch_cluster_launch(Context* c, const BatchCluster& bc, const double* b, do
     a.tol = tol;
     a.rel = rel;
     a.rel_update = c->batch_rel_update;
-    return cl_launch<float>(c, pl, a);
+    return bc.mixed ? cl_launch<float>(c, pl, a) : cl_launch<double>(c, pl, a);
 }
+template int batch_cluster_prepare<float>(Context*, CSR&, BatchCluster*, bool*);
+template int batch_cluster_prepare<double>(Context*, CSR&, BatchCluster*, bool*);
 
 }  // namespace tf

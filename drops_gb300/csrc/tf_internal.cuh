@@ -566,9 +566,11 @@ int pcg_cluster(Context* c, CSR& A, int ctas, const double* b, double* x, int* m
 struct BatchCluster {
     alignas(16) unsigned char blob[512];
     int grid = 0, ctas = 0;
+    bool mixed = true;
     void* scratch = nullptr;
     void* z = nullptr;
 };
+template <class V>
 int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok);
 int batch_cluster_launch(Context* c, const BatchCluster& bc, const double* b, double* x, int max_iter, double tol, int rel);
 int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);

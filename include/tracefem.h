@@ -370,11 +370,12 @@ int tf_batch_lincomb(tf_context* ctx, int nterms, const int* forms, const double
  * TF_PREC_MIXED: FP32 iterations with FP64 iterate and FP64 residual
  * replacement.  iters[count] and resids[count] (may be NULL) receive each
  * instance's iterations and reached residual; TF_ERR_NOT_CONVERGED when any
- * instance missed tol.  TF_PREC_MIXED solves every instance on a thread-block
- * cluster of 1 to 8 CTAs, their number chosen from the batch's row counts,
- * unless tf_batch_config fixed lanes or an instance does not fit.  Otherwise one
- * CTA solves an instance, and unless fixed the lanes per row and CTA size come
- * from tf_batch_tune, run on the first solve of a pattern.  The launch sequence
+ * instance missed tol.  Every instance is solved on a thread-block cluster of 1
+ * to 8 CTAs, their number chosen from the batch's row counts, unless
+ * tf_batch_config fixed lanes or an instance does not fit (about 18,000 rows in
+ * FP64, 36,000 mixed).  Otherwise one CTA solves an instance, and unless fixed
+ * the lanes per row and CTA size come from tf_batch_tune, run on the first
+ * solve of a pattern.  The launch sequence
  * is captured once as a CUDA graph and replayed while matrix, vectors and
  * parameters stay the same.                                                    */
 int tf_batch_pcg_jacobi(tf_context* ctx, int mat, int vec_b, int vec_x, int precision, int max_iter, double tol,
