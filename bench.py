@@ -474,11 +474,12 @@ def run_batch(args, rank, ws, dist):
     lv_chk, le_chk = ctx.levelset_download()
     assert np.array_equal(lv_chk, lv_dev) and np.array_equal(le_chk, le_dev), "P1 edge values differ after upload"
 
-    # solve only: FP64 vs mixed, graph replay vs direct launch
+    # solve only: FP64 vs mixed, graph replay vs direct launch, clusters vs one tuned CTA per problem
     solve = {}
-    for prec, name, graph in ((tf.PREC_FP64, "fp64", True), (tf.PREC_MIXED, "mixed", True),
-                              (tf.PREC_MIXED, "mixed_no_graph", False)):
-        ctx.batch_config(lanes, threads, use_graph=graph)
+    for prec, name, graph, fixed in ((tf.PREC_FP64, "fp64", True, False), (tf.PREC_MIXED, "mixed", True, False),
+                                     (tf.PREC_MIXED, "mixed_no_graph", False, False),
+                                     (tf.PREC_MIXED, "mixed_cta_per_problem", True, True)):
+        ctx.batch_config(lanes if fixed else 0, threads if fixed else 0, use_graph=graph)
         ts = []
         for rep in range(3):
             ctx.vec_fill(tf.VEC_X, state["m"], 0.0)
