@@ -802,7 +802,8 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble(AsmArgs A) {
 // The linear tets of a chunk.  Four lanes per tet while that is at most one block
 // per SM (latency: the facets of a tet in a quarter of the steps), else one; 160
 // registers while all blocks are resident at three per SM, else 128 and four.
-// A load with a point rule, us: 1,920 tets 111 / 73 on 1 / 4 lanes, 4,458 112 / 74, 13,010
+// A load with a point rule, us, when the lines were drawn (each about 5% less since):
+// 1,920 tets 111 / 73 on 1 / 4 lanes, 4,458 112 / 74, 13,010
 // 112 / 171; 28,800 tets 143 / 149 on three / four blocks per SM, 71,300 289 / 222,
 // 126,800 448 / 374.
 static void launch_p1_linear(Context* c, const AsmArgs& A, int64_t n, int32_t* rest, int* nrest) {
