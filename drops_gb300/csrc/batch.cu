@@ -683,7 +683,12 @@ int batch_pcg(Context* c, CSR& A, const double* b, double* x, int precision, int
     TF_TRY(batch_workspace(c, A));
     BatchCluster bc;
     bool cluster = false;
-    if (c->pcg_cluster != 0 && c->batch_fixed_lanes == 0)
+    // A cluster holds the vectors of its own instance and finds a column there by its slot: every column of a row must
+    // belong to the row's instance.  That holds for the matrices assembled on the present numbering; an uploaded matrix,
+    // or one left from an earlier numbering of as many rows, may link instances and stays with k_batch_pcg, whose
+    // vectors hold all rows.
+    const bool own = c->pattern_dof_version == c->dof_version && A.pattern_gen == c->mats[TF_FORM_M].pattern_gen;
+    if (own && c->pcg_cluster != 0 && c->batch_fixed_lanes == 0)
         TF_TRY(mixed ? batch_cluster_prepare<float>(c, A, &bc, &cluster) : batch_cluster_prepare<double>(c, A, &bc, &cluster));
     if (!cluster) TF_TRY(batch_lanes_workspace(c, A, mixed));
     if (!cluster && c->batch_fixed_lanes == 0 && (c->batch_lanes == 0 || c->batch_tuned_key != batch_key(c, c->h_batch_nnz, mixed)))

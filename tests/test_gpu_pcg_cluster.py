@@ -192,3 +192,45 @@ def test_batch(context, ctas, graph, precision):
         s = slice(rows[i], rows[i + 1])
         assert np.linalg.norm(x[s] - y[s]) <= 2e4 * TOL * np.linalg.norm(y[s])
     assert np.all(np.abs(it - jt) <= (1 if precision == tf.PREC_FP64 else 2 + jt // 4))
+
+
+@pytest.mark.parametrize("precision", [tf.PREC_MIXED, tf.PREC_FP64])
+def test_batch_uploaded_matrix(context, precision):
+    """A caller's matrix as large as the numbering: block diagonal it is solved like the assembled one; with entries
+    between instances, which no cluster can hold, the call ends within its iterations and the context stays usable."""
+    W = ellipsoid_batch(9, nmin=6, nmax=20, seed=5)
+    forms = [tf.FORM_M, tf.FORM_A, tf.FORM_CN]
+    ctx = context(8)
+    ctx.brick_batch(W["n"], W["orig"], W["axes"])
+    ctx.levelset_analytic_batch(tf.LS_ELLIPSOID, W["par"], p2=False)
+    _, m = ctx.distribute_dofs(tf.P1IF)
+    ctx.setup_fe_system(forms, tf.RHS_SPHERE_XYZ, [0.0, 0.0, 0.0, 1.0, 12.0])
+    ctx.batch_lincomb(forms, np.stack([np.ones(9), np.ones(9), W["h"]], axis=1))
+    rp, ci, v = ctx.matrix(tf.MAT_SYS)
+    b = ctx.vec_download(tf.VEC_RHS)
+    rows = ctx.batch_info(nnz=False)[2]
+
+    def solve(mat, **kw):
+        ctx.vec_fill(tf.VEC_X, m, 0.0)
+        st, it, res = ctx.batch_pcg_jacobi(mat, tf.VEC_RHS, tf.VEC_X, tol=TOL, precision=precision, check=False, **kw)
+        return st, res, ctx.vec_download(tf.VEC_X)
+
+    def solved(st, res, x):
+        r = b - mul((rp, ci, v, b), x)
+        return st == tf.OK and res.max() <= TOL and all(
+            np.linalg.norm(r[s:e]) <= 1.01 * TOL * np.linalg.norm(b[s:e]) for s, e in zip(rows[:-1], rows[1:]))
+
+    ctx.matrix_upload(rp, ci, v)
+    assert solved(*solve(tf.MAT_USER))
+    # the last row of every instance linked to the first and the last of all others
+    ends = np.unique(np.concatenate([rows[:-1], rows[1:] - 1]))
+    import scipy.sparse as sp
+
+    E = sp.coo_matrix((np.full(len(ends) * (len(ends) - 1), -1e-3),
+                       (np.repeat(ends, len(ends) - 1), np.concatenate([np.delete(ends, i) for i in range(len(ends))]))),
+                      shape=(m, m))
+    L = (sp.csr_matrix((v, ci, rp), shape=(m, m)) + E).tocsr()
+    L.sort_indices()
+    ctx.matrix_upload(L.indptr.astype(np.int64), L.indices.astype(np.int64), L.data)
+    assert solve(tf.MAT_USER, max_iter=40)[0] in (tf.OK, tf.ERR_NOT_CONVERGED)
+    assert solved(*solve(tf.MAT_SYS))
