@@ -206,6 +206,17 @@ int fill_f64(Context* c, double* p, int64_t n, double v) {
     return TF_OK;
 }
 
+int max_dynamic_smem(Context* c, const void* fn, int64_t* room) {
+    cudaFuncAttributes fa{};
+    int optin = 0;
+    TF_CUDA(c, cudaFuncGetAttributes(&fa, fn));
+    TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    const int64_t all = (int64_t)optin - (int64_t)fa.sharedSizeBytes;
+    TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all));
+    *room = all - 1024;
+    return TF_OK;
+}
+
 int sync_status(Context* c, int* status_out) {
     TF_CUDA(c, cudaMemcpyAsync(c->h_status, c->status.p, kStatusWords * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     TF_CUDA(c, cudaStreamSynchronize(c->stream));

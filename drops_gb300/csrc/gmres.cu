@@ -632,11 +632,8 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
     unsigned long long* pw = nullptr;
     TF_TRY(packed_words(c, 2, &pw));
-    cudaFuncAttributes fa{};
-    int optin = 0;
-    TF_CUDA(c, cudaFuncGetAttributes(&fa, (const void*)k_gmres_ls<V, true>));
-    TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    const int64_t room = (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024;
+    int64_t room = 0;
+    TF_TRY(max_dynamic_smem(c, (const void*)k_gmres_ls<V, true>, &room));
     const size_t small = (sizeof(LsSmall<V>) + 15) & ~(size_t)15;
     const int64_t run = 32 * ((ns + blocks - 1) / blocks);  // slots of the largest run
     const int64_t both = (int64_t)small + 2 * run * (int64_t)sizeof(V);
@@ -647,7 +644,7 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     if (ccap < 0) ccap = 0;
     const size_t dyn = smem ? (size_t)(both + ccap * (int64_t)(sizeof(V) + 4)) : small;
     const void* fn = smem ? (const void*)k_gmres_ls<V, true> : (const void*)k_gmres_ls<V, false>;
-    TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    if (!smem) TF_TRY(max_dynamic_smem(c, fn, &room));
     int per_sm = 0;
     TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLsThreads, dyn));
     if (per_sm < 1) return set_err(c, TF_ERR_CUDA, "gmres: kernel does not fit the SM");

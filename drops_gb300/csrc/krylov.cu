@@ -1328,16 +1328,12 @@ static int run_pcg_cg1(Context* c, const CSR& A, const double* b, double* x, int
     size_t dyn = 0;
     int32_t cap = 0;
     if (c->pcg_blocked && nt == 512 && c->pcg_smem_cache_kb > 0) {
-        cudaFuncAttributes fa{};
-        int optin = 0;
-        TF_CUDA(c, cudaFuncGetAttributes(&fa, fn));
-        TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-        const int64_t room = std::min<int64_t>((int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024,
-                                               (int64_t)c->pcg_smem_cache_kb * 1024);
+        int64_t room = 0;
+        TF_TRY(max_dynamic_smem(c, fn, &room));
+        room = std::min<int64_t>(room, (int64_t)c->pcg_smem_cache_kb * 1024);
         if (room > 4096) {
             cap = (int32_t)((room / 8) & ~(int64_t)3);
             dyn = (size_t)cap * 8;
-            TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
         }
     }
     int blocks = 0;

@@ -730,16 +730,6 @@ int res_blocks(const Context* c, const CSR& A) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(c->num_sms, kPkMaxBlocks), A.sell.used / 2));
 }
 
-// shared memory a block of fn can use besides its static part
-int res_room(Context* c, const void* fn, int64_t* room) {
-    cudaFuncAttributes fa{};
-    int optin = 0;
-    TF_CUDA(c, cudaFuncGetAttributes(&fa, fn));
-    TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    *room = (int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024;
-    return TF_OK;
-}
-
 }  // namespace
 
 // zeroed words for n packed reductions
@@ -764,7 +754,7 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     const Sell& S = A.sell;
     if (!S.res_ok || S.res_smax <= 0 || S.res_smax > kBalMaxSlices) return TF_OK;
     int64_t room = 0;
-    TF_TRY(res_room(c, fn, &room));
+    TF_TRY(max_dynamic_smem(c, fn, &room));
     const int32_t ccap = (S.res_maxslots + 15) & ~15;
     const int64_t fixed = (int64_t)res_fixed_bytes<T>(S.res_smax, S.res_hmax, ccap);
     if (fixed > room) return TF_OK;
@@ -772,7 +762,6 @@ int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, 
     if (c->pcg_res_vcap_kb >= 0)
         vcap = std::min<int32_t>(vcap, (int32_t)(((int64_t)c->pcg_res_vcap_kb * 1024 / (int64_t)sizeof(T)) & ~7));
     const size_t dyn = (size_t)fixed + (size_t)vcap * sizeof(T);
-    TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     int per_sm = 0;
     TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kResThreads, dyn));
     if (per_sm < 1) return TF_OK;
@@ -872,12 +861,11 @@ int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter
     if (!S.res_ok || S.res_smax <= 0 || S.res_smax > kBalMaxSlices) return TF_OK;
     const int32_t ccap = (S.res_maxslots + 15) & ~15;
     int64_t room = 0;
-    TF_TRY(res_room(c, fn, &room));
+    TF_TRY(max_dynamic_smem(c, fn, &room));
     const int64_t fixed = (int64_t)pcg64_fixed_bytes(S.res_smax, S.res_hmax, ccap);
     if (fixed > room) return TF_OK;
     const int32_t vcap = (int32_t)std::min<int64_t>((room - fixed) / (int64_t)sizeof(double), (int64_t)ccap) & ~7;
     const size_t dyn = (size_t)fixed + (size_t)vcap * sizeof(double);
-    TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     int per_sm = 0;
     TF_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kResThreads, dyn));
     if (per_sm < 1) return TF_OK;

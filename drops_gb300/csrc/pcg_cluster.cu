@@ -653,11 +653,8 @@ bool cl_fits(int64_t rows, int C, int64_t room) {
 
 template <class V>
 int cl_room(Context* c, int64_t* room) {
-    cudaFuncAttributes fa{};
-    int optin = 0;
-    TF_CUDA(c, cudaFuncGetAttributes(&fa, (const void*)k_pcg_cluster<V>));
-    TF_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
-    *room = ((int64_t)optin - (int64_t)fa.sharedSizeBytes - 1024) & ~(int64_t)127;
+    TF_TRY(max_dynamic_smem(c, (const void*)k_pcg_cluster<V>, room));
+    *room &= ~(int64_t)127;
     return TF_OK;
 }
 
@@ -674,7 +671,6 @@ int cl_plan(Context* c, int C, int count, int64_t rows, int64_t nnz, int64_t roo
     if (e > (int64_t)1 << 28) return TF_OK;
     a->ecap = (int)((e + 63) & ~(int64_t)63);
     a->room = (int)room;
-    TF_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room));
     pl->C = C;
     pl->attr.id = cudaLaunchAttributeClusterDimension;
     pl->attr.val.clusterDim.x = (unsigned)C;

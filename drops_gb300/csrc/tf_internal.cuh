@@ -514,6 +514,10 @@ int exclusive_scan_i32_status(Context* c, const int32_t* in, int32_t* out, int64
 // *order: the rows of the current DistributeDOFs numbering in Morton order of
 // their nodes, or nullptr where there is none (explicit or batch meshes)
 int dof_locality_order(Context* c, const int32_t** order);
+// Lets kernel fn use all of a block's shared memory; *room: the bytes of it a launch may ask for.  The limit is one of the
+// kernel in the whole process: it always gets the same value, whatever a launch takes, as a smaller one set by a context
+// on another thread between the setting here and the launch would fail that launch.
+int max_dynamic_smem(Context* c, const void* fn, int64_t* room);
 // fetches the status words (kStatusWords) into h_status and waits
 int sync_status(Context* c, int* status_out);
 int fill_f64(Context* c, double* p, int64_t n, double v);
