@@ -138,6 +138,7 @@ int tf_create(tf_context** out, int device) {
         const int n = std::atoi(e);
         if (n == 0 || n == 1 || n == 2 || n == 4 || n == 8) c->pcg_cluster = n;
     }
+    if (const char* e = std::getenv("TF_PCG_CLUSTER_EXTRA_MB")) c->cl_scratch_extra = (size_t)std::atoll(e) << 20;
     if (const char* e = std::getenv("TF_PCG_RES_VCAP_KB")) c->pcg_res_vcap_kb = std::atoi(e);
     if (const char* e = std::getenv("TF_PCG_REL_UPDATE")) c->pcg_rel_update = std::atof(e);
     if (const char* e = std::getenv("TF_BATCH_REL_UPDATE")) c->batch_rel_update = std::atof(e);

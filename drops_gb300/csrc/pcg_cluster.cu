@@ -658,7 +658,7 @@ int cl_room(Context* c, int64_t* room) {
     return TF_OK;
 }
 
-// fills plan, a.pcap .. a.room, a.scratch and a.z; *ok = false when the device has no room for it
+// fills plan, a.pcap .. a.room, a.scratch, a.z and a.slotmap (a.m given); *ok = false when the device has no room for it
 template <class V>
 int cl_plan(Context* c, int C, int count, int64_t rows, int64_t nnz, int64_t room, ClPlan* pl, ClArgs* a, bool* ok) {
     *ok = false;
@@ -688,14 +688,18 @@ int cl_plan(Context* c, int C, int count, int64_t rows, int64_t nnz, int64_t roo
     pl->clusters = std::min(n, count);
     pl->cfg.gridDim = dim3((unsigned)(pl->clusters * C));
     a->scratch_cta = cl_scratch<V>(a->ncap, a->ecap);
-    if (ensure(c, c->cl_scratch, a->scratch_cta * pl->clusters * C) != TF_OK ||
-        ensure(c, c->cl_z, (size_t)a->pcap * pl->clusters) != TF_OK) {
-        c->err.clear();
+    TF_TRY(ensure_if_room(c, c->cl_scratch, a->scratch_cta * pl->clusters * C + c->cl_scratch_extra, ok));
+    if (*ok) TF_TRY(ensure_if_room(c, c->cl_z, (size_t)a->pcap * pl->clusters, ok));
+    if (*ok) TF_TRY(ensure_if_room(c, c->cl_slots, (size_t)a->m, ok));
+    if (!*ok) {  // the other kernels need the memory that was had
+        release(c->cl_scratch);
+        release(c->cl_z);
+        release(c->cl_slots);
         return TF_OK;
     }
     a->scratch = c->cl_scratch.p;
     a->z = c->cl_z.p;
-    *ok = true;
+    a->slotmap = c->cl_slots.p;
     return TF_OK;
 }
 
@@ -738,19 +742,17 @@ int pcg_cluster(Context* c, CSR& A, int C, const double* b, double* x, int* max_
     if (A.m > INT32_MAX / 2 || !cl_fits<V>(A.m, C, room)) return TF_OK;
     ClPlan pl;
     ClArgs a{};
-    TF_TRY(ensure(c, c->cl_slots, (size_t)A.m));
+    a.m = A.m;
     TF_TRY(ensure(c, c->kry_iters, 4));
     TF_TRY(ensure(c, c->kry_resid, 1));
     TF_TRY(cl_plan<V>(c, C, 1, A.m, A.nnz, room, &pl, &a, applied));
     if (!*applied) return TF_OK;
     a.count = 1;
-    a.m = A.m;
     a.rowptr = A.rowptr;
     a.col = A.colind;
     a.val = A.vals;
     a.b = b;
     a.x = x;
-    a.slotmap = c->cl_slots.p;
     a.queue = c->kry_iters.p;
     a.out_iter = c->kry_iters.p + 1;
     a.out_updates = c->kry_iters.p + 2;
@@ -817,20 +819,18 @@ int batch_cluster_prepare(Context* c, CSR& A, BatchCluster* bc, bool* ok) {
     }
     if (c->pcg_cluster > 0) C = cl_fits<V>(rmax, c->pcg_cluster, room) ? c->pcg_cluster : 0;
     if (C == 0) return TF_OK;
-    TF_TRY(ensure(c, c->cl_slots, (size_t)A.m));
     static_assert(sizeof(bc->blob) >= sizeof(ClPlan) + sizeof(ClArgs), "batch cluster blob");
     ClPlan pl;
     ClArgs a{};
+    a.m = A.m;
     TF_TRY(cl_plan<V>(c, C, n, rmax, nmax, room, &pl, &a, ok));
     if (!*ok) return TF_OK;
     a.count = n;
     a.order = c->batch_order.p;
     a.rows = c->batch_rows.p;
-    a.m = A.m;
     a.rowptr = A.rowptr;
     a.col = A.colind;
     a.val = A.vals;
-    a.slotmap = c->cl_slots.p;
     a.queue = c->batch_queue.p;
     a.out_iter = c->batch_iters.p;
     a.out_resid = c->batch_resid.p;

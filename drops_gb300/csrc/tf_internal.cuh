@@ -341,6 +341,7 @@ struct Context {
     DBuf<double> cl_z;        // cluster PCG: z per cluster
     DBuf<int32_t> cl_slots;   // cluster slot of every row
     DBuf<unsigned char> cl_scratch;  // what the CTAs' shared memory does not hold
+    size_t cl_scratch_extra = 0;     // bytes asked for besides (TF_PCG_CLUSTER_EXTRA_MB: for a test of the full device)
     DBuf<int> kry_iters;
     // scratch
     DBuf<unsigned char> scratch;
@@ -480,18 +481,33 @@ int set_err(Context* c, int code, const std::string& msg);
     } while (0)
 
 template <class T>
-int ensure(Context* c, DBuf<T>& b, size_t n) {
+cudaError_t grow(DBuf<T>& b, size_t n) {
     if (b.cap < n) {
         if (b.p) cudaFree(b.p);
         b.p = nullptr;
         b.cap = 0;
-        size_t bytes = (n > 0 ? n : 1) * sizeof(T);
-        cudaError_t e = cudaMalloc((void**)&b.p, bytes);
-        if (e != cudaSuccess) return set_err(c, TF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        const cudaError_t e = cudaMalloc((void**)&b.p, (n > 0 ? n : 1) * sizeof(T));
+        if (e != cudaSuccess) {
+            cudaGetLastError();  // reported here: the next launch's check must not find it again
+            return e;
+        }
         b.cap = n > 0 ? n : 1;
     }
     b.n = n;
-    return TF_OK;
+    return cudaSuccess;
+}
+template <class T>
+int ensure(Context* c, DBuf<T>& b, size_t n) {
+    const cudaError_t e = grow(b, n);
+    return e == cudaSuccess ? TF_OK : set_err(c, TF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+}
+// the same where the caller has another way without the buffer: *ok = false when the device has no memory for it
+template <class T>
+int ensure_if_room(Context* c, DBuf<T>& b, size_t n, bool* ok) {
+    const cudaError_t e = grow(b, n);
+    *ok = e == cudaSuccess;
+    if (*ok || e == cudaErrorMemoryAllocation) return TF_OK;
+    return set_err(c, TF_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
 }
 template <class T>
 void release(DBuf<T>& b) {

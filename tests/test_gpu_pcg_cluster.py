@@ -234,3 +234,55 @@ def test_batch_uploaded_matrix(context, precision):
     ctx.matrix_upload(L.indptr.astype(np.int64), L.indices.astype(np.int64), L.data)
     assert solve(tf.MAT_USER, max_iter=40)[0] in (tf.OK, tf.ERR_NOT_CONVERGED)
     assert solved(*solve(tf.MAT_SYS))
+
+
+def _no_memory(monkeypatch):
+    monkeypatch.setenv("TF_PCG_CLUSTER_EXTRA_MB", str(1 << 30))  # more than any device has: the scratch cannot be had
+
+
+@pytest.mark.parametrize("precision", [tf.PREC_FP64, tf.PREC_MIXED])
+def test_single_system_without_room_for_a_cluster(context, monkeypatch, precision):
+    """No memory for the cluster's scratch: the grid-wide kernels solve, and no error is left behind."""
+    _no_memory(monkeypatch)
+    A, its = system("ragged")
+    b = A[3]
+    ctx = context(4)
+    ctx.matrix_upload(*A[:3])
+    ctx.vec_upload(tf.VEC_B, b)
+    ctx.vec_upload(tf.VEC_X, np.zeros(len(b)))
+    st, it, res = ctx.pcg_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, tol=TOL, precision=precision)
+    assert st == tf.OK and res <= TOL
+    assert np.linalg.norm(b - mul(A, ctx.vec_download(tf.VEC_X))) <= 1.01 * TOL * np.linalg.norm(b)
+    assert abs(it - its) <= (1 if precision == tf.PREC_FP64 else 2 + its // 4)
+
+
+@pytest.mark.parametrize("graph", [True, False])
+@pytest.mark.parametrize("precision", [tf.PREC_FP64, tf.PREC_MIXED])
+@pytest.mark.parametrize("why", ["no memory", "rows"])
+def test_batch_without_room_for_clusters(context, monkeypatch, precision, graph, why):
+    """Scratch that cannot be had, and an instance of more rows than a cluster holds: a CTA per instance solves."""
+    W = ellipsoid_batch(6, nmin=6, nmax=20, seed=31)
+    if why == "rows":
+        W["n"][2] = 160  # about 47,000 rows
+    else:
+        _no_memory(monkeypatch)
+    forms = [tf.FORM_M, tf.FORM_A, tf.FORM_CN]
+    ctx = context(8)
+    ctx.brick_batch(W["n"], W["orig"], W["axes"])
+    ctx.levelset_analytic_batch(tf.LS_ELLIPSOID, W["par"], p2=False)
+    _, m = ctx.distribute_dofs(tf.P1IF)
+    ctx.setup_fe_system(forms, tf.RHS_SPHERE_XYZ, [0.0, 0.0, 0.0, 1.0, 12.0])
+    ctx.batch_lincomb(forms, np.stack([np.ones(6), np.ones(6), W["h"]], axis=1))
+    rows = ctx.batch_info(nnz=False)[2]
+    if why == "rows":
+        assert rows[3] - rows[2] > 37000
+    ctx.batch_config(0, 0, use_graph=graph)
+    rp, ci, v = ctx.matrix(tf.MAT_SYS)
+    b = ctx.vec_download(tf.VEC_RHS)
+    for _ in range(2):
+        ctx.vec_fill(tf.VEC_X, m, 0.0)
+        st, it, res = ctx.batch_pcg_jacobi(tf.MAT_SYS, tf.VEC_RHS, tf.VEC_X, tol=TOL, precision=precision)
+        assert st == tf.OK and res.max() <= TOL
+        r = b - mul((rp, ci, v, b), ctx.vec_download(tf.VEC_X))
+        for s, e in zip(rows[:-1], rows[1:]):
+            assert np.linalg.norm(r[s:e]) <= 1.01 * TOL * np.linalg.norm(b[s:e])
