@@ -95,9 +95,16 @@ __device__ __forceinline__ unsigned cl_id() {
     return r;
 }
 // barrier over all threads of the cluster; writes before the arrival (shared,
-// distributed shared and global memory) are visible to the cluster after the wait
-__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// distributed shared and global memory) are visible to the cluster after the wait.
+// .aligned: a warp's lanes execute it together, so they meet before it.
+__device__ __forceinline__ void cl_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cl_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cl_sync() {
     cl_arrive();
     cl_wait();
@@ -238,7 +245,6 @@ __global__ void __launch_bounds__(kClThreads<V>, 1) k_pcg_cluster(ClArgs a) {
             const double s = warp_fx_sum(one);
             if (lane < C) cl_store(&sh.slot[flip][warp][rank], (unsigned)lane, s);
         }
-        __syncwarp();
         cl_arrive();
         meanwhile();
         cl_wait();
