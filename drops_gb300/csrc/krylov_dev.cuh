@@ -206,6 +206,33 @@ __device__ __forceinline__ double warp_fx_sum8(const double (&v)[8], int lane) {
     return fx_value(tot, e, kLeft);
 }
 
+// The stopping test sqrt(rr) / normb <= tol on squares (a square root and a division are 1,200 cycles of the FP64 pipe):
+// rr <= the threshold.  A negative tol holds for no rr.  NaN where the square of tol normb leaves the doubles' normal
+// range; the test then takes the roots.
+__device__ __forceinline__ double rr_threshold(double tol, double normb) {
+    const double t = tol * normb;
+    if (tol < 0.) return -1.;
+    return tol == 0. || (t > 1e-150 && t < 1e150) ? t * t : __longlong_as_double(0x7fffffffffffffffll);
+}
+static __device__ __noinline__ bool rr_reached_roots(double rr, double tol, double normb) { return sqrt(rr) / normb <= tol; }
+__device__ __forceinline__ bool rr_reached(double rr, double thr, double tol, double normb) {
+    // NaN told by its bits: an FP64 comparison more is 64 cycles on the path of every iteration
+    if (((unsigned)__double2hiint(thr) >> 19 & 0xfffu) == 0xfffu) return rr_reached_roots(rr, tol, normb);
+    return rr <= thr;
+}
+// x / rho and rho / x with the reciprocal of rho formed beforehand, off the path of the reduction that gives x; by division
+// where that reciprocal could overflow or underflow
+__device__ __forceinline__ bool rho_plain(double rho) {
+    return ((unsigned)__double2hiint(rho) >> 20 & 0x7ffu) - 32u < 1984u;  // 2^-991 <= |rho| < 2^993
+}
+static __device__ __noinline__ double rho_quotient(double x, double y) { return x / y; }
+__device__ __forceinline__ double by_rho(double x, double rho, double rho_inv) {
+    return rho_plain(rho) ? x * rho_inv : rho_quotient(x, rho);
+}
+__device__ __forceinline__ double rho_by(double rho, double rho_inv, double x) {
+    return rho_plain(rho) ? 1.0 / (x * rho_inv) : rho_quotient(rho, x);
+}
+
 template <int NV, class T>
 __device__ void block_partials(T (&v)[NV], double* part /* [nblocks][NV] */) {
     __shared__ double red[NV][32];

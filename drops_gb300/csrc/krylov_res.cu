@@ -445,8 +445,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
     uint16_t* ccol = reinterpret_cast<uint16_t*>(hrow + a.hmax);
     double* cval = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ccol) + (((size_t)a.ccap * 2 + 31) & ~(size_t)31));
     __shared__ BalShared<NW, double> bsh;
-    __shared__ double sh[4];
-    __shared__ int flag;
+    __shared__ double sh[4];  // alpha, beta, 1 / rho, rho
+    __shared__ int flag, conv;
 
     unsigned long long epoch = 0;
     PkState pk1, pk2;
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
             });
         return pq;
     };
-    double thr2, rr;
+    double thr2, normb, rr;
     int it = 0;
     {
         walk();
@@ -523,16 +523,17 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
             nb = sqrt(o[1]);
             if (nb == 0.0 || !a.rel) nb = 1.0;
             sh[0] = nb;
-            sh[1] = 0.;                // beta
-            sh[2] = 1.0 / o[2];        // 1 / rho
-            sh[3] = (a.tol * nb) * (a.tol * nb);
-            flag = o[0] <= sh[3] || a.max_iter <= 0;
+            sh[1] = 0.;
+            sh[2] = 1.0 / o[2];
+            sh[3] = o[2];
+            conv = rr_reached(o[0], rr_threshold(a.tol, nb), a.tol, nb);
+            flag = conv || a.max_iter <= 0;
         }
         rr = o[0];
         __syncthreads();
-        thr2 = sh[3];
+        normb = sh[0];
+        thr2 = rr_threshold(a.tol, normb);
     }
-    const double normb = sh[0];
     bool done = flag != 0;
     while (!done) {
         const double beta = sh[1];
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
         double v1[1], o1[1];
         v1[0] = walk();
         if (!packed_allreduce<1>(a.pk1, pk1, a.g, epoch, v1, o1, false)) return;
-        if (threadIdx.x == 0) sh[0] = 1.0 / (o1[0] * sh[2]);  // alpha = rho / <p, A p>
+        if (threadIdx.x == 0) sh[0] = rho_by(sh[3], sh[2], o1[0]);  // alpha = rho / <p, A p>
         __syncthreads();
         const double alpha = sh[0];
         double v[2] = {0., 0.}, o[2];
@@ -560,8 +561,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
         ++it;
         rr = o[0];
         if (threadIdx.x == 0) {
-            sh[1] = o[1] * sh[2];
-            flag = rr <= thr2 || it >= a.max_iter;
+            sh[1] = by_rho(o[1], sh[3], sh[2]);
+            sh[3] = o[1];
+            conv = rr_reached(rr, thr2, a.tol, normb);
+            flag = conv || it >= a.max_iter;
         }
         __syncthreads();
         // 1 / rho of the next iteration, off the path of the others (read after two barriers)
@@ -571,7 +574,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg64_res(Pcg64Args a) {
     for (int t = threadIdx.x; t < NS; t += kResThreads)
         if (sperm[t] >= 0) a.x[sperm[t]] = xs[t];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *a.out_iter = rr <= thr2 ? it : -1 - it;
+        *a.out_iter = conv ? it : -1 - it;
         *a.out_resid = sqrt(rr) / normb;
     }
 }

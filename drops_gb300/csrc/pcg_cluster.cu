@@ -537,15 +537,15 @@ __global__ void __launch_bounds__(kClThreads<V>, 1) k_pcg_cluster(ClArgs a) {
                     double nb = sqrt(o[1]);
                     if (nb == 0.0 || !a.rel) nb = 1.0;
                     sh.normb = nb;
-                    sh.thr_tol = (a.tol * nb) * (a.tol * nb);
+                    sh.thr_tol = rr_threshold(a.tol, nb);
                     sh.beta = 0.;
                 } else {
-                    sh.beta = o[2] * sh.rho_inv;
+                    sh.beta = by_rho(o[2], sh.rho, sh.rho_inv);
                 }
                 sh.rr = o[0];
                 sh.thr_last = kMixed ? a.rel_update * a.rel_update * o[0] : 0.;
                 sh.rho = o[2];
-                sh.converged = o[0] <= sh.thr_tol;
+                sh.converged = rr_reached(o[0], sh.thr_tol, a.tol, sh.normb);
             });
         };
         int it = 0;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(kClThreads<V>, 1) k_pcg_cluster(ClArgs a) {
             ++it;
             {
                 const V v[1] = {product()};
-                cluster_sum(N1{}, v, [] {}, [&](const double* o) { sh.alpha = 1.0 / (o[0] * sh.rho_inv); });
+                cluster_sum(N1{}, v, [] {}, [&](const double* o) { sh.alpha = rho_by(sh.rho, sh.rho_inv, o[0]); });
             }
             {
                 const double alpha = sh.alpha;
@@ -614,16 +614,16 @@ __global__ void __launch_bounds__(kClThreads<V>, 1) k_pcg_cluster(ClArgs a) {
                 cluster_sum(N2{}, v, update_x, [&](const double* o) {
                     sh.rr = o[0];
                     if (kMixed) {
-                        sh.refine = o[0] <= sh.thr_last || o[0] <= sh.thr_tol || it >= a.max_iter;
+                        sh.refine = o[0] <= sh.thr_last || rr_reached(o[0], sh.thr_tol, a.tol, sh.normb) || it >= a.max_iter;
                         if (!sh.refine) {
-                            sh.beta = o[1] * sh.rho_inv;
+                            sh.beta = by_rho(o[1], sh.rho, sh.rho_inv);
                             sh.rho = o[1];
                         }
                     } else {
                         sh.refine = 0;
-                        sh.converged = o[0] <= sh.thr_tol;
+                        sh.converged = rr_reached(o[0], sh.thr_tol, a.tol, sh.normb);
                         sh.done = sh.converged || it >= a.max_iter;
-                        sh.beta = o[1] * sh.rho_inv;
+                        sh.beta = by_rho(o[1], sh.rho, sh.rho_inv);
                         sh.rho = o[1];
                     }
                 });
