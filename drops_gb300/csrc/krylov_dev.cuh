@@ -542,13 +542,16 @@ __device__ bool grid_allreduce(const GridAR& g, unsigned long long& epoch, const
 // polls the word sees the finished sum with the last arrival: one atomic add
 // and one poll.  Integer sums do not depend on the order of arrival, so every
 // block gets the same bits.  The unit of a value follows from its previous sum,
-// which all blocks know: an FP32 value takes one word with 2^34 units to that
-// sum, an FP64 value two (a 48-bit high and a 40-bit low part) with 2^67.  The
-// blocks repeat the reduction with grid_allreduce when a partial exceeds the
-// previous sum 2^5 (2^12) times or is not finite, and when the sum is smaller
-// than 2^-10 (2^-14) of it, so that no sum has fewer bits than its type holds.
-// (Without the second condition a GMRES basis vector a thousand times shorter
-// than the one before lost its norm, and the solver stagnated.)
+// which all blocks know: an FP32 value takes one word with 2^38 units to that
+// sum, an FP64 value two (a 48-bit high and a 40-bit low part) with 2^76.  The
+// blocks repeat the reduction with grid_allreduce when a block's sum exceeds the
+// previous sum twice (8 times; on fewer than 128 blocks more) or is not finite,
+// and when the sum is smaller than 2^-6 of it.  So the rounding of all the terms
+// that are aligned to the unit - the blocks' sums in FP32, at most 255; the
+// threads' values in FP64, at most 2^17 - adds up to at most 255 x 2^-39 x 2^6 =
+// 2^-25 (2^17 x 2^-77 x 2^6 = 2^-54) of the sum: half of what rounding it to its
+// type costs.  (Without the last condition a GMRES basis vector a thousand times
+// shorter than the one before lost its norm, and the solver stagnated.)
 //
 // Words are never reset: two buffers alternate, and a block remembers the value
 // each of its words had when it last read it (a block is at most one reduction
@@ -570,6 +573,10 @@ struct PackedAR {
 __device__ __forceinline__ void red_relaxed_add_u64(unsigned long long* p, unsigned long long v) {
     asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+constexpr int kPkUnits32 = 38, kPkUnits64 = 76;  // log2 of the units to the previous sum
+constexpr int kPkDrop32 = 6, kPkDrop64 = 6;      // exponents a sum may fall below the previous one
+// log2 of the range of a block's sum in a word of 48 bits
+__device__ __forceinline__ int pk_range() { return 15 + __clz((int)gridDim.x); }
 __device__ __forceinline__ unsigned long long pk_word(long long t, bool bad) {
     return bad ? 257ull : ((unsigned long long)t << 16) + 1ull;
 }
@@ -601,12 +608,12 @@ __device__ __forceinline__ int pk_exp(double x) {
     const int e = __double2hiint(x) >> 20 & 0x7ff;
     return e == 0 || e == 2047 ? kPkUnknown : e - 1023;
 }
-// x in units of 2^(E - 67) as hi 2^40 + lo (both with the sign of x); *bad when it exceeds 2^87 units
+// x in units of 2^(E - kPkUnits64) as hi 2^40 + lo (both with the sign of x); *bad when it exceeds 2^87 units
 __device__ __forceinline__ void pk_fix(double x, int E, long long* hi, long long* lo, bool* bad) {
     const long long b = __double_as_longlong(x);
     const int e = (int)(b >> 52) & 0x7ff;
     const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
-    const int s = max(e, 1) - 1075 - E + 67;
+    const int s = max(e, 1) - 1075 - E + kPkUnits64;
     *bad = e == 2047 || s > 34;
     const unsigned __int128 t = s >= 0 ? (unsigned __int128)m << min(s, 34)
                                        : (unsigned __int128)(s > -62 ? (m + ((1ull << -s) >> 1)) >> -s : 0ull);
@@ -618,19 +625,19 @@ __device__ __forceinline__ void pk_fix(double x, int E, long long* hi, long long
 __device__ __forceinline__ bool pk_carry(long long* hi, long long* lo) {
     *hi += *lo >> 40;
     *lo &= 0xffffffffffll;
-    return *hi < (1ll << 39) && *hi > -(1ll << 39);
+    const long long cap = 1ll << pk_range();
+    return *hi < cap && *hi > -cap;
 }
-// x in units of 2^(E - 34), rounded to nearest; *bad when it exceeds 2^39 units
+// x in units of 2^(E - kPkUnits32), rounded to nearest; *bad when it exceeds a block's range
 __device__ __forceinline__ long long pk_fix(float x, int E, bool* bad) {
     const int b = __float_as_int(x), e = b >> 23 & 0xff;
     const long long m = (b & 0x7fffff) | (e ? 0x800000 : 0);
-    const int s = max(e, 1) - 150 - E + 34;  // m 2^(e - 150)
-    *bad = e == 255 || s > 15;
-    const long long t = s >= 0 ? m << min(s, 15) : (s > -40 ? (m + ((1ll << -s) >> 1)) >> -s : 0ll);
+    const int s = max(e, 1) - 150 - E + kPkUnits32, top = pk_range() - 24;  // m 2^(e - 150)
+    *bad = e == 255 || s > top;
+    const long long t = s >= 0 ? m << min(s, top) : (s > -40 ? (m + ((1ll << -s) >> 1)) >> -s : 0ll);
     return b < 0 ? -t : t;
 }
-__device__ __forceinline__ float pk_value(long long t, int E) { return ldexpf(__ll2float_rn(t), E - 34); }
-constexpr int kPkDrop32 = 10, kPkDrop64 = 14;  // exponents a sum may fall below the previous one
+__device__ __forceinline__ float pk_value(long long t, int E) { return ldexpf(__ll2float_rn(t), E - kPkUnits32); }
 
 // hi 2^40 + lo as a 62-bit magnitude and a shift
 __device__ __forceinline__ unsigned long long pk_magnitude(long long hi, long long lo, bool* neg, int* shift) {
@@ -649,7 +656,7 @@ __device__ __forceinline__ double pk_value(long long hi, long long lo, int E) {
     bool neg;
     int k;
     const unsigned long long u = pk_magnitude(hi, lo, &neg, &k);
-    const double d = fx_value((long long)u, (unsigned)(E - 67 + k + 1075 + 4096), 4096);
+    const double d = fx_value((long long)u, (unsigned)(E - kPkUnits64 + k + 1075 + 4096), 4096);
     return neg ? -d : d;
 }
 
