@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
             if (blockIdx.x == 0 && threadIdx.x == 0) {
                 // the reference counts a cycle that ends on the new residual one further; the mixed solver
                 // counts Arnoldi steps
-                *a.out_iter = resid <= a.tol ? (kMixed || it == 0 ? it : it + 1) : (kMixed ? -1 - it : -it);
+                *a.out_iter = resid <= a.tol ? (kMixed || it == 0 ? it : it + 1) : -1 - it;
                 *a.out_resid = resid;
                 *a.out_cycles = cycles;
             }
@@ -694,12 +694,10 @@ int gmres_ls(Context* c, CSR& A, const double* b, double* x, int R, int left, in
     if (st) return set_err(c, st, "gmres: grid barrier watchdog fired");
     c->last_refinements = it[1];
     *tol = res;
-    if (sizeof(V) == 4) {
-        *max_iter = it[0] >= 0 ? it[0] : -1 - it[0];
-        return it[0] >= 0 ? TF_OK : set_err(c, TF_ERR_NOT_CONVERGED, "gmres (mixed): no convergence within max_iter");
-    }
-    *max_iter = it[0] >= 0 ? it[0] : -it[0];
-    return it[0] >= 0 ? TF_OK : set_err(c, TF_ERR_NOT_CONVERGED, "gmres: no convergence within max_iter");
+    *max_iter = it[0] >= 0 ? it[0] : -1 - it[0];
+    return it[0] >= 0 ? TF_OK
+                      : set_err(c, TF_ERR_NOT_CONVERGED, sizeof(V) == 4 ? "gmres (mixed): no convergence within max_iter"
+                                                                        : "gmres: no convergence within max_iter");
 }
 
 template int gmres_ls<double>(Context*, CSR&, const double*, double*, int, int, int*, double*, int);

@@ -115,3 +115,25 @@ def test_uneven_rows_beyond_the_cached_part_of_the_matrix(precision):
         r = b - mul(A, ctx.vec_download(tf.VEC_X))
     # the FP64 solver stops on the rotated residual, which follows the true one of a well conditioned system closely
     assert np.linalg.norm(r) <= 1.01e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("limit", [0, 1, 5, 23])
+@pytest.mark.parametrize("method,prec", [(0, tf.PREC_FP64), (1, tf.PREC_FP64), (0, tf.PREC_MIXED)])
+def test_iteration_limit(ctx, limit, method, prec):
+    """No step, fewer than a restart cycle and more: not converged, the steps counted, the residual that of x."""
+    rp, ci, v, b = banded(700, 2)
+    ctx.matrix_upload(rp, ci, v)
+    ctx.vec_upload(tf.VEC_B, b)
+    ctx.vec_upload(tf.VEC_X, np.zeros(b.size))
+    st, it, res = ctx.gmres_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, restart=8, tol=0.0, max_iter=limit, method=method,
+                                   precision=prec)
+    assert st == tf.ERR_NOT_CONVERGED and it == limit
+    r = b - O.spmv(rp, ci, v, ctx.vec_download(tf.VEC_X))  # D = 2 drops out of |D^-1 r| / |D^-1 b|
+    want = np.linalg.norm(r) / np.linalg.norm(b)
+    assert abs(res - want) <= 1e-6 * want + 1e-15
+    # a start that solves the system needs no step
+    ctx.vec_upload(tf.VEC_B, np.zeros(b.size))
+    ctx.vec_upload(tf.VEC_X, np.zeros(b.size))
+    st, it, res = ctx.gmres_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, restart=8, tol=1e-9, max_iter=limit, method=method,
+                                   precision=prec)
+    assert st == tf.OK and it == 0 and res == 0.0
