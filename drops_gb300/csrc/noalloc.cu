@@ -63,6 +63,7 @@ struct Ctrl {
     int status, iters;
     double resid;
     int converged;
+    int nnz, longest;  // k_longest_row
 };
 
 // block 0 publishes the outcome of the solve (every exit path calls this)
@@ -88,6 +89,47 @@ struct Args {
     int rel;
 };
 
+constexpr int kInFlight = 8;   // entries a lane has in flight
+constexpr int kFarTrips = 16;  // a row of more trips than this (128 entries on one lane) is summed by its warp
+constexpr int far_length(int lanes) { return kFarTrips * kInFlight * lanes; }
+
+// a lane's part of a row: every L-th entry from k
+template <int L, class A, class LOAD, class TERM>
+__device__ __forceinline__ A entries(const Args& a, A acc, int64_t row, int32_t k, int32_t e, LOAD load, TERM term) {
+    constexpr int U = kInFlight;
+    for (; k < e; k += U * L) {
+        int32_t c[U];
+        double v[U];
+        decltype(load(0)) x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = k + u * L < e;
+            c[u] = in ? __ldg(a.colind + k + u * L) : 0;
+            v[u] = in ? __ldg(a.vals + k + u * L) : 0.;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u * L < e) x[u] = load(c[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k + u * L < e) acc = term(acc, row, c[u], v[u], x[u]);
+    }
+    return acc;
+}
+struct RowAndDiag {
+    double sum, diag;
+};
+template <int L>
+__device__ __forceinline__ void lanes_sum(double& v) {
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, L);
+}
+template <int L>
+__device__ __forceinline__ void lanes_sum(RowAndDiag& v) {
+    lanes_sum<L>(v.sum);
+    lanes_sum<L>(v.diag);
+}
+
 // The rows go round-robin over the blocks, a warp's share at a time (small systems
 // use every SM); a lane keeps eight entries in flight.  p = z + beta p is formed in
 // the gathers, so an iteration has two grid steps, both packed integer reductions
@@ -97,7 +139,12 @@ struct Args {
 // for 4 rows at a time.  Per iteration of a 7-point matrix, call included: 512 rows
 // 16.1 -> 8.5 us, 8,000 23.0 -> 8.8, 65,231 34.4 -> 10.7, 238,328 70.4 -> 20.1 (before: 8
 // lanes per row, up to 8 blocks of 256 per SM, counter barriers and FP64 tree sums).
-template <int G>
+//
+// A matrix with rows of more than far_length(G) entries (bordered systems: a constraint, a Lagrange multiplier) takes the
+// form that gives such a row to all lanes of its warp; on one lane every block waits for it.  With one dense row and
+// column, us per iteration, one lane / the warp: 65,536 rows of 3 entries 8,192 / 339, 20,000 of 7 2,567 / 112, 20,000 of 41
+// (8 lanes) 392 / 121.  The other matrices would pay 3 to 5% for the test in every product, k_longest_row costs them 3 us.
+template <int G, bool FAR>
 __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(Args a) {
     const int64_t m = a.m;
     Ctrl* ctl = reinterpret_cast<Ctrl*>(a.scratch);
@@ -117,34 +164,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(Args a) {
     const int64_t step = (int64_t)gridDim.x * kThreads / G;
     __shared__ double sh[3];
 
-    // sum over the entries of a row of f(column, value), all lanes of the warp
-    auto row_sum = [&](int64_t row, auto load, auto term) {
-        constexpr int U = 8;
-        double acc = 0.;
+    // sum over the entries of a row of term(row, column, value, load(column)), all lanes of the warp; FAR: the rows far above
+    // the mean one after the other by the whole warp
+    auto row_sum = [&](int64_t row, auto zero, auto load, auto term) {
         int32_t s = 0, e = 0;
         if (row < m) {
-            s = __ldg(a.rowptr + row) + sub;
+            s = __ldg(a.rowptr + row);
             e = __ldg(a.rowptr + row + 1);
         }
-        for (int32_t k = s; k < e; k += U * G) {
-            int32_t c[U];
-            double v[U];
-            decltype(load(0)) x[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool in = k + u * G < e;
-                c[u] = in ? __ldg(a.colind + k + u * G) : 0;
-                v[u] = in ? __ldg(a.vals + k + u * G) : 0.;
+        const bool far = FAR && e - s > far_length(G);
+        auto acc = entries<G>(a, zero, row, s + sub, far ? s : e, load, term);
+        lanes_sum<G>(acc);
+        if constexpr (FAR) {
+            for (unsigned todo = __ballot_sync(0xffffffffu, far && sub == 0); todo; todo &= todo - 1u) {
+                const int src = __ffs((int)todo) - 1;
+                const int64_t fr = __shfl_sync(0xffffffffu, row, src);
+                const int32_t fs = __shfl_sync(0xffffffffu, s, src), fe = __shfl_sync(0xffffffffu, e, src);
+                auto w = entries<32>(a, zero, fr, fs + lane, fe, load, term);
+                lanes_sum<32>(w);
+                if (lane / G == src / G) acc = w;
             }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (k + u * G < e) x[u] = load(c[u]);
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (k + u * G < e) acc = term(acc, c[u], v[u], x[u]);
         }
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
         return acc;
     };
     const int64_t rounds = (m + step - 1) / step;  // the warps of a block make the same number of passes
@@ -154,17 +194,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(Args a) {
         double v[3] = {0., 0., 0.};
         for (int64_t k = 0; k < rounds; ++k) {
             const int64_t row = first + k * step;
-            double dg = 0.;
-            const double acc = row_sum(
-                row, [&](int32_t c) { return __ldcg(a.x + c); },
-                [&](double s, int32_t c, double av, double x) {
-                    if (c == row) dg = av;
-                    return s + av * x;
+            const RowAndDiag t = row_sum(
+                row, RowAndDiag{0., 0.}, [&](int32_t c) { return __ldcg(a.x + c); },
+                [](const RowAndDiag& s, int64_t rw, int32_t c, double av, double x) {
+                    return RowAndDiag{s.sum + av * x, c == rw ? av : s.diag};
                 });
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, o, G);
             if (sub == 0 && row < m) {
-                const double bi = a.b[row], ri = bi - acc, di = 1.0 / dg, zi = ri * di;
+                const double bi = a.b[row], ri = bi - t.sum, di = 1.0 / t.diag, zi = ri * di;
                 d[row] = di;
                 r[row] = ri;
                 z[row] = zi;
@@ -202,8 +238,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(Args a) {
             for (int64_t k = 0; k < rounds; ++k) {
                 const int64_t row = first + k * step;
                 const double acc = row_sum(
-                    row, [&](int32_t c) { return Pair{__ldcg(z + c), __ldcg(pc + c)}; },
-                    [&](double s, int32_t, double av, const Pair& x) { return s + av * (x.z + beta * x.p); });
+                    row, 0., [&](int32_t c) { return Pair{__ldcg(z + c), __ldcg(pc + c)}; },
+                    [&](double s, int64_t, int32_t, double av, const Pair& x) { return s + av * (x.z + beta * x.p); });
                 if (sub == 0 && row < m) {
                     const double pi = __ldcg(z + row) + beta * __ldcg(pc + row);
                     pn[row] = pi;
@@ -252,6 +288,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_noalloc(Args a) {
     }
 }
 
+__global__ void k_longest_row(int64_t m, const int32_t* __restrict__ rowptr, Ctrl* ctl) {
+    int n = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m; i += (int64_t)gridDim.x * blockDim.x)
+        n = max(n, rowptr[i + 1] - rowptr[i]);
+    n = __reduce_max_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && n > 0) atomicMax(&ctl->longest, n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->nnz = rowptr[m];
+}
+
 }  // namespace
 
 extern "C" int tf_pcg_jacobi_noalloc(int64_t m, const int32_t* rowptr, const int32_t* colind, const double* vals,
@@ -265,27 +310,32 @@ extern "C" int tf_pcg_jacobi_noalloc(int64_t m, const int32_t* rowptr, const int
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return TF_ERR_CUDA;
-    // average row length picks the lanes per row; the matrix's row pointers are on the device
-    int32_t nnz = 0;
-    if (cudaMemcpyAsync(&nnz, rowptr + m, sizeof(int32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    if (sms > kMaxBlocks) sms = kMaxBlocks;
+    // the control words must start at zero; everything else is written before it is read
+    if (cudaMemsetAsync(scratch, 0, sizeof(double) * (kCtrlDoubles + kWordDoubles), s) != cudaSuccess) return TF_ERR_CUDA;
+    // average row length picks the lanes per row, the longest row their form; the matrix's row pointers are on the device
+    Ctrl ctl;
+    const int64_t scan = (m + 1023) / 1024;
+    void* scan_args[] = {&m, &rowptr, &scratch};
+    if (cudaLaunchKernel((const void*)k_longest_row, dim3((unsigned)(scan < sms ? scan : sms)), dim3(1024), scan_args, 0, s) !=
+            cudaSuccess ||
+        cudaMemcpyAsync(&ctl, scratch, sizeof(Ctrl), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return TF_ERR_CUDA;
-    const double avg = (double)nnz / (double)m;
+    const double avg = (double)ctl.nnz / (double)m;
     // long rows are spread over lanes; 152 x 512 lanes hold 77,824 rows
     const int G = avg <= 32 ? 1 : avg <= 128 ? 8 : 32;
-    const void* fn = G == 1 ? (const void*)k_pcg_noalloc<1> : G == 8 ? (const void*)k_pcg_noalloc<8>
-                                                                     : (const void*)k_pcg_noalloc<32>;
-    if (sms > kMaxBlocks) sms = kMaxBlocks;
+    const bool far = ctl.longest > far_length(G);
+    const void* fn = G == 1   ? (far ? (const void*)k_pcg_noalloc<1, true> : (const void*)k_pcg_noalloc<1, false>)
+                     : G == 8 ? (far ? (const void*)k_pcg_noalloc<8, true> : (const void*)k_pcg_noalloc<8, false>)
+                              : (const void*)k_pcg_noalloc<32, false>;
     // at least four warps per block
     const int64_t want = (m * G + 127) / 128;
     int blocks = (int)(want < sms ? want : sms);
     if (blocks < 1) blocks = 1;
-    // the control words must start at zero; everything else is written before it is read
-    if (cudaMemsetAsync(scratch, 0, sizeof(double) * (kCtrlDoubles + kWordDoubles), s) != cudaSuccess) return TF_ERR_CUDA;
     Args a{m, rowptr, colind, vals, b, x, scratch, *max_iter, *tol, rel};
     void* args[] = {&a};
     if (cudaLaunchCooperativeKernel(fn, blocks, kThreads, args, 0, s) != cudaSuccess) return TF_ERR_CUDA;
-    Ctrl ctl;
     if (cudaMemcpyAsync(&ctl, scratch, sizeof(Ctrl), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return TF_ERR_CUDA;
