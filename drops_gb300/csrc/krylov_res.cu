@@ -859,12 +859,16 @@ int pcg64_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter
     const int64_t m = A.m;
     const void* fn = (const void*)k_pcg64_res;
     const int blocks = res_blocks(c, A);
-    TF_TRY(ensure_res_plan(c, A, blocks));
-    const Sell& S = A.sell;
-    if (!S.res_ok || S.res_smax <= 0 || S.res_smax > kBalMaxSlices) return TF_OK;
-    const int32_t ccap = (S.res_maxslots + 15) & ~15;
     int64_t room = 0;
     TF_TRY(max_dynamic_smem(c, fn, &room));
+    // No run is smaller than the mean, so a mean that does not fit rules the system out before its plan: a kernel over the
+    // matrix and a wait.
+    const Sell& S = A.sell;
+    const int64_t mean_slices = (S.used + blocks - 1) / blocks, mean_slots = (S.npad + blocks - 1) / blocks;
+    if (mean_slices > kBalMaxSlices || (int64_t)pcg64_fixed_bytes((int)mean_slices, 0, (int32_t)mean_slots) > room) return TF_OK;
+    TF_TRY(ensure_res_plan(c, A, blocks));
+    if (!S.res_ok || S.res_smax <= 0 || S.res_smax > kBalMaxSlices) return TF_OK;
+    const int32_t ccap = (S.res_maxslots + 15) & ~15;
     const int64_t fixed = (int64_t)pcg64_fixed_bytes(S.res_smax, S.res_hmax, ccap);
     if (fixed > room) return TF_OK;
     const int32_t vcap = (int32_t)std::min<int64_t>((room - fixed) / (int64_t)sizeof(double), (int64_t)ccap) & ~7;

@@ -86,3 +86,31 @@ def test_pcg_zero_and_converged_start(ctx):
     ctx.vec_upload(tf.VEC_B, O.spmv(rp, ci, v, b))
     st, it, res = ctx.pcg_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, tol=1e-10)
     assert st == tf.OK and it == 0 and np.array_equal(ctx.vec_download(tf.VEC_X), b)
+
+
+@pytest.mark.parametrize("m,extra", [(400000, 0), (60000, 80)])
+def test_systems_beyond_shared_memory_build_no_plan(monkeypatch, m, extra):
+    """Too many rows, or too many entries, for the blocks' shared memory: the first solve launches what it launches with
+    the resident solver off."""
+    rng = np.random.default_rng(2)
+    if extra:  # a band: the 16-bit columns of a block (60000 * 321 * 2 / 152 bytes) exceed its 227 KB
+        off = np.arange(-extra * 2, extra * 2 + 1)
+    else:
+        off = np.arange(-1, 2)
+    cols = np.arange(m)[:, None] + off[None, :]
+    keep = (cols >= 0) & (cols < m)
+    vals = np.where(off == 0, 2.0 * len(off), -1.0) * np.ones((m, 1))
+    rp = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int64)
+    b = rng.standard_normal(m)
+    launches = []
+    for resident in ("0", "1"):
+        monkeypatch.setenv("TF_PCG_RESIDENT", resident)
+        with tf.TraceFEM(0) as ctx:
+            ctx.matrix_upload(rp, cols[keep].astype(np.int64), vals[keep])
+            ctx.vec_upload(tf.VEC_B, b)
+            ctx.vec_upload(tf.VEC_X, np.zeros(m))
+            n0 = ctx.launch_count()
+            st, it, res = ctx.pcg_jacobi(tf.MAT_USER, tf.VEC_B, tf.VEC_X, tol=1e-10)
+            launches.append(ctx.launch_count() - n0)
+            assert st == tf.OK and res <= 1e-10
+    assert launches[0] == launches[1]
