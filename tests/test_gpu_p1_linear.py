@@ -161,3 +161,20 @@ def test_linear_and_other_tets_together(ctx, n, share):
     ctx.levelset_upload(lv, le)
     ctx.distribute_dofs(tf.P1IF)
     compare(ctx)
+
+
+@pytest.mark.parametrize("rhs,par", LOADS)
+def test_repeated_calls_agree(ctx, rhs, par):
+    """The tets that are not linear are listed in the order in which warps reach the list, which differs from call to
+    call; every tet writes its own record, so the results are the same bits."""
+    rng = np.random.default_rng(8)
+    ctx.brick_cube(40, 5.0 / 3.0)
+    ctx.levelset_analytic(tf.LS_SPHERE, [0.0, 0.1, 0.0, 1.0], False)
+    lv, le = ctx.levelset_download()
+    ctx.levelset_upload(lv, np.where(rng.uniform(size=le.size) < 0.1, le + 2e-5 * rng.uniform(-1.0, 1.0, le.size), le))
+    ctx.distribute_dofs(tf.P1IF)
+    first = None
+    for _ in range(8):
+        now = [x.tobytes() for x in forms(ctx, tf.ASM_KERNEL_PAIR, rhs, par)[1]]
+        assert first is None or now == first
+        first = now
