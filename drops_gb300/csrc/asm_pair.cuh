@@ -46,27 +46,16 @@ static int ensure_tables_ff(Context* c) {
     return TF_OK;
 }
 
-// Per warp.  The FP64 per-tet scratch (geometry, patch) is dead once split
-// into pairs, so it shares storage with the point rows.  Point rows are padded
-// to an odd number of pairs per lane (11 and 21): a lane's row starts 22 or 42
-// words after its neighbour's, so the lanes' 64-bit stores of one column fall
-// in distinct banks, and the contraction's reads of one row (one point, ten
-// columns) do too.
-struct AsmPairFp64 {
-    TetGeom g;
-    double gM[9], gC[9];
-    double ls10[10];
-    PatchSmem P;
-};
+// Per warp.  Point rows are padded to an odd number of pairs per lane (11 and
+// 21): a lane's row starts 22 or 42 words after its neighbour's, so the lanes'
+// 64-bit stores of one column fall in distinct banks, and the contraction's
+// reads of one row (one point, ten columns) do too.
 struct AsmPairPts {
     ff phi[32][11];  // sqrt(w) phi_i; n . grad(phi_i) sqrt(w) for the volume rule
     ff sg[32][21];   // [2 i + c]: sqrt(w) grad(phi_i) in an orthonormal basis of the tangent plane
 };
 struct AsmPairSmem {
-    union {
-        AsmPairFp64 d;
-        AsmPairPts p;
-    } u;
+    AsmPairPts p;
     ff gl[4][3], G[4][3], X[4][3], absdet;
     ff fb[16][3][4], fw[16];
     ff fx[32];  // sqrt(w) f(x_p)
@@ -339,7 +328,7 @@ __global__ void __launch_bounds__(32 * kAsmWarps) k_assemble_p2_pair(AsmArgs A) 
                 S.fb[f][j >> 2][j & 3] = Q.fb[f][j >> 2][j & 3];
         }
         __syncwarp();
-        AsmPairPts& P = S.u.p;
+        AsmPairPts& P = S.p;
 
         ffacc accM[EPL], accA[EPL], accF;
         const int npts = 7 * nf;

@@ -248,18 +248,6 @@ __device__ inline void warp_tet_geometry(TetGeom& g, const double* ls10, double*
     __syncwarp();
 }
 
-// 1/sqrt(s) to FP64 accuracy: FP32 seed and two Newton steps
-// y <- y (3/2 - s/2 y^2) (relative error ~1e-16); FP64 division and square
-// root are long instruction sequences on the FP64 pipe, this is ~10 operations.
-__device__ inline double rsqrt_fp64(double s) {
-    if (!(s > 1e-30 && s < 1e30)) return 1.0 / sqrt(s);
-    double y = (double)rsqrtf((float)s);
-    const double h = 0.5 * s;
-    y = y * (1.5 - h * y * y);
-    y = y * (1.5 - h * y * y);
-    return y;
-}
-
 __device__ inline void unit_normal(const TetGeom& g, const double b[4], double n[3]) {
     double v[3];
     for (int r = 0; r < 3; ++r) v[r] = b[0] * g.G[0][r] + b[1] * g.G[1][r] + b[2] * g.G[2][r] + b[3] * g.G[3][r];

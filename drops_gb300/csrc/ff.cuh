@@ -143,6 +143,17 @@ __device__ __forceinline__ double widen_f32(float x) {
 // pair -> double with one FP64 instruction
 __device__ __forceinline__ double ff_widen(ff a) { return __dadd_rn(widen_f32(a.h), widen_f32(a.l)); }
 
+// 1/sqrt(s) to FP64 accuracy: FP32 seed and two Newton steps
+// y <- y (3/2 - s/2 y^2) (relative error ~1e-16); FP64 division and square
+// root are long instruction sequences on the FP64 pipe, this is ~10 operations.
+__device__ __forceinline__ double rsqrt_fp64(double s) {
+    if (!(s > 1e-30 && s < 1e30)) return 1.0 / sqrt(s);
+    double y = (double)rsqrtf((float)s);
+    const double h = 0.5 * s;
+    y = y * (1.5 - h * y * y);
+    return y * (1.5 - h * y * y);
+}
+
 // x 2^e, exact where the result is normal
 __device__ __forceinline__ double scale_pow2(double x, int e) {
     const int hi = __double2hiint(x), ex = hi >> 20 & 0x7ff, to = ex + e;

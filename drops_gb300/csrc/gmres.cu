@@ -120,17 +120,8 @@ __device__ __forceinline__ double ls_sum1(double v) {
     return warp_fx_sum(one);
 }
 
-// 1 / sqrt(x): FP64 from an FP32 seed and two Newton steps (relative error
-// about 2^-52; a square root and a division are 1,200 cycles of the FP64 pipe
-// on GB300, this is 9 operations of 64)
 __device__ __forceinline__ float ls_rsqrt(float x) { return 1.0f / sqrtf(x); }
-__device__ __forceinline__ double ls_rsqrt(double x) {
-    if (!(x > 1e-30 && x < 1e30)) return 1.0 / sqrt(x);
-    double y = (double)rsqrtf((float)x);
-    const double h = 0.5 * x;
-    y = y * (1.5 - h * y * y);
-    return y * (1.5 - h * y * y);
-}
+__device__ __forceinline__ double ls_rsqrt(double x) { return rsqrt_fp64(x); }
 
 // The n block partials in part[block][value] summed over the blocks into tot
 // (all blocks the same bits): thread t takes value t % n over every G-th
@@ -572,12 +563,6 @@ __global__ void __launch_bounds__(kLsThreads, 1) k_gmres_ls(GmLsArgs<V> a) {
 }
 
 // the SELL columns as slots (pad entries: the slot of their row, or 0)
-__global__ void k_ls_slots(int64_t nslots, const int32_t* __restrict__ perm, int32_t* __restrict__ iperm) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nslots; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t r = perm[i];
-        if (r >= 0) iperm[r] = (int32_t)i;
-    }
-}
 __global__ void k_ls_cols(int64_t npad, const int32_t* __restrict__ col, const int32_t* __restrict__ iperm,
                           int32_t* __restrict__ cols) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < npad; i += (int64_t)gridDim.x * blockDim.x)
@@ -589,11 +574,9 @@ int ensure_slot_cols(Context* c, CSR& A, int id, const int32_t** cols) {
     Sell& S = A.sell;
     TF_TRY(ensure(c, c->sell_cols[id], (size_t)(S.npad > 0 ? S.npad : 1)));
     if (c->sell_cols_gen[id] != S.pattern_gen) {
-        TF_TRY(ensure(c, c->scratch, sizeof(int32_t) * (size_t)A.m));
-        int32_t* iperm = (int32_t*)c->scratch.p;
-        k_ls_slots<<<grid_for(c, S.nslices * 32), kBlock, 0, c->stream>>>(S.nslices * 32, S.perm, iperm);
-        k_ls_cols<<<grid_for(c, S.npad), kBlock, 0, c->stream>>>(S.npad, S.col, iperm, c->sell_cols[id].p);
-        c->launches += 2;
+        TF_TRY(ensure_sell_iperm(c, A));
+        k_ls_cols<<<grid_for(c, S.npad), kBlock, 0, c->stream>>>(S.npad, S.col, S.iperm, c->sell_cols[id].p);
+        ++c->launches;
         TF_CUDA(c, cudaGetLastError());
         c->sell_cols_gen[id] = S.pattern_gen;
     }

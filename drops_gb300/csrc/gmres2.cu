@@ -30,33 +30,32 @@ struct Gm2Scal {
     long long it, done, converged, cycle_end, cycles, i, pad;
 };
 
-template <class V>
 struct Gm2Args {
     int64_t m, nslices;
     const int32_t* perm;
     const int32_t* ptr;
     const int32_t* col;
-    const V* bval;        // SELL values of B = A P^{-1}
-    const double* aval;   // SELL values of A (FP64), true residual
+    const double* bval;   // SELL values of B = A P^{-1}
+    const double* aval;   // SELL values of A, true residual
     const double* b;
     double* x;
     const double* diag;   // point Jacobi (nullptr with binv)
     const double* binv;   // nodal 2x2 inverses [m/2][4]
-    V* basis;             // (R+1) x m, unnormalised; v_k = scl[k] * basis_k
+    double* basis;        // (R+1) x m, unnormalised; v_k = scl[k] * basis_k
     double* part;         // [nblocks][kGm2Stride]
     Gm2Scal* sc;
-    V* small;             // H (R+1) x R column-major, cs[R], sn[R], s[R+1], y[R], scl[R+1], coef[R+1]
+    double* small;        // H (R+1) x R column-major, cs[R], sn[R], s[R+1], y[R], scl[R+1], coef[R+1]
     GridSync gs;
     unsigned* mcount;  // grid-step arrivals (monotone)
     int R, max_iter, rel;
-    double tol, inner_floor;
+    double tol;
     int* out_iter;
     double* out_resid;
     int* out_cycles;
 };
 
 // Grid step with a fixed master block.  Every block has written n partial
-// sums (type S) for this step; block 0 waits until all others have arrived,
+// sums for this step; block 0 waits until all others have arrived,
 // sums the partials in a fixed order, and its thread 0 runs f(sums, state) on
 // block 0's shared-memory copy of the state (the Hessenberg matrix and the
 // Givens rotations live in block 0's shared memory too, so the serial scalar
@@ -80,11 +79,11 @@ __device__ __forceinline__ unsigned gm2_ld_relaxed(const unsigned* p) {
     return v;
 }
 
-template <class S, class F>
-__device__ bool gm2_step(const GridSync& g, unsigned* mcount, Gm2Sync& sy, const S* part, int n, Gm2Scal* gsc,
+template <class F>
+__device__ bool gm2_step(const GridSync& g, unsigned* mcount, Gm2Sync& sy, const double* part, int n, Gm2Scal* gsc,
                          Gm2Scal& ssc, F f) {
     __shared__ int st;
-    __shared__ S sums[kGm2Stride];
+    __shared__ double sums[kGm2Stride];
     const unsigned target_gen = sy.gen + 1;
     __syncthreads();
     if (blockIdx.x != 0) {
@@ -138,19 +137,19 @@ __device__ bool gm2_step(const GridSync& g, unsigned* mcount, Gm2Sync& sy, const
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const int nb = (int)gridDim.x;
         for (int k0 = warp; k0 < n; k0 += kGm2Warps * kGm2Group) {
-            S v[kGm2Group][kGm2Chunks];
+            double v[kGm2Group][kGm2Chunks];
 #pragma unroll
             for (int g = 0; g < kGm2Group; ++g) {
                 const int k = k0 + g * kGm2Warps;
 #pragma unroll
                 for (int j = 0; j < kGm2Chunks; ++j) {
                     const int b = lane + 32 * j;
-                    v[g][j] = k < n && b < nb ? __ldcg(part + (size_t)k * nb + b) : S(0);
+                    v[g][j] = k < n && b < nb ? __ldcg(part + (size_t)k * nb + b) : 0.;
                 }
             }
 #pragma unroll
             for (int g = 0; g < kGm2Group; ++g) {
-                S acc = S(0);
+                double acc = 0.;
 #pragma unroll
                 for (int j = 0; j < kGm2Chunks; ++j) acc += v[g][j];
                 acc = warp_sum(acc);
@@ -174,42 +173,39 @@ __device__ bool gm2_step(const GridSync& g, unsigned* mcount, Gm2Sync& sy, const
 }
 
 // warp partials (wred[k][warp]) -> block partials part[k][block] (value-major)
-template <class S>
-__device__ __forceinline__ void gm2_block_partials(S (*wred)[kGm2Warps], int n, S* part) {
+__device__ __forceinline__ void gm2_block_partials(double (*wred)[kGm2Warps], int n, double* part) {
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        S x = S(0);
+        double x = 0.;
         for (int w = 0; w < kGm2Warps; ++w) x += wred[k][w];
         part[(size_t)k * gridDim.x + blockIdx.x] = x;
     }
 }
 
-template <class V>
-__global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
+__global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args a) {
     __shared__ Gm2Scal sc;
-    __shared__ V wred[kGm2Stride][kGm2Warps];   // Arnoldi dots, in V
+    __shared__ double wred[kGm2Stride][kGm2Warps];  // Arnoldi dots
     // least-squares state, used by block 0 (the master of every grid step)
-    __shared__ V H[(kGm2MaxR + 1) * kGm2MaxR];  // H[k][i] at H[i * (R + 1) + k]
-    __shared__ V cs[kGm2MaxR], sn[kGm2MaxR], s[kGm2MaxR + 1], ys[kGm2MaxR];
-    __shared__ double wres[2][kGm2Warps];       // FP64 true residual
-    double* const part64 = a.part;
-    V* const partV = reinterpret_cast<V*>(a.part);
+    __shared__ double H[(kGm2MaxR + 1) * kGm2MaxR];  // H[k][i] at H[i * (R + 1) + k]
+    __shared__ double cs[kGm2MaxR], sn[kGm2MaxR], s[kGm2MaxR + 1], ys[kGm2MaxR];
+    __shared__ double wres[2][kGm2Warps];            // true residual
+    double* const part = a.part;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t m = a.m;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
     const int R = a.R;
     // published by the master for every block: solution of the least-squares
     // problem, basis scales, projection coefficients
-    V* const y = a.small;
-    V* const scl = y + R;
-    V* const coef = scl + R + 1;
-    const double tol = a.tol, inner_floor = a.inner_floor;
+    double* const y = a.small;
+    double* const scl = y + R;
+    double* const coef = scl + R + 1;
+    const double tol = a.tol;
     const int max_iter = a.max_iter, rel = a.rel;
     bool first = true;
     Gm2Sync sy;
 
     for (;;) {
-        // ---- cycle start: r = b - A x (FP64) into basis_0; |r|^2, |b|^2 ----
+        // ---- cycle start: r = b - A x into basis_0; |r|^2, |b|^2 ----
         {
             double v[2] = {0., 0.};
             const double* x = a.x;
@@ -219,7 +215,7 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                 if (row >= 0) {
                     const double bi = a.b[row];
                     const double r = bi - ax;
-                    a.basis[row] = (V)r;
+                    a.basis[row] = r;
                     v[0] += r * r;
                     v[1] += bi * bi;
                 }
@@ -228,9 +224,9 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                 const double t = warp_sum(v[k]);
                 if (lane == 0) wres[k][warp] = t;
             }
-            gm2_block_partials<double>(wres, 2, part64);
+            gm2_block_partials(wres, 2, part);
             const bool init = first;
-            if (!gm2_step<double>(a.gs, a.mcount, sy, part64, 2, a.sc, sc, [&](const double* t, Gm2Scal& g) {
+            if (!gm2_step(a.gs, a.mcount, sy, part, 2, a.sc, sc, [&](const double* t, Gm2Scal& g) {
                     if (init) {
                         double nb = sqrt(t[1]);
                         if (nb == 0.0 || !rel) nb = 1.0;
@@ -246,9 +242,9 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                     g.i = 0;
                     if (!g.done) {
                         ++g.cycles;
-                        scl[0] = (V)(1.0 / g.beta);
-                        s[0] = (V)g.beta;
-                        for (int k = 1; k <= R; ++k) s[k] = V(0);
+                        scl[0] = 1.0 / g.beta;
+                        s[0] = g.beta;
+                        for (int k = 1; k <= R; ++k) s[k] = 0.;
                     }
                 }))
                 return;
@@ -258,35 +254,35 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
         // ---- Arnoldi steps ----
         while (!sc.cycle_end) {
             const int i = (int)sc.i;
-            V* const Vi = a.basis + (size_t)i * m;
-            V* const W = a.basis + (size_t)(i + 1) * m;
-            const V sci = scl[i];
+            double* const Vi = a.basis + (size_t)i * m;
+            double* const W = a.basis + (size_t)(i + 1) * m;
+            const double sci = scl[i];
             // (1) w = B v_i and the first projection dots <v_k, w>, k <= i
             for (int k = threadIdx.x; k <= i; k += blockDim.x)
-                for (int w = 0; w < kGm2Warps; ++w) wred[k][w] = V(0);
+                for (int w = 0; w < kGm2Warps; ++w) wred[k][w] = 0.;
             __syncthreads();
             TF_SLICE_LOOP_BAL(a.nslices, sl) {
-                const V acc = sell_row<V>(a.ptr, a.col, a.bval, sl, lane, [&](int32_t j) { return sci * kld(Vi + j); });
+                const double acc = sell_row<double>(a.ptr, a.col, a.bval, sl, lane, [&](int32_t j) { return sci * kld(Vi + j); });
                 const int32_t row = __ldg(a.perm + sl * 32 + lane);
                 if (row >= 0) W[row] = acc;
                 // eight dots per transposing warp butterfly (9 shuffles instead of 40)
                 for (int k0 = 0; k0 <= i; k0 += 8) {
-                    V t8[8];
+                    double t8[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int k = k0 + q;
-                        t8[q] = row >= 0 && k <= i ? scl[k] * kld(a.basis + (size_t)k * m + row) * acc : V(0);
+                        t8[q] = row >= 0 && k <= i ? scl[k] * kld(a.basis + (size_t)k * m + row) * acc : 0.;
                     }
-                    const V tot = warp_sum8(t8, lane);
+                    const double tot = warp_sum8(t8, lane);
                     const int k = k0 + warp_sum8_index(lane);
                     if ((lane & 3) == 0 && k <= i) wred[k][warp] += tot;
                 }
             }
-            gm2_block_partials<V>(wred, i + 1, partV);
-            if (!gm2_step<V>(a.gs, a.mcount, sy, partV, i + 1, a.sc, sc, [&](const V* t, Gm2Scal& g) {
+            gm2_block_partials(wred, i + 1, part);
+            if (!gm2_step(a.gs, a.mcount, sy, part, i + 1, a.sc, sc, [&](const double* t, Gm2Scal& g) {
                     for (int k = 0; k <= i; ++k) {
-                        coef[k] = (V)t[k];
-                        H[(size_t)i * (R + 1) + k] = (V)t[k];
+                        coef[k] = t[k];
+                        H[(size_t)i * (R + 1) + k] = t[k];
                     }
                 }))
                 return;
@@ -296,18 +292,18 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
             // barrier, as the next product gathers w2 across blocks
             for (int pass = 0; pass < 2; ++pass) {
                 for (int k = threadIdx.x; k <= i + 1; k += blockDim.x)
-                    for (int w = 0; w < kGm2Warps; ++w) wred[k][w] = V(0);
+                    for (int w = 0; w < kGm2Warps; ++w) wred[k][w] = 0.;
                 __syncthreads();
                 // warp-uniform trip count (the warp's first row decides), so every
                 // lane reaches the warp reductions; rows past m are masked
                 for (int64_t e0 = tid; e0 - lane < m; e0 += 4 * nth) {
-                    V wv[4];
+                    double wv[4];
                     bool in[4];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int64_t e = e0 + q * nth;
                         in[q] = e < m;
-                        V w = in[q] ? kld(W + e) : V(0);
+                        double w = in[q] ? kld(W + e) : 0.;
                         if (in[q])
                             for (int k = 0; k <= i; ++k) w -= coef[k] * (scl[k] * kld(a.basis + (size_t)k * m + e));
                         wv[q] = w;
@@ -316,13 +312,13 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                     if (pass == 0) {
                         // values 0..i: <v_k, w1>; value i + 1: |w1|^2
                         for (int k0 = 0; k0 <= i + 1; k0 += 8) {
-                            V t8[8];
+                            double t8[8];
 #pragma unroll
                             for (int g = 0; g < 8; ++g) {
                                 const int k = k0 + g;
-                                V t = V(0);
+                                double t = 0.;
                                 if (k <= i) {
-                                    const V* Vk = a.basis + (size_t)k * m;
+                                    const double* Vk = a.basis + (size_t)k * m;
 #pragma unroll
                                     for (int q = 0; q < 4; ++q)
                                         if (in[q]) t += scl[k] * kld(Vk + e0 + q * nth) * wv[q];
@@ -332,7 +328,7 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                                 }
                                 t8[g] = t;
                             }
-                            const V tot = warp_sum8(t8, lane);
+                            const double tot = warp_sum8(t8, lane);
                             const int k = k0 + warp_sum8_index(lane);
                             if ((lane & 3) == 0 && k <= i + 1) wred[k][warp] += tot;
                         }
@@ -343,47 +339,46 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                     ++sy.gen;  // the barrier's last arrival bumped the generation word
                     continue;
                 }
-                gm2_block_partials<V>(wred, i + 2, partV);
-                if (!gm2_step<V>(a.gs, a.mcount, sy, partV, i + 2, a.sc, sc, [&](const V* t, Gm2Scal& g) {
-                        V* hc = H + (size_t)i * (R + 1);
-                        V h2sq = V(0);
+                gm2_block_partials(wred, i + 2, part);
+                if (!gm2_step(a.gs, a.mcount, sy, part, i + 2, a.sc, sc, [&](const double* t, Gm2Scal& g) {
+                        double* hc = H + (size_t)i * (R + 1);
+                        double h2sq = 0.;
                         for (int k = 0; k <= i; ++k) {
-                            coef[k] = (V)t[k];
-                            hc[k] += (V)t[k];
-                            h2sq += (V)t[k] * (V)t[k];
+                            coef[k] = t[k];
+                            hc[k] += t[k];
+                            h2sq += t[k] * t[k];
                         }
-                        const V n2 = (V)t[i + 1] - h2sq;
-                        const V hn = n2 > V(0) ? (V)sqrt(n2) : V(0);
+                        const double n2 = t[i + 1] - h2sq;
+                        const double hn = n2 > 0. ? sqrt(n2) : 0.;
                         hc[i + 1] = hn;
-                        scl[i + 1] = hn != V(0) ? V(1) / hn : V(0);
+                        scl[i + 1] = hn != 0. ? 1. / hn : 0.;
                         // previous rotations on column i, then the new one
                         for (int k = 0; k < i; ++k) {
-                            const V t0 = cs[k] * hc[k] + sn[k] * hc[k + 1];
+                            const double t0 = cs[k] * hc[k] + sn[k] * hc[k + 1];
                             hc[k + 1] = -sn[k] * hc[k] + cs[k] * hc[k + 1];
                             hc[k] = t0;
                         }
-                        const V dx = hc[i], dy = hc[i + 1];
-                        if (dy == V(0)) {
-                            cs[i] = V(1);
-                            sn[i] = V(0);
+                        const double dx = hc[i], dy = hc[i + 1];
+                        if (dy == 0.) {
+                            cs[i] = 1.;
+                            sn[i] = 0.;
                         } else {
-                            const V r = sqrt(dx * dx + dy * dy);
+                            const double r = sqrt(dx * dx + dy * dy);
                             cs[i] = dx / r;
                             sn[i] = dy / r;
                         }
                         hc[i] = cs[i] * dx + sn[i] * dy;
-                        hc[i + 1] = V(0);
-                        const V si = s[i];
+                        hc[i + 1] = 0.;
+                        const double si = s[i];
                         s[i] = cs[i] * si;
                         s[i + 1] = -sn[i] * si;
                         g.it += 1;
-                        const double est = fabs((double)s[i + 1]);
-                        const bool stop = est <= fmax(inner_floor * g.beta, 0.5 * tol * g.normb) || i + 1 == R ||
-                                          g.it >= max_iter || hn == V(0);
+                        const double est = fabs(s[i + 1]);
+                        const bool stop = est <= 0.5 * tol * g.normb || i + 1 == R || g.it >= max_iter || hn == 0.;
                         if (stop) {
                             // y = H^{-1} s on the leading (i+1) x (i+1) triangle
                             for (int q = i; q >= 0; --q) {
-                                V acc = s[q];
+                                double acc = s[q];
                                 for (int p2 = q + 1; p2 <= i; ++p2) acc -= H[(size_t)p2 * (R + 1) + q] * ys[p2];
                                 ys[q] = acc / H[(size_t)q * (R + 1) + q];
                             }
@@ -395,27 +390,27 @@ __global__ void __launch_bounds__(kKryThreads, 2) k_gmres2(Gm2Args<V> a) {
                     return;
             }
         }
-        // ---- x += P^{-1} sum_k y_k v_k (FP64 update) ----
+        // ---- x += P^{-1} sum_k y_k v_k ----
         {
             const int kk = (int)sc.i - 1;
             if (a.binv) {
                 const int64_t half = m / 2;
                 for (int64_t e = tid; e < half; e += nth) {
-                    V za = V(0), zb = V(0);
+                    double za = 0., zb = 0.;
                     for (int q = 0; q <= kk; ++q) {
-                        const V c = y[q] * scl[q];
+                        const double c = y[q] * scl[q];
                         za += c * kld(a.basis + (size_t)q * m + e);
                         zb += c * kld(a.basis + (size_t)q * m + e + half);
                     }
                     const double* q4 = a.binv + 4 * e;
-                    a.x[e] += q4[0] * (double)za + q4[1] * (double)zb;
-                    a.x[e + half] += q4[2] * (double)za + q4[3] * (double)zb;
+                    a.x[e] += q4[0] * za + q4[1] * zb;
+                    a.x[e + half] += q4[2] * za + q4[3] * zb;
                 }
             } else {
                 for (int64_t e = tid; e < m; e += nth) {
-                    V z = V(0);
+                    double z = 0.;
                     for (int q = 0; q <= kk; ++q) z += (y[q] * scl[q]) * kld(a.basis + (size_t)q * m + e);
-                    a.x[e] += (double)z / a.diag[e];
+                    a.x[e] += z / a.diag[e];
                 }
             }
             if (!grid_barrier(a.gs)) return;
@@ -518,13 +513,12 @@ int gmres_operator(Context* c, CSR& A, int left, const V** out) {
 template int gmres_operator<double>(Context*, CSR&, int, const double**);
 template int gmres_operator<float>(Context*, CSR&, int, const float**);
 
-template <class V>
 static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int* max_iter, double* tol, int rel) {
     const int64_t m = A.m;
     const bool block = &A == &c->mats[TF_MAT_BLOCK];
-    const V* bval = nullptr;
-    TF_TRY(gmres_operator<V>(c, A, 0, &bval));
-    const void* fn = (const void*)k_gmres2<V>;
+    const double* bval = nullptr;
+    TF_TRY(gmres_operator<double>(c, A, 0, &bval));
+    const void* fn = (const void*)k_gmres2;
     int blocks = 0;
     TF_TRY(coop_blocks(c, fn, A.sell.nslices, &blocks, kKryThreads));
     blocks = std::min(blocks, kGm2MaxBlocks);  // the master's partial reads cover kGm2MaxBlocks blocks
@@ -538,7 +532,7 @@ static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int
     TF_TRY(ensure(c, c->kry_resid, 1));
     TF_CUDA(c, cudaMemsetAsync(c->kry_bar.p, 0, 4 * sizeof(unsigned), c->stream));
     TF_CUDA(c, cudaMemsetAsync(c->status.p, 0, 4 * sizeof(int), c->stream));
-    Gm2Args<V> g{};
+    Gm2Args g{};
     g.m = m;
     g.nslices = A.sell.nslices;
     g.perm = A.sell.perm;
@@ -560,7 +554,6 @@ static int run_gmres2(Context* c, CSR& A, const double* b, double* x, int R, int
     g.max_iter = *max_iter;
     g.rel = rel;
     g.tol = *tol;
-    g.inner_floor = 0.0;
     g.out_iter = c->kry_iters.p;
     g.out_resid = c->kry_resid.p;
     g.out_cycles = c->kry_iters.p + 1;
@@ -586,7 +579,7 @@ int gmres2(Context* c, CSR& A, const double* b, double* x, int restart, int* max
     TF_TRY(ensure_diag(c, A));
     TF_TRY(ensure_sell(c, A, false));
     TimedLaunch tl(c, TF_K_GMRES);
-    return run_gmres2<double>(c, A, b, x, restart, max_iter, tol, rel);
+    return run_gmres2(c, A, b, x, restart, max_iter, tol, rel);
 }
 
 }  // namespace tf

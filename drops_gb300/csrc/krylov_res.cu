@@ -688,19 +688,11 @@ int mat_slot(Context* c, const CSR& A) {
     return 0;
 }
 
-// row -> slot map, halo lists and translated columns, once per pattern and grid
+// halo lists and translated columns, once per pattern and grid
 int ensure_res_plan(Context* c, CSR& A, int blocks) {
     Sell& S = A.sell;
     const int id = mat_slot(c, A);
-    if (S.iperm_gen != S.pattern_gen || !S.iperm) {
-        TF_TRY(ensure(c, c->sell_iperm[id], (size_t)(A.m > 0 ? A.m : 1)));
-        S.iperm = c->sell_iperm[id].p;
-        k_sell_iperm<<<grid_for(c, S.nslices * 32), kBlock, 0, c->stream>>>(S.nslices * 32, S.perm, S.iperm);
-        ++c->launches;
-        TF_CUDA(c, cudaGetLastError());
-        S.iperm_gen = S.pattern_gen;
-        S.res_blocks = 0;
-    }
+    TF_TRY(ensure_sell_iperm(c, A));
     if (S.res_blocks != blocks) {
         TF_TRY(ensure(c, c->sell_coltr[id], (size_t)(S.npad > 0 ? S.npad : 1)));
         TF_TRY(ensure(c, c->sell_halo[id], (size_t)blocks * kHaloMax + blocks));
@@ -734,6 +726,21 @@ int res_blocks(const Context* c, const CSR& A) {
 }
 
 }  // namespace
+
+// row -> slot map of the SELL layout, once per pattern
+int ensure_sell_iperm(Context* c, CSR& A) {
+    Sell& S = A.sell;
+    if (S.iperm_gen == S.pattern_gen && S.iperm) return TF_OK;
+    const int id = mat_slot(c, A);
+    TF_TRY(ensure(c, c->sell_iperm[id], (size_t)(A.m > 0 ? A.m : 1)));
+    S.iperm = c->sell_iperm[id].p;
+    k_sell_iperm<<<grid_for(c, S.nslices * 32), kBlock, 0, c->stream>>>(S.nslices * 32, S.perm, S.iperm);
+    ++c->launches;
+    TF_CUDA(c, cudaGetLastError());
+    S.iperm_gen = S.pattern_gen;
+    S.res_blocks = 0;  // its plan follows the old map
+    return TF_OK;
+}
 
 // zeroed words for n packed reductions
 int packed_words(Context* c, int n, unsigned long long** w) {

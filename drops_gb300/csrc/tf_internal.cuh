@@ -578,6 +578,7 @@ int spmv(Context* c, const CSR& A, const double* x, double* y);
 int pcg_jacobi(Context* c, CSR& A, const double* b, double* x, int precision, int* max_iter, double* tol, int rel);
 template <class T>
 int pcg_resident(Context* c, CSR& A, const double* b, double* x, int* max_iter, double* tol, int rel, bool* applied);
+int ensure_sell_iperm(Context* c, CSR& A);
 int packed_words(Context* c, int n, unsigned long long** w);
 int pcg_cluster_ctas(const Context* c, const CSR& A);
 template <class V>
