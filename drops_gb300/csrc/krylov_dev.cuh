@@ -544,9 +544,9 @@ __device__ bool grid_allreduce(const GridAR& g, unsigned long long& epoch, const
 // block gets the same bits.  The unit of a value follows from its previous sum,
 // which all blocks know: an FP32 value takes one word with 2^38 units to that
 // sum, an FP64 value two (a 48-bit high and a 40-bit low part) with 2^76.  The
-// blocks repeat the reduction with grid_allreduce when a block's sum exceeds the
-// previous sum twice (8 times; on fewer than 128 blocks more) or is not finite,
-// and when the sum is smaller than 2^-6 of it.  So the rounding of all the terms
+// blocks repeat the reduction with grid_allreduce when a block's sum exceeds twice
+// (8 times in FP64; on fewer than 128 blocks more) the previous sum or is not
+// finite, and when the sum is smaller than 2^-6 of it.  So the rounding of all the terms
 // that are aligned to the unit - the blocks' sums in FP32, at most 255; the
 // threads' values in FP64, at most 2^17 - adds up to at most 255 x 2^-39 x 2^6 =
 // 2^-25 (2^17 x 2^-77 x 2^6 = 2^-54) of the sum: half of what rounding it to its

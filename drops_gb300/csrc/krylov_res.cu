@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_pcg_res(PcgResArgs<T> a) {
 // instruction and quarter of an SM).  Against the kernel that walks the SELL
 // matrix in global memory and forms z + beta p per entry (k_pcg, which remains
 // for systems whose block share does not fit), per iteration on GB300:
-// P2 torus on 41^3 cubes (35,592 rows, 152 blocks) 23.1 -> 11.7 us, P1 sphere on
+// P2 torus on 41^3 cubes (35,592 rows, 152 blocks) 23.1 -> 9.6 us, P1 sphere on
 // 16^3 (664 rows, 16 blocks) 12.1 -> 8.4 us.
 // ---------------------------------------------------------------------------
 struct Pcg64Args {

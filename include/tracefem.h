@@ -372,9 +372,10 @@ int tf_batch_lincomb(tf_context* ctx, int nterms, const int* forms, const double
  * instance's iterations and reached residual; TF_ERR_NOT_CONVERGED when any
  * instance missed tol.  Every instance is solved on a thread-block cluster of 1
  * to 8 CTAs, their number chosen from the batch's row counts, unless
- * tf_batch_config fixed lanes or an instance does not fit (about 18,000 rows in
- * FP64, 36,000 mixed).  Otherwise one CTA solves an instance, and unless fixed
- * the lanes per row and CTA size come from tf_batch_tune, run on the first
+ * tf_batch_config fixed lanes, the matrix is an uploaded one, an instance does
+ * not fit (about 18,000 rows in FP64, 36,000 mixed) or the device has no memory
+ * for the clusters' scratch.  Otherwise one CTA solves an instance, and unless
+ * fixed the lanes per row and CTA size come from tf_batch_tune, run on the first
  * solve of a pattern.  The launch sequence
  * is captured once as a CUDA graph and replayed while matrix, vectors and
  * parameters stay the same.                                                    */
